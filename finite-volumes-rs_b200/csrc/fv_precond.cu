@@ -31,6 +31,7 @@
 #include <cub/cub.cuh>
 
 #include "fv_internal.cuh"
+#include "fv_resident.cuh"
 
 struct fv_symbolic {
     int64_t n = 0, nnz_l = 0, nnz_u = 0;
@@ -122,7 +123,59 @@ struct fv_precond {
     float *t_rhs32[2] = {nullptr, nullptr};
     unsigned t_rec64_epoch = 0, t_rec32_version = 0;
     unsigned f32_version = 0;  // incremented by every fv_precond_make_f32
+    // resident sweeps (fv_resident.cuh): the plan when the factor has one, and
+    // the records of the current factors; a schedule or launch shape asked for
+    // explicitly takes the other kernels
+    fv_resident *res = nullptr;
+    void *res_rec = nullptr, *res_rec32 = nullptr;
+    bool explicit_schedule = false;
 };
+
+static fv_resident_src resident_src(const fv_precond *P, const int32_t *perm) {
+    const fv_symbolic *s = P->sym;
+    fv_resident_src q;
+    q.n = P->n;
+    q.nnz_l = s->nnz_l;
+    q.nnz_u = s->nnz_u;
+    q.l_ptr = s->l_ptr;
+    q.l_col = s->l_col;
+    q.u_ptr = s->u_ptr;
+    q.u_col = s->u_col;
+    q.fwd_order = s->fwd_order;
+    q.fwd_level = s->d_fwd_level;
+    q.bwd_level = s->d_bwd_level;
+    q.n_fwd_levels = s->n_fwd_levels;
+    q.n_bwd_levels = s->n_bwd_levels;
+    q.max_side = std::max(s->max_lower, s->max_upper);
+    q.sorted = P->contiguous;
+    q.perm = perm;
+    if (P->A->mesh && P->A->mesh->n_cells == P->n) q.cell = P->A->mesh->cell;
+    return q;
+}
+
+static bool use_resident(const fv_precond *P) {
+    return P->res && !P->explicit_schedule && P->sweep_blocks == 0 && P->sweep_rpt == 0;
+}
+
+// The plan and its records are an optimisation: without memory for them the
+// other sweeps run.
+static fv_status resident_no_memory(fv_precond *P) {
+    cudaGetLastError();
+    fv_resident_free(P->res);
+    P->res = nullptr;
+    return FV_OK;
+}
+
+static fv_status resident_plan(fv_precond *P, const int32_t *perm, cudaStream_t st) {
+    const fv_resident_src q = resident_src(P, perm);
+    const fv_status s = fv_resident_build(q, st, &P->res);
+    if (s == FV_ERR_ALLOC) return resident_no_memory(P);
+    if (s != FV_OK || !P->res) return s;
+    const cudaError_t e = cudaMalloc(&P->res_rec, fv_resident_record_bytes(P->res, sizeof(double)));
+    if (e == cudaErrorMemoryAllocation) return resident_no_memory(P);
+    FV_CUDA_TRY(e);
+    return FV_OK;
+}
 
 // ------------------------------------------------------------------ symbolic
 static fv_status build_symbolic_impl(const fv_csr *A, cudaStream_t st, fv_symbolic **out) {
@@ -1781,6 +1834,10 @@ fv_status fv_precond_apply_dev(fv_precond *P, const double *r, double *z, cudaSt
         FV_CUDA_TRY(cudaGetLastError());
         return FV_OK;
     }
+    if (use_resident(P)) {
+        FV_CUDA_TRY(fv_resident_apply<double>(P->res, P->res_rec, r, z, skip, rs, P->err, st));
+        return FV_OK;
+    }
     const int G = P->sweep_blocks > 0 ? P->sweep_blocks : sweep_grid(n);
     if (P->perm) {  // reordered factorisation: gather r, sweep in B's numbering, scatter z
         const bool pf = P->schedule == 3;
@@ -1888,6 +1945,14 @@ fv_status fv_precond_make_f32(fv_precond *P, cudaStream_t st) {
     if (s->nnz_u) fv_note_launch(), k_to_f32<<<G, 256, 0, st>>>(s->nnz_u, P->u_val, P->u32);
     fv_note_launch(), k_to_f32<<<G, 256, 0, st>>>(n, P->dinv, P->dinv32);
     FV_CUDA_TRY(cudaGetLastError());
+    if (P->res) {
+        if (!P->res_rec32 &&
+            cudaMalloc(&P->res_rec32, fv_resident_record_bytes(P->res, sizeof(float))) != cudaSuccess)
+            cudaGetLastError();  // no memory: the other sweeps run
+        if (P->res_rec32)
+            FV_CUDA_TRY(fv_resident_records<float>(P->res, resident_src(P, P->perm), P->kind == 2, P->l32, P->u32, P->dinv32,
+                                                   P->res_rec32, st));
+    }
     P->f32_version += 1;
     return FV_OK;
 }
@@ -1905,6 +1970,10 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
         return FV_OK;
     }
     if (!P->l32) return FV_ERR_INVALID;
+    if (use_resident(P) && P->res_rec32) {
+        FV_CUDA_TRY(fv_resident_apply<float>(P->res, P->res_rec32, r, z, skip, rs, P->err, st));
+        return FV_OK;
+    }
     const int G = P->sweep_blocks > 0 ? P->sweep_blocks : sweep_grid(n);
     if (P->perm) {  // reordered factorisation: gather r, sweep in B's numbering, scatter z
         const bool pf = P->schedule == 3;
@@ -1973,7 +2042,10 @@ extern "C" fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t
     if (request == 2) FV_TRY(build_tiles(s, P->A, fv_stream(nullptr)));
     if (request == 2 && !s->tiled) return FV_ERR_UNSUPPORTED;
     if (request == 4 && (P->perm || P->fill)) return FV_ERR_UNSUPPORTED;
-    if (request >= 0) P->schedule = request <= 1 ? 1 : request;
+    if (request >= 0) {
+        P->schedule = request <= 1 ? 1 : request;
+        P->explicit_schedule = true;
+    }
     if (active) *active = use_tiles(P) ? 2 : (P->schedule == 3 || P->schedule == 4 ? P->schedule : 1);
     if (stats) {
         stats[0] = s->t_edge;
@@ -2004,6 +2076,9 @@ extern "C" fv_status fv_precond_destroy(fv_precond *P) {
     cudaFree(P->perm);
     cudaFree(P->zint);
     cudaFree(P->zint32);
+    fv_resident_free(P->res);
+    cudaFree(P->res_rec);
+    cudaFree(P->res_rec32);
     for (int d = 0; d < 2; ++d) {
         cudaFree(P->t_rec64[d]);
         cudaFree(P->t_rec32[d]);
@@ -2040,7 +2115,9 @@ __global__ void k_order_not_identity(int64_t n, const int32_t *__restrict__ orde
 }
 }  // namespace
 
-static fv_status factor_common(const fv_csr *Ac, int kind, cudaStream_t st, fv_precond **out) {
+// perm: the caller's row of every row of Ac when Ac is a reordered matrix (fv_*_factor_perm).
+static fv_status factor_common(const fv_csr *Ac, int kind, cudaStream_t st, fv_precond **out,
+                               const int32_t *perm = nullptr) {
     if (!Ac || !out) return FV_ERR_INVALID;
     if (Ac->nrows != Ac->ncols) return FV_ERR_INVALID;
     fv_csr *A = const_cast<fv_csr *>(Ac);
@@ -2133,7 +2210,16 @@ static fv_status factor_common(const fv_csr *Ac, int kind, cudaStream_t st, fv_p
 #undef FV_IC
     }
     FV_CUDA_TRY(cudaGetLastError());
-    fv_status es = fv_precond_check_error(P, st);
+    fv_status es = fresh ? resident_plan(P, perm, st) : FV_OK;
+    if (es == FV_OK && P->res) {
+        const cudaError_t e = fv_resident_records<double>(P->res, resident_src(P, perm), kind == 2, P->l_val, P->u_val,
+                                                          P->dinv, P->res_rec, st);
+        if (e != cudaSuccess) {
+            fv_internal_set_cuda_error(e, "resident sweep records");
+            es = FV_ERR_CUDA;
+        }
+    }
+    if (es == FV_OK) es = fv_precond_check_error(P, st);
     if (es != FV_OK) {
         if (fresh) fv_precond_destroy(P);
         return es;
@@ -2421,7 +2507,7 @@ static fv_status perm_factor_impl(const fv_csr *Ac, const int32_t *perm_host, in
     tmp.fill = nullptr;
     tmp.amap = nullptr;
     fv_precond *P = nullptr;
-    if (s == FV_OK) s = factor_common(B, kind, st, &P);
+    if (s == FV_OK) s = factor_common(B, kind, st, &P, perm);
     if (s == FV_OK) P->schedule = 1;  // the reordered sweeps have their own kernels (P->perm)
     if (s == FV_OK) {
         e = cudaMalloc(&P->zint, sizeof(double) * n);

@@ -1,0 +1,318 @@
+// Resident triangular sweeps: one thread-block cluster applies M^-1 with the
+// whole vector in (distributed) shared memory.
+//
+// What bounds the level-chunk sweeps on small systems is the hand-off of a
+// level through L2 (0.8-1.1 us per level, whatever its width).  Here every
+// CTA of a cluster owns a set of rows and keeps their slots of the vector in
+// its shared memory; it walks its rows level by level, each step one row per
+// thread, and the few values that other CTAs need are pushed into halo slots
+// of their shared memory (st.shared::cluster), where the consumer polls its own
+// copy.  The vector is updated in place: right-hand side, forward result and
+// backward result occupy the same slot, so nothing but the factor's records
+// streams from memory.  A level costs 0.13-0.15 us: operands from shared
+// memory (30 cycles), the row's FP64 chain (40), one store and one barrier.
+//
+// Measured per apply (both sweeps; level chunks -> resident): 131,072-row IC(0)
+// in natural order (512 levels) 790 -> 150 us, 24,576-row ILU(0) (64 levels)
+// 140 -> 38 us, 196,608-row ILU(0) (128 levels) 247 -> 62 us; 65,522-row IC(0)
+// in box order (18 wide levels; consecutive rows -> resident) 42 -> 25 us.
+//
+// Rows are computed with the operations of k_sweep in the same order, so the
+// results are the same bits.
+//
+// Forward progress: the CTAs of a cluster are co-resident.  A CTA at level L
+// waits only for values of lower levels, so the CTA at the lowest level never
+// waits on anything unfinished.  Every wait is bounded in time.
+#pragma once
+
+#include "fv_internal.cuh"
+
+// One row of a sweep: factor values, 1/diagonal (1 where the diagonal is a
+// unit), the shared-memory slots of its dependencies and its own, the first
+// remote reader of its value (rank << 16 | slot) and
+//   meta = offset of further readers in the push table << 8 | their number << 4
+//          | kResPush | kResHalo
+// Unused entries have value 0 and read the slot that holds 0 (x - 0 * 0 keeps
+// every x, signed zeros included); idle lanes of a step write the slot after it.
+enum : uint32_t { kResHalo = 1, kResPush = 2 };
+template <typename T, int ML>
+struct __align__(16) fv_res_rec {
+    T val[ML];
+    T d;
+    uint16_t dep[ML];
+    uint16_t self;
+    uint32_t push0, meta;
+};
+static_assert(sizeof(fv_res_rec<double, 3>) == 48 && sizeof(fv_res_rec<double, 4>) == 64 &&
+                  sizeof(fv_res_rec<double, 6>) == 80 && sizeof(fv_res_rec<float, 3>) == 32,
+              "record sizes are multiples of 16");
+
+constexpr int kResMaxCta = 16;  // largest cluster
+constexpr size_t kResSmem = 226 * 1024;  // dynamic shared memory of a CTA (1 KB is left for static use)
+// The records stream into shared memory as bulk copies of whole groups of
+// steps (about 16 KB, one copy by one thread), kResBuffers groups deep: a copy
+// takes about a microsecond from L2, a group of steps as long.  (Loading them
+// into registers ahead of use was slower: a ring of loads per step runs out of
+// the six scoreboards a warp tracks its loads with, and the unrolled code out
+// of the instruction cache.)
+constexpr int kResBuffers = 4;
+constexpr int kResGroupBytes = 16 * 1024;
+
+// The plan of an apply.  Every CTA has one list of steps, the levels of its
+// rows forward and then backward; a level is one or more steps of `width`
+// slots, one row per thread, and every step ends with a barrier.
+struct fv_resident {
+    int C = 0, width = 0, sets = 0, ml = 0;  // CTAs, rows per step, thread sets (below), entries per record
+    int32_t cap = 0;               // most rows of a CTA
+    int32_t halo = 0;              // most halo slots of a CTA
+    int64_t nslots = 0;            // slots of all steps
+    int32_t *cta_ptr = nullptr;    // [C + 1] first entry of a CTA in `rows`
+    int32_t *rows = nullptr;       // slot k of CTA c holds row rows[cta_ptr[c] + k]
+    int32_t *nat = nullptr;        // the same rows in the caller's numbering (null: no permutation)
+    uint16_t *slot_of = nullptr;   // the slot of every row in its CTA
+    int32_t *step_ptr = nullptr;   // [C + 1] first step of every CTA
+    uint32_t *push = nullptr;      // further push targets, rank << 16 | slot
+    int32_t *slot_item = nullptr;  // row (forward) or n + row (backward) of every slot, -1: idle
+    uint16_t *slot_dep = nullptr;  // [ml] per slot
+    uint32_t *slot_push = nullptr; // push0, meta per slot
+    void *arena[2] = {nullptr, nullptr};  // the allocations the arrays lie in
+};
+
+__device__ __forceinline__ unsigned fv_cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void fv_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void fv_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned fv_mapa(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void fv_push(unsigned addr, double v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(fv_pack_value(v)) : "memory");
+}
+__device__ __forceinline__ void fv_push(unsigned addr, float v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(fv_pack_value(v)) : "memory");
+}
+__device__ __forceinline__ bool fv_halo_ready(unsigned addr, double &v) {
+    unsigned long long b;
+    asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(b) : "r"(addr) : "memory");
+    v = __longlong_as_double((long long)b);
+    return b != FV_SENTINEL_U64;
+}
+__device__ __forceinline__ bool fv_halo_ready(unsigned addr, float &v) {
+    unsigned b;
+    asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(b) : "r"(addr) : "memory");
+    v = __uint_as_float(b);
+    return b != FV_SENTINEL_U32;
+}
+__device__ __forceinline__ bool fv_is_sentinel(double v) {
+    return (unsigned long long)__double_as_longlong(v) == FV_SENTINEL_U64;
+}
+__device__ __forceinline__ bool fv_is_sentinel(float v) { return __float_as_uint(v) == FV_SENTINEL_U32; }
+__device__ __forceinline__ double fv_sentinel(double) { return __longlong_as_double(-1LL); }
+__device__ __forceinline__ float fv_sentinel(float) { return __uint_as_float(FV_SENTINEL_U32); }
+
+// The value of a halo slot, waited for (bounded like fv_wait_value).
+template <typename T>
+__device__ __noinline__ T fv_halo_value(unsigned addr, int *err) {
+    T v;
+    if (fv_halo_ready(addr, v)) return v;
+    const unsigned long long t0 = fv_globaltimer();
+    for (unsigned it = 1; !fv_halo_ready(addr, v); ++it)
+        if ((it & 255u) == 0 && (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS)) {
+            if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
+            return T(NAN);
+        }
+    return v;
+}
+
+__device__ __forceinline__ uint4 fv_lds16(unsigned a) {
+    uint4 v;
+    asm volatile("ld.shared::cta.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fv_lds(unsigned a, double &v) {
+    asm volatile("ld.shared::cta.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void fv_lds(unsigned a, float &v) {
+    asm volatile("ld.shared::cta.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void fv_sts(unsigned a, double v) {
+    asm volatile("st.shared::cta.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void fv_sts(unsigned a, float v) {
+    asm volatile("st.shared::cta.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// Both sweeps over this CTA's rows, in place in xs, by the first S * width
+// threads of the block (the others skip it; the caller synchronises the block
+// before and after).  rec: the CTA's first step, a step being `PL` planes of
+// `width` 16-byte pieces (conflict-free reads); nsteps steps, `group` of them
+// per copy (both multiples of S).  The S sets of threads take the steps in
+// turn, and a set waits only for the step before its own (arrive / sync on the
+// steps' named barriers; what lies further back is ordered through it).  While
+// the others compute, a set unpacks the record of its next step, so from one
+// step to the next lie only the operands' loads, the row's arithmetic and one
+// store: with all threads at one barrier per step the unpacking (about 400
+// cycles) set the pace.  buf: kResBuffers
+// groups of records; bars: kResBuffers mbarriers, initialised with count 1;
+// groups: copies made through them before, kept across calls.  halo0: first
+// halo slot (the slots before it are the constant 0 and the idle lanes' slot).
+template <typename T, int ML, int S>
+__device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec, int nsteps, int width, int group,
+                                                   T *xs, unsigned halo0, uint4 *buf, unsigned long long *bars,
+                                                   unsigned &groups, const uint32_t *__restrict__ push, int *err) {
+    using R = fv_res_rec<T, ML>;
+    constexpr int PL = (int)(sizeof(R) / 16);
+    const int set = S == 1 ? 0 : (int)threadIdx.x / width, lane = (int)threadIdx.x - set * width;
+    const int ng = (nsteps + group - 1) / group;
+    const unsigned xbase = (unsigned)__cvta_generic_to_shared(xs);
+    const unsigned bbase = (unsigned)__cvta_generic_to_shared(buf) + (unsigned)lane * 16u;
+    const unsigned mbase = (unsigned)__cvta_generic_to_shared(bars);
+    const unsigned step_bytes = (unsigned)(width * PL) * 16u;
+    const unsigned g0 = groups;
+    auto copy = [&](int g) {  // one thread
+        if (g >= ng) return;
+        const unsigned b = (g0 + g) % kResBuffers, bytes = (unsigned)min(group, nsteps - g * group) * step_bytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbase + 8 * b), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         bbase + b * group * step_bytes),
+                     "l"(rec + (int64_t)g * group * width * PL), "r"(bytes), "r"(mbase + 8 * b)
+                     : "memory");
+    };
+    // step k ends with barrier 1 + k % S: its set arrives, the next step's set waits
+    const int after_prev = 1 + (set + S - 1) % S, after_own = 1 + set, two = 2 * width;
+    auto wait_prev = [&]() {
+        __syncwarp();
+        asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(after_prev), "r"(two) : "memory");
+    };
+    auto end_own = [&]() {
+        __syncwarp();
+        if (S == 1)
+            asm volatile("barrier.cta.sync.aligned 1, %0;" ::"r"(width) : "memory");
+        else
+            asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(after_own), "r"(two) : "memory");
+    };
+    union Stage {
+        uint4 q[PL];
+        R r;
+        __device__ Stage() {}
+    };
+    Stage u;
+    unsigned a_self = 0, a_push = 0, a_dep[ML], slow = 0;
+    // the set's next step: steps left of its group, that group's successor, its record's address
+    int left = 0, g = 0, todo = nsteps / S;
+    unsigned src = 0;
+    auto fetch = [&]() {
+        if (todo == 0) return;
+        --todo;
+        bool late = false;
+        if (left == 0) {  // the set's first step of group g: its copy has landed
+            // the step computed last lies in group g - 1: every record of group g - 2 has been read
+            if (threadIdx.x == 0 && g > 1) copy(g - 2 + kResBuffers);
+            const unsigned b = (g0 + g) % kResBuffers, parity = ((g0 + g) / kResBuffers) & 1u;
+            unsigned done = 0;
+            unsigned long long t0 = 0;
+            for (unsigned it = 0; !done && !late; ++it) {
+                asm volatile(
+                    "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                    : "=r"(done)
+                    : "r"(mbase + 8 * b), "r"(parity)
+                    : "memory");
+                if (!done && (it & 63u) == 63u) {
+                    if (!t0) t0 = fv_globaltimer();
+                    late = fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS;
+                }
+            }
+            if (late) atomicOr(err, FV_DEV_TIMEOUT);
+            left = group / S;
+            src = bbase + (b * group + set) * step_bytes;
+            ++g;
+        }
+        --left;
+#pragma unroll
+        for (int p = 0; p < PL; ++p) u.q[p] = fv_lds16(src + (unsigned)(p * width) * 16u);
+        src += S * step_bytes;
+        if (late) {  // an idle slot: the steps and their barriers go on
+#pragma unroll
+            for (int q = 0; q < ML; ++q) u.r.dep[q] = (uint16_t)(halo0 - 2);
+            u.r.self = (uint16_t)(halo0 - 1);
+            u.r.meta = u.r.push0 = 0;
+        }
+        a_self = xbase + u.r.self * (unsigned)sizeof(T);
+#pragma unroll
+        for (int q = 0; q < ML; ++q) a_dep[q] = xbase + u.r.dep[q] * (unsigned)sizeof(T);
+        slow = __any_sync(0xffffffffu, (u.r.meta & (kResHalo | kResPush)) != 0);
+        if (slow) a_push = fv_mapa(xbase + (u.r.push0 & 0xFFFFu) * (unsigned)sizeof(T), u.r.push0 >> 16);
+    };
+    if (threadIdx.x == 0)
+        for (int g = 0; g < kResBuffers; ++g) copy(g);
+    fetch();
+    for (int st = set; st < nsteps; st += S) {
+        if (S > 1 && st > 0) wait_prev();
+        T x, xv[ML];
+#pragma unroll
+        for (int q = 0; q < ML; ++q) fv_lds(a_dep[q], xv[q]);
+        fv_lds(a_self, x);
+        if (slow) {
+            if (u.r.meta & kResHalo) {
+#pragma unroll
+                for (int q = 0; q < ML; ++q)
+                    if (u.r.dep[q] >= halo0 && fv_is_sentinel(xv[q])) xv[q] = fv_halo_value<T>(a_dep[q], err);
+            }
+#pragma unroll
+            for (int q = 0; q < ML; ++q) x = x - u.r.val[q] * xv[q];
+            x = u.r.d * x;
+            fv_sts(a_self, x);
+            if (u.r.meta & kResPush) {
+                fv_push(a_push, x);
+                for (uint32_t e = u.r.meta >> 8, last = e + ((u.r.meta >> 4) & 15u); e < last; ++e) {
+                    const uint32_t t = __ldg(&push[e]);
+                    fv_push(fv_mapa(xbase + (t & 0xFFFFu) * (unsigned)sizeof(T), t >> 16), x);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < ML; ++q) x = x - u.r.val[q] * xv[q];
+            x = u.r.d * x;
+            fv_sts(a_self, x);
+        }
+        if (S > 1) end_own();
+        fetch();
+        if (S == 1) end_own();
+    }
+    if (S > 1 && set == 0 && nsteps > 0) wait_prev();  // the last step's arrivals are met
+    groups = g0 + ng;
+}
+
+// The symbolic side of a factor a plan is built from (all arrays on the device).
+struct fv_resident_src {
+    int64_t n = 0, nnz_l = 0, nnz_u = 0;
+    const int32_t *l_ptr = nullptr, *l_col = nullptr, *u_ptr = nullptr, *u_col = nullptr;
+    const int32_t *fwd_level = nullptr, *bwd_level = nullptr;
+    const int32_t *fwd_order = nullptr;  // rows by forward level
+    int32_t n_fwd_levels = 0, n_bwd_levels = 0, max_side = 0;  // max_side: longest strict-lower / strict-upper row
+    bool sorted = false;                                       // rows sorted by forward level
+    const int32_t *perm = nullptr;                             // caller's row of every row (null: the same)
+    const double4 *cell = nullptr;                             // the rows' cell centres (null: unknown)
+};
+
+// The plan for a factor, or null when the resident sweeps do not apply (too
+// many rows or entries per row, or a shape the level-chunk sweeps serve better).
+fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out);
+void fv_resident_free(fv_resident *p);
+
+// Records of the factor's current values (rec: fv_resident_record_bytes of
+// device memory).  unit_fwd: the forward sweep has a unit diagonal.
+size_t fv_resident_record_bytes(const fv_resident *p, size_t value_bytes);
+template <typename T>
+cudaError_t fv_resident_records(const fv_resident *p, const fv_resident_src &s, bool unit_fwd, const T *l_val,
+                                const T *u_val, const T *dinv, void *rec, cudaStream_t st);
+
+// z = M^-1 r (one kernel); rows that rs skips keep their z.
+template <typename T>
+cudaError_t fv_resident_apply(const fv_resident *p, const void *rec, const T *r, T *z, const int *skip,
+                              const fv_row_skip &rs, int *err, cudaStream_t st);

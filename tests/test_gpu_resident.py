@@ -1,0 +1,102 @@
+"""Resident sweeps (one cluster, the vector in shared memory) against the
+level-chunk kernels of the same factor, asked for explicitly: the same bits,
+at sizes around the step width, the cluster sizes and the record sizes, on
+repeated applies and after a refactorisation, in FP64 (preconditioner apply)
+and FP32 (mixed batch solve), with rows without any dependency and with
+non-finite right-hand sides."""
+import numpy as np
+import pytest
+
+from cases import convdiff_3d, diffusion_2d, equation
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(fv, cls, A, **kw):
+    P, Q = cls.from_matrix(A, 0, **kw), cls.from_matrix(A, 0, **kw)
+    Q.schedule(1)
+    return P, Q
+
+
+def _same_apply(fv, P, Q, n, seed=0):
+    rng = np.random.default_rng(seed)
+    z, y = fv.DistributedVector.from_size(n), fv.DistributedVector.from_size(n)
+    for k in range(3):
+        r = rng.standard_normal(n)
+        if k == 2 and n > 3:
+            r[n // 2], r[n // 3], r[0] = np.inf, np.nan, -0.0
+        P.precondition(z, fv.DistributedVector(r))
+        Q.precondition(y, fv.DistributedVector(r))
+        a, b = z.numpy(), y.numpy()
+        assert np.array_equal(a, b, equal_nan=True)
+        assert np.array_equal(np.signbit(a[a == 0]), np.signbit(b[b == 0]))
+
+
+@pytest.mark.parametrize("dim,side", [(2, 1), (2, 3), (2, 31), (2, 33), (2, 95), (2, 141), (3, 1), (3, 2), (3, 7),
+                                      (3, 13), (3, 21), (3, 31)])
+def test_resident_equals_level_chunks(fv, dim, side):
+    case = diffusion_2d(fv, side, seed=61) if dim == 2 else convdiff_3d(fv, side, seed=62)
+    cls = fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper
+    A, _ = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    n = case["mesh"].n_cells
+    B = A.permuted(fv.order_boxes(A)[0])
+    for M, kw in ((A, {}), (A, {"ordering": "boxes"}), (B, {})):
+        P, Q = _pair(fv, cls, M, **kw)
+        _same_apply(fv, P, Q, n)
+    case["kappa"] = case["kappa"] * 1.7  # new values, the plan kept
+    fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"], lhs=A)
+    P, Q = _pair(fv, cls, A)
+    case["kappa"] = case["kappa"] * 0.3
+    fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"], lhs=A)
+    P.refactor()
+    Q.refactor()
+    _same_apply(fv, P, Q, n, 1)
+
+
+def _grid7(m):
+    """7-point operator on an m^3 grid: rows of up to 7 entries, no mesh behind it."""
+    i = np.arange(m ** 3)
+    x, y, z = i % m, (i // m) % m, i // (m * m)
+    rows, cols, vals = [i], [i], [np.full(m ** 3, 6.5)]
+    for ok, off in ((x > 0, -1), (x < m - 1, 1), (y > 0, -m), (y < m - 1, m), (z > 0, -m * m), (z < m - 1, m * m)):
+        rows.append(i[ok])
+        cols.append(i[ok] + off)
+        vals.append(np.full(ok.sum(), -1.0) + 0.01 * np.sin(i[ok] + off + i[ok]))
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    o = np.lexsort((c, r))
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=m ** 3))])
+    return ptr, c[o], v[o], (x + y + z) % 2
+
+
+@pytest.mark.parametrize("m", [2, 9, 24])
+@pytest.mark.parametrize("kind", ["ic", "ilu"])
+def test_resident_without_a_mesh_and_long_rows(fv, m, kind):
+    ptr, cols, vals, colour = _grid7(m)
+    A = fv.DistributedMatrix.from_csr(ptr, cols, vals)
+    cls = fv.IncompleteCholesky if kind == "ic" else fv.IncompleteLowerUpper
+    red_black = np.argsort(colour, kind="stable").astype(np.int32)  # 6 entries on one side of a row
+    shuffled = np.random.default_rng(5).permutation(m ** 3).astype(np.int32)
+    for kw in ({}, {"ordering": red_black}, {"ordering": shuffled}):
+        P, Q = _pair(fv, cls, A, **kw)
+        _same_apply(fv, P, Q, m ** 3)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_resident_in_a_batch(fv, precision):
+    """Problems that converge at different iterations: converged rows are skipped the same way."""
+    from fvb200.batch import BatchCG, MeshBatch
+    meshes = [fv.Mesh.cube(s, 0.15, 70 + s) for s in (3, 9, 5)]
+    f = [m.fields(70, 0.1, 0.5, velocity=(1.0, 0.5, 0.25), source_uniform=True) for m in meshes]
+    mb = MeshBatch(meshes)
+    kf, fl, sc = (mb.face_field([q[0] for q in f]), mb.face_field([q[1] for q in f]), mb.cell_field([q[2] for q in f]))
+    bc = (np.zeros(mb.n_boundary_faces), np.zeros(mb.n_boundary_faces))
+    A, b = fv.assemble(fv.convection(fv.Upwind(fl), fl) - fv.laplacian(fv.Orthogonal(), kf) - fv.source(sc), bc, mb)
+    out = []
+    for explicit in (False, True):
+        P = fv.IncompleteLowerUpper.from_matrix(A, 0)
+        if explicit:
+            P.schedule(1)
+        x = fv.DistributedVector.from_size(mb.n_cells)
+        info = BatchCG(A, mb.cell_offsets, 256).solve(P, b, x, precision=precision, solver="bicgstab")
+        out.append((x.numpy(), info["iterations"].tolist()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
