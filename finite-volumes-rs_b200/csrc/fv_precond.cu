@@ -1909,6 +1909,13 @@ fv_status fv_precond_check_error(fv_precond *P, cudaStream_t st) {
 }
 
 int *fv_precond_err_ptr(fv_precond *P) { return P->err; }
+// The plan of the resident sweeps when they serve this preconditioner's applies, with the records and error word.
+const fv_resident *fv_precond_resident(const fv_precond *P, const void **rec, int **err) {
+    if (P->kind == 3 || !use_resident(P)) return nullptr;
+    *rec = P->res_rec;
+    *err = P->err;
+    return P->res;
+}
 int64_t fv_precond_rows(const fv_precond *P) { return P->n; }
 
 namespace {

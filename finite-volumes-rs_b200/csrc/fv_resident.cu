@@ -338,116 +338,39 @@ __global__ void k_res_records(fv_resident p, int64_t n, bool unit_fwd, const int
 }
 
 // ------------------------------------------------------------------ the apply
-struct ResArgs {
-    const uint4 *rec;
-    const uint32_t *push;
-    const int32_t *step_ptr, *cta_ptr, *rows;  // rows: in the caller's numbering
-    int cap, halo, width, group;
-};
-
 template <typename T, int ML, int S>
-__global__ void __launch_bounds__(512, 1) k_resident_apply(ResArgs a, const T *__restrict__ r, T *__restrict__ z,
-                                                           const int *skip, fv_row_skip rs, int *err) {
+__global__ void __launch_bounds__(kResThreads, 1) k_resident_apply(const __grid_constant__ fv_res_args a, const T *__restrict__ r,
+                                                                   T *__restrict__ z, const int *skip, fv_row_skip rs,
+                                                                   int *err) {
     if (skip && *(volatile const int *)skip) return;  // the same answer in every CTA of the cluster
-    constexpr int PL = (int)(sizeof(fv_res_rec<T, ML>) / 16);
     extern __shared__ __align__(128) unsigned char res_smem[];
     __shared__ unsigned long long bars[kResBuffers];
-    uint4 *buf = reinterpret_cast<uint4 *>(res_smem);
-    T *xs = reinterpret_cast<T *>(buf + kResBuffers * a.group * a.width * PL);
-    const unsigned c = fv_cluster_rank();
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int r0 = a.cta_ptr[c], nr = a.cta_ptr[c + 1] - r0;
-    const int s0 = a.step_ptr[c], ns = a.step_ptr[c + 1] - s0;
-    const int32_t *__restrict__ rows = a.rows + r0;
-    if (tid == 0) {
-        for (int b = 0; b < kResBuffers; ++b)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&bars[b])));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (tid < 2) xs[a.cap + tid] = T(0);
-    for (int k = tid; k < a.halo; k += nt) xs[a.cap + 2 + k] = fv_sentinel(T(0));
+    fv_res_cta<T, ML, S> cta(a, res_smem, bars);
     fv_cluster_arrive();  // no push before every CTA's halo is reset
-#pragma unroll 8
-    for (int k = tid; k < nr; k += nt) xs[k] = r[__ldg(&rows[k])];
+    cta.load(r);
     fv_cluster_wait();
-    __syncthreads();
-    unsigned groups = 0;
-    if (tid < S * a.width)
-        fv_resident_sweeps<T, ML, S>(a.rec + (int64_t)s0 * a.width * PL, ns, a.width, a.group, xs, a.cap + 2, buf, bars,
-                                     groups, a.push, err);
-    __syncthreads();
+    cta.sweeps(err);
     fv_cluster_arrive();  // a CTA leaves only when no other can still push into its halo
-    if (!rs.group) {
-#pragma unroll 8
-        for (int k = tid; k < nr; k += nt) z[__ldg(&rows[k])] = xs[k];
-    } else {  // rows of a batch's converged problems keep their value
-        for (int k = tid; k < nr; k += nt) {
-            const int32_t i = __ldg(&rows[k]);
-            if (!rs.done[(int64_t)__ldg(&rs.group[i]) * rs.stride]) z[i] = xs[k];
-        }
-    }
+    cta.store(z, rs);
     fv_cluster_wait();
 }
 
-template <typename F>
-auto res_dispatch(int ml, int sets, F &&f) {
-    auto by_sets = [&](auto M) {
-        if (sets == 4) return f(M, std::integral_constant<int, 4>());
-        if (sets == 2) return f(M, std::integral_constant<int, 2>());
-        return f(M, std::integral_constant<int, 1>());
-    };
-    if (ml == 3) return by_sets(std::integral_constant<int, 3>());
-    if (ml == 4) return by_sets(std::integral_constant<int, 4>());
-    return by_sets(std::integral_constant<int, 6>());
-}
-
-// Bytes of a record, steps per copy and shared memory of a CTA.
+// Bytes of a record, steps per copy.
 size_t res_rec_bytes(int ml, size_t tb) {
-    return res_dispatch(ml, 1, [&](auto M, auto) {
+    return fv_res_dispatch(ml, 1, [&](auto M, auto) {
         return tb == 8 ? sizeof(fv_res_rec<double, M()>) : sizeof(fv_res_rec<float, M()>);
     });
 }
-int res_group(int ml, int width, int sets, size_t tb) {
-    int g = sets;  // a multiple of the thread sets
-    while (g < 16 && (size_t)(2 * g * width) * res_rec_bytes(ml, tb) <= (size_t)kResGroupBytes) g *= 2;
+int res_group(const fv_resident *p, size_t tb) {
+    int g = p->sets;  // a multiple of the thread sets
+    while (g < 16 && (size_t)(2 * g * p->width) * res_rec_bytes(p->ml, tb) <= (size_t)kResGroupBytes) g *= 2;
     return g;
 }
-size_t res_smem_bytes(const fv_resident *p, size_t tb) {
-    return (size_t)kResBuffers * res_group(p->ml, p->width, p->sets, tb) * p->width * res_rec_bytes(p->ml, tb) +
-           (size_t)(p->cap + 2 + p->halo) * tb;
-}
-constexpr int kResThreads = 512;  // enough to load and store the vector; the sweeps use sets * width of them
 
-cudaLaunchConfig_t res_config(int C, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kResThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    at->id = cudaLaunchAttributeClusterDimension;
-    at->val.clusterDim.x = C;
-    at->val.clusterDim.y = at->val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cfg;
-}
-
-// Sets an apply kernel's launch attributes; false when the GPU cannot run a cluster of this shape.
 template <typename T>
 bool res_launchable(const fv_resident *p) {
-    const size_t smem = res_smem_bytes(p, sizeof(T));
-    if (smem > kResSmem) return false;
-    return res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
-        auto *k = k_resident_apply<T, M(), S()>;
-        cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = res_config(p->C, smem, nullptr, &at);
-        int nc = 0;
-        const bool ok =
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess && nc >= 1;
-        if (!ok) cudaGetLastError();
-        return ok;
+    return fv_res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
+        return fv_res_launchable(k_resident_apply<T, M(), S()>, p->C, fv_resident_smem(p, sizeof(T)));
     });
 }
 
@@ -462,6 +385,26 @@ struct Layout {
 };
 
 }  // namespace
+
+size_t fv_resident_smem(const fv_resident *p, size_t tb) {
+    return (size_t)kResBuffers * res_group(p, tb) * p->width * res_rec_bytes(p->ml, tb) +
+           (size_t)(p->cap + 2 + p->halo) * tb;
+}
+
+fv_res_args fv_resident_args(const fv_resident *p, const void *rec, size_t tb) {
+    fv_res_args a;
+    a.rec = (const uint4 *)rec;
+    a.push = p->push;
+    a.step_ptr = p->step_ptr;
+    a.cta_ptr = p->cta_ptr;
+    a.rows = p->nat ? p->nat : p->rows;
+    a.C = p->C;
+    a.cap = p->cap;
+    a.halo = p->halo;
+    a.width = p->width;
+    a.group = res_group(p, tb);
+    return a;
+}
 
 void fv_resident_free(fv_resident *p) {
     if (!p) return;
@@ -492,6 +435,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     if (!p) return FV_ERR_ALLOC;
     p->C = C;
     p->width = width;
+    p->sorted = s.sorted;
     p->sets = sets;
     p->ml = s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6;
     ResPattern a;
@@ -628,7 +572,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
 template <typename T>
 cudaError_t fv_resident_records(const fv_resident *p, const fv_resident_src &s, bool unit_fwd, const T *l_val,
                                 const T *u_val, const T *dinv, void *rec, cudaStream_t st) {
-    res_dispatch(p->ml, 1, [&](auto M, auto) {
+    fv_res_dispatch(p->ml, 1, [&](auto M, auto) {
         fv_note_launch(), k_res_records<T, M()><<<(unsigned)((p->nslots + 255) / 256), 256, 0, st>>>(
                               *p, s.n, unit_fwd, s.l_ptr, s.u_ptr, l_val, u_val, dinv, (uint4 *)rec);
         return 0;
@@ -639,21 +583,12 @@ cudaError_t fv_resident_records(const fv_resident *p, const fv_resident_src &s, 
 template <typename T>
 cudaError_t fv_resident_apply(const fv_resident *p, const void *rec, const T *r, T *z, const int *skip,
                               const fv_row_skip &rs, int *err, cudaStream_t st) {
-    return res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
-        ResArgs a;
-        a.rec = (const uint4 *)rec;
-        a.step_ptr = p->step_ptr;
-        a.push = p->push;
-        a.cta_ptr = p->cta_ptr;
-        a.rows = p->nat ? p->nat : p->rows;
-        a.cap = p->cap;
-        a.halo = p->halo;
-        a.width = p->width;
-        a.group = res_group(p->ml, p->width, p->sets, sizeof(T));
+    return fv_res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
         cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = res_config(p->C, res_smem_bytes(p, sizeof(T)), st, &at);
+        const cudaLaunchConfig_t cfg = fv_res_config(p->C, fv_resident_smem(p, sizeof(T)), st, &at);
         fv_note_launch();
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_resident_apply<T, M(), S()>, a, r, z, skip, rs, err);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_resident_apply<T, M(), S()>,
+                                                 fv_resident_args(p, rec, sizeof(T)), r, z, skip, rs, err);
         return e == cudaSuccess ? cudaGetLastError() : e;
     });
 }

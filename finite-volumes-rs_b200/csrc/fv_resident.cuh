@@ -25,6 +25,8 @@
 // waits on anything unfinished.  Every wait is bounded in time.
 #pragma once
 
+#include <type_traits>
+
 #include "fv_internal.cuh"
 
 // One row of a sweep: factor values, 1/diagonal (1 where the diagonal is a
@@ -66,6 +68,7 @@ struct fv_resident {
     int32_t cap = 0;               // most rows of a CTA
     int32_t halo = 0;              // most halo slots of a CTA
     int64_t nslots = 0;            // slots of all steps
+    bool sorted = false;           // rows sorted by forward level
     int32_t *cta_ptr = nullptr;    // [C + 1] first entry of a CTA in `rows`
     int32_t *rows = nullptr;       // slot k of CTA c holds row rows[cta_ptr[c] + k]
     int32_t *nat = nullptr;        // the same rows in the caller's numbering (null: no permutation)
@@ -286,6 +289,130 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
     }
     if (S > 1 && set == 0 && nsteps > 0) wait_prev();  // the last step's arrivals are met
     groups = g0 + ng;
+}
+
+// What the kernels of a plan take.
+struct fv_res_args {
+    const uint4 *rec;
+    const uint32_t *push;
+    const int32_t *step_ptr, *cta_ptr, *rows;  // rows: in the caller's numbering
+    int C, cap, halo, width, group;
+};
+fv_res_args fv_resident_args(const fv_resident *p, const void *rec, size_t value_bytes);
+// Dynamic shared memory of a CTA for values of this size; the kernels run
+// kResThreads threads per CTA (enough to load and store the vector; the sweeps
+// use sets * width of them) as one cluster of at least p->C CTAs; further CTAs
+// hold no rows.
+size_t fv_resident_smem(const fv_resident *p, size_t value_bytes);
+constexpr int kResThreads = 512;
+
+// A CTA's part of a plan: its shared memory and its rows.
+template <typename T, int ML, int S>
+struct fv_res_cta {
+    static constexpr int PL = (int)(sizeof(fv_res_rec<T, ML>) / 16);
+    const fv_res_args &a;
+    uint4 *buf;
+    T *xs;
+    unsigned long long *bars;
+    const int32_t *rows;
+    const uint4 *rec;
+    int nr, ns;
+    unsigned groups = 0;
+
+    // smem: fv_resident_smem bytes; bars: kResBuffers mbarriers.  A cluster
+    // barrier has to follow before the first sweeps.
+    __device__ __forceinline__ fv_res_cta(const fv_res_args &args, unsigned char *smem, unsigned long long *mbar)
+        : a(args), buf(reinterpret_cast<uint4 *>(smem)), bars(mbar) {
+        xs = reinterpret_cast<T *>(buf + kResBuffers * a.group * a.width * PL);
+        const unsigned c = fv_cluster_rank();
+        const bool mine = c < (unsigned)a.C;
+        const int r0 = mine ? a.cta_ptr[c] : 0, s0 = mine ? a.step_ptr[c] : 0;
+        nr = mine ? a.cta_ptr[c + 1] - r0 : 0;
+        ns = mine ? a.step_ptr[c + 1] - s0 : 0;
+        rows = a.rows + r0;
+        rec = a.rec + (int64_t)s0 * a.width * PL;
+        if (threadIdx.x == 0) {
+            for (int b = 0; b < kResBuffers; ++b)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&bars[b])));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        if (threadIdx.x < 2) xs[a.cap + threadIdx.x] = T(0);
+        reset_halo();
+    }
+    // The halo's slots wait for values again: after the sweeps have read them,
+    // and with a cluster barrier before the next ones push.
+    __device__ __forceinline__ void reset_halo() {
+        for (int k = threadIdx.x; k < a.halo; k += kResThreads) xs[a.cap + 2 + k] = fv_sentinel(T(0));
+    }
+    // (k0: addresses are formed at each call; hoisted out of a solver's loop they would spill)
+    __device__ __forceinline__ void load(const T *r) {
+        int k0 = threadIdx.x;
+        asm volatile("" : "+r"(k0));
+#pragma unroll 8
+        for (int k = k0; k < nr; k += kResThreads) xs[k] = __ldcg(&r[__ldg(&rows[k])]);
+    }
+    __device__ __forceinline__ void store(T *z, const fv_row_skip &rs) {
+        int k0 = threadIdx.x;
+        asm volatile("" : "+r"(k0));
+        if (!rs.group) {
+#pragma unroll 8
+            for (int k = k0; k < nr; k += kResThreads) z[__ldg(&rows[k])] = xs[k];
+        } else {  // rows of a batch's converged problems keep their value
+            for (int k = k0; k < nr; k += kResThreads) {
+                const int32_t i = __ldg(&rows[k]);
+                if (!rs.done[(int64_t)__ldg(&rs.group[i]) * rs.stride]) z[i] = xs[k];
+            }
+        }
+    }
+    // Between load and store: the block is synchronised before and after.
+    __device__ __forceinline__ void sweeps(int *err) {
+        __syncthreads();
+        if ((int)threadIdx.x < S * a.width)
+            fv_resident_sweeps<T, ML, S>(rec, ns, a.width, a.group, xs, a.cap + 2, buf, bars, groups, a.push, err);
+        __syncthreads();
+    }
+};
+
+template <typename F>
+auto fv_res_dispatch(int ml, int sets, F &&f) {
+    auto by_sets = [&](auto M) {
+        if (sets == 4) return f(M, std::integral_constant<int, 4>());
+        if (sets == 2) return f(M, std::integral_constant<int, 2>());
+        return f(M, std::integral_constant<int, 1>());
+    };
+    if (ml == 3) return by_sets(std::integral_constant<int, 3>());
+    if (ml == 4) return by_sets(std::integral_constant<int, 4>());
+    return by_sets(std::integral_constant<int, 6>());
+}
+
+// Launch configuration of a plan's kernels on one cluster of C CTAs (at: storage for its attribute).
+inline cudaLaunchConfig_t fv_res_config(int C, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kResThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = C;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Sets a kernel's launch attributes; false when the GPU cannot run such a cluster of it.
+template <class K>
+bool fv_res_launchable(K *k, int C, size_t smem) {
+    if (smem > kResSmem) return false;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = fv_res_config(C, smem, nullptr, &at);
+    int nc = 0;
+    const bool ok =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess && nc >= 1;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 // The symbolic side of a factor a plan is built from (all arrays on the device).

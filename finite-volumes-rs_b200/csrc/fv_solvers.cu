@@ -20,12 +20,14 @@
 #include <vector>
 
 #include "fv_internal.cuh"
+#include "fv_resident.cuh"
 
 struct fv_symbolic;
 struct fv_precond;
 fv_status fv_precond_apply_dev(fv_precond *P, const double *r, double *z, cudaStream_t st, const int *skip,
                                const fv_row_skip *rskip);
 fv_status fv_precond_check_error(fv_precond *P, cudaStream_t st);
+const fv_resident *fv_precond_resident(const fv_precond *P, const void **rec, int **err);
 void fv_symbolic_free(fv_symbolic *s);
 
 // ------------------------------------------------------------------ CSR API
@@ -456,6 +458,385 @@ __global__ void k_bi_finish(int64_t n, double *__restrict__ x, const double *__r
 
 }  // namespace
 
+// ------------------------------------------------------------------ resident solves
+// Small systems: the cluster that holds the preconditioner's sweeps
+// (fv_resident.cuh) runs whole iterations, so an iteration costs no launches
+// and its reductions a cluster barrier (0.3 us) instead of a kernel each.  What
+// bounds the separate kernels at these sizes is latency: the four vector
+// kernels of a CG iteration take 16-23 us on 2,048-131,072 rows, their launches'
+// gaps about 5 us more.  Where the line to the separate kernels lies is said at
+// loop_resident.
+//
+// Same bits as the kernels above: the reductions keep their shape.  Virtual
+// block b of the G blocks of fv_reduce_grid sums the same elements in the same
+// threads' order with the same shuffle trees; its partial is pushed to every
+// CTA, and every CTA sums the partials as the last block does.
+namespace {
+
+constexpr int kRsMaxBlocks = 80;        // reduction blocks (75,000 rows)
+constexpr int kRsMaxPerHalf = 4;        // of them per 256 threads of a CTA
+constexpr int64_t kRsIterations = 256;  // iterations per launch (the host looks in between)
+
+// The solve's scalars, kept by every CTA in its shared memory (thread 0 updates
+// them after a reduction): held in registers they would make the sweeps spill.
+struct RsScalars {
+    double tol, rtol, bnorm, init_res, error, rz, rho, alpha, omega, beta;
+    int64_t iter, max_it;
+    int done, restart, restarts, finish_h, breakdown, lead;
+};
+struct RsShared {
+    double part[2][2][kRsMaxBlocks];         // [alternating][value][virtual block]
+    double wsum[2][kRsMaxPerHalf][2][8];     // [half][its block][value][warp]
+    double fin[2][8];
+    RsScalars sc;
+    int turn;
+};
+
+// One system's arrays.
+struct RsSystem {
+    int64_t n;
+    int G, C;
+    const int32_t *ptr, *col;
+    const double *val;
+    double *x, *r;
+    SolverState *S;
+    int *err;
+};
+
+// A row's entries and the vector's values at its columns (a vector this kernel
+// writes: no read-only loads of it), and their sum in entry order.
+struct RsRow {
+    static constexpr int E = 5;
+    double av[E], xv[E];
+    int k0, len;
+    __device__ __forceinline__ void load(const RsSystem &q, const double *x, int64_t i) {
+        k0 = __ldg(&q.ptr[i]);
+        len = __ldg(&q.ptr[i + 1]) - k0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            av[e] = 0.0;
+            xv[e] = 0.0;
+            if (e < len) {
+                av[e] = __ldg(&q.val[k0 + e]);
+                xv[e] = __ldcg(&x[__ldg(&q.col[k0 + e])]);
+            }
+        }
+    }
+    __device__ __forceinline__ double dot(const RsSystem &q, const double *x) const {
+        double s = 0.0;
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (e < len) s += av[e] * xv[e];
+        for (int k = k0 + E; k < k0 + len; ++k) s += __ldg(&q.val[k]) * __ldcg(&x[__ldg(&q.col[k])]);
+        return s;
+    }
+};
+
+// fv_block_reduce's second stage over 8 warps, in one thread (the absent warps add 0.0).
+__device__ __forceinline__ double rs_sum8(const double *v) {
+    return (((v[0] + 0.0) + (v[4] + 0.0)) + ((v[2] + 0.0) + (v[6] + 0.0))) +
+           (((v[1] + 0.0) + (v[5] + 0.0)) + ((v[3] + 0.0) + (v[7] + 0.0)));
+}
+
+__device__ __forceinline__ void rs_barrier() {
+    fv_cluster_arrive();
+    fv_cluster_wait();
+}
+
+// The at most 4 rows of a thread of virtual block b in row order: load(i,
+// state), then use(i, state).  (Two or four rows' loads in flight at once need
+// registers the kernel does not have: the spills, with most of the L1 given to
+// shared memory, cost more than the latency they hide.)
+template <class St, class Load, class Use>
+__device__ __forceinline__ void rs_rows(const RsSystem &q, int b, int t, Load load, Use use) {
+    asm volatile("" : "+r"(t));  // addresses are formed here: hoisted out of the iteration loop they would spill
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const int64_t i = ((int64_t)b + (int64_t)k * q.G) * RB + t;
+        if (i >= q.n) return;
+        St st;
+        load(i, st);
+        use(i, st);
+    }
+}
+
+// use(i, state, v) for every row i of this CTA's virtual blocks, then epi(the
+// sums of v over all rows) in thread 0, which updates sh->sc.  Contains a
+// cluster barrier after the rows; the block is synchronised at the end.
+template <int NV, class St, class Load, class Use, class Epi>
+__device__ __forceinline__ void rs_reduce(const RsSystem &q, RsShared *sh, Load load, Use use, Epi epi) {
+    const int tid = threadIdx.x, half = tid >> 8, t = tid & 255, w = t >> 5, lane = tid & 31;
+    const int b0 = 2 * (int)fv_cluster_rank() + half;
+    int nb = 0;
+    for (int b = b0; b < q.G; b += 2 * q.C, ++nb) {
+        double v[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = 0.0;
+        rs_rows<St>(q, b, t, load, [&](int64_t i, St &st) { use(i, st, v); });
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+            if (lane == 0) sh->wsum[half][nb][k][w] = v[k];
+        }
+    }
+    __syncthreads();
+    const int turn = sh->turn;
+    if (t < nb * NV) {
+        const int m = t / NV, k = t - m * NV;
+        const double s = rs_sum8(sh->wsum[half][m][k]);
+        const unsigned a = (unsigned)__cvta_generic_to_shared(&sh->part[turn][k][b0 + 2 * q.C * m]);
+        for (int c = 0; c < q.C; ++c)
+            asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(fv_mapa(a, c)), "d"(s) : "memory");
+    }
+    rs_barrier();
+    if (tid < RB) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            double s = 0.0;
+            for (int b = tid; b < q.G; b += RB) s += sh->part[turn][k][b];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0) sh->fin[k][w] = s;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double tot[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) tot[k] = rs_sum8(sh->fin[k]);
+        sh->turn = turn ^ 1;
+        epi(sh->sc, tot);
+    }
+    __syncthreads();
+}
+
+// Rows of this CTA's virtual blocks, without a reduction.
+template <class St, class Load, class Use>
+__device__ __forceinline__ void rs_each(const RsSystem &q, Load load, Use use) {
+    const int half = (int)threadIdx.x >> 8, t = threadIdx.x & 255;
+    for (int b = 2 * (int)fv_cluster_rank() + half; b < q.G; b += 2 * q.C) rs_rows<St>(q, b, t, load, use);
+}
+
+struct Rs2 {
+    double a, b;
+};
+struct Rs4 {
+    double a, b, c, d;
+};
+struct Rs6 {
+    double x, y, z, s, t, h;
+};
+
+// z = M^-1 r; r was written before the last cluster barrier, z is visible after this one.
+template <int ML, int SETS>
+__device__ __forceinline__ void rs_apply(fv_res_cta<double, ML, SETS> &cta, const double *r, double *z, int *err) {
+    cta.load(r);
+    cta.sweeps(err);
+    cta.store(z, fv_row_skip{});
+    cta.reset_halo();
+    rs_barrier();
+}
+
+// Shared memory of a resident solve: the reductions' part, then the sweeps'.
+constexpr size_t kRsBytes = (sizeof(RsShared) + 127) / 128 * 128;
+
+__device__ __forceinline__ void rs_open(RsShared *sh, const SolverState *S) {
+    if (threadIdx.x == 0) {
+        sh->sc = RsScalars{S->tol,   S->rtol, S->bnorm, S->init_res, S->error, S->rz,      S->rho,
+                           S->alpha, S->omega, S->beta, S->iter,     S->max_it, 0,         0,
+                           S->restarts, 0,    S->breakdown, fv_cluster_rank() == 0 ? 1 : 0};
+        sh->turn = 0;
+    }
+    rs_barrier();  // and no push before every CTA's halo is reset
+    __syncthreads();
+}
+__device__ __forceinline__ void rs_close(const RsShared *sh, SolverState *S) {
+    if (threadIdx.x != 0 || !sh->sc.lead) return;
+    const RsScalars &c = sh->sc;
+    S->error = c.error;
+    S->rz = c.rz;
+    S->rho = c.rho;
+    S->alpha = c.alpha;
+    S->omega = c.omega;
+    S->beta = c.beta;
+    S->iter = c.iter;
+    S->restart = c.restart;
+    S->restarts = c.restarts;
+    S->finish_h = c.finish_h;
+    S->breakdown = c.breakdown;
+    S->done = c.done;
+}
+
+// CG iterations from (x, r, p, rz) as k_cg_spmv, k_cg_update, the apply, k_cg_rz and k_cg_p run them.
+template <int ML, int SETS>
+__global__ void __launch_bounds__(kResThreads, 1) k_resident_cg(const __grid_constant__ fv_res_args a,
+                                                                const __grid_constant__ RsSystem q, double *z, double *p,
+                                                                double *ap) {
+    SolverState *S = q.S;
+    if (S->done) return;
+    extern __shared__ __align__(128) unsigned char rs_smem[];
+    __shared__ unsigned long long bars[kResBuffers];
+    RsShared *sh = reinterpret_cast<RsShared *>(rs_smem);
+    fv_res_cta<double, ML, SETS> cta(a, rs_smem + kRsBytes, bars);
+    rs_open(sh, S);
+    double *x = q.x, *r = q.r, *hist = S->hist;
+    for (int64_t it = 0; it < kRsIterations; ++it) {
+        rs_reduce<1, RsRow>(q, sh, [&](int64_t i, RsRow &w) { w.load(q, p, i); },
+                               [&](int64_t i, RsRow &w, double (&v)[1]) {
+                                   const double y = w.dot(q, p);
+                                   ap[i] = y;
+                                   v[0] += p[i] * y;
+                               },
+                               [](RsScalars &c, const double *t) { c.alpha = c.rz / t[0]; });
+        const double alpha = sh->sc.alpha;
+        rs_reduce<1, Rs4>(q, sh, [&](int64_t i, Rs4 &w) { w = Rs4{x[i], p[i], r[i], ap[i]}; },
+                             [&](int64_t i, Rs4 &w, double (&v)[1]) {
+                                 x[i] = w.a + w.b * alpha;
+                                 const double ri = w.c - w.d * alpha;
+                                 r[i] = ri;
+                                 v[0] += ri * ri;
+                             },
+                             [&](RsScalars &c, const double *t) {
+                                 c.error = sqrt(t[0]) / c.bnorm;
+                                 if ((c.error < c.tol) || (c.error / c.init_res < c.rtol)) {
+                                     if (c.lead) hist[c.iter] = c.error;
+                                     c.iter += 1;
+                                     c.done = 1;
+                                 }
+                                 if (bad(c.alpha)) c.breakdown = 1;
+                             });
+        if (sh->sc.done) break;
+        rs_apply(cta, r, z, q.err);
+        rs_reduce<1, Rs2>(q, sh, [&](int64_t i, Rs2 &w) { w = Rs2{r[i], __ldcg(&z[i])}; },
+                             [&](int64_t, Rs2 &w, double (&v)[1]) { v[0] += w.a * w.b; },
+                             [&](RsScalars &c, const double *t) {
+                                 c.beta = t[0] / c.rz;
+                                 c.rz = t[0];
+                                 if (c.lead) hist[c.iter] = c.error;
+                                 c.iter += 1;
+                                 if (!(c.error > c.tol) || c.iter > c.max_it) c.done = 1;
+                             });
+        if (sh->sc.done) break;
+        const double beta = sh->sc.beta;
+        rs_each<Rs2>(q, [&](int64_t i, Rs2 &w) { w = Rs2{__ldcg(&z[i]), p[i]}; },
+                        [&](int64_t i, Rs2 &w) { p[i] = w.a + w.b * beta; });
+        rs_barrier();
+    }
+    rs_close(sh, S);
+}
+
+// BiCGStab iterations from (x, r, rh, p, rho) as the k_bi_* kernels run them.
+struct RsBiVecs {
+    double *rh, *p, *y, *v, *s, *z, *t;
+};
+template <int ML, int SETS>
+__global__ void __launch_bounds__(kResThreads, 1) k_resident_bicgstab(const __grid_constant__ fv_res_args a,
+                                                                      const __grid_constant__ RsSystem q,
+                                                                      const __grid_constant__ RsBiVecs b) {
+    SolverState *S = q.S;
+    if (S->done) return;
+    extern __shared__ __align__(128) unsigned char rs_smem[];
+    __shared__ unsigned long long bars[kResBuffers];
+    RsShared *sh = reinterpret_cast<RsShared *>(rs_smem);
+    fv_res_cta<double, ML, SETS> cta(a, rs_smem + kRsBytes, bars);
+    rs_open(sh, S);
+    double *hist = S->hist;
+    for (int64_t it = 0; it < kRsIterations; ++it) {
+        rs_apply(cta, b.p, b.y, q.err);
+        rs_reduce<1, RsRow>(q, sh, [&](int64_t i, RsRow &w) { w.load(q, b.y, i); },
+                               [&](int64_t i, RsRow &w, double (&v)[1]) {
+                                   const double vi = w.dot(q, b.y);
+                                   b.v[i] = vi;
+                                   v[0] += b.rh[i] * vi;
+                               },
+                               [](RsScalars &c, const double *t) { c.alpha = c.rho / t[0]; });
+        {
+            const double alpha = sh->sc.alpha;
+            rs_reduce<1, Rs2>(q, sh, [&](int64_t i, Rs2 &w) { w = Rs2{q.r[i], b.v[i]}; },
+                                 [&](int64_t i, Rs2 &w, double (&v)[1]) {
+                                     const double si = w.a - w.b * alpha;
+                                     b.s[i] = si;
+                                     v[0] += si * si;
+                                 },
+                                 [&](RsScalars &c, const double *t) {
+                                     const double sn = sqrt(t[0]) / c.bnorm;
+                                     if ((sn < c.tol) || (sn / c.init_res < c.rtol)) {
+                                         c.error = sn;
+                                         if (c.lead) hist[c.iter] = sn;
+                                         c.finish_h = 1;
+                                         c.iter += 1;
+                                         c.done = 1;
+                                     }
+                                     if (bad(c.alpha)) c.breakdown = 1;
+                                 });
+        }
+        if (sh->sc.done) break;
+        rs_apply(cta, b.s, b.z, q.err);
+        rs_reduce<2, RsRow>(q, sh, [&](int64_t i, RsRow &w) { w.load(q, b.z, i); },
+                               [&](int64_t i, RsRow &w, double (&v)[2]) {
+                                   const double ti = w.dot(q, b.z);
+                                   b.t[i] = ti;
+                                   v[0] += ti * b.s[i];
+                                   v[1] += ti * ti;
+                               },
+                               [](RsScalars &c, const double *t) { c.omega = t[0] / t[1]; });
+        {
+            const double alpha = sh->sc.alpha, omega = sh->sc.omega;
+            rs_reduce<2, Rs6>(q, sh, [&](int64_t i, Rs6 &w) {
+                                     w = Rs6{q.x[i], __ldcg(&b.y[i]), __ldcg(&b.z[i]), b.s[i], b.t[i], b.rh[i]};
+                                 },
+                                 [&](int64_t i, Rs6 &w, double (&v)[2]) {
+                                     const double h = w.x + w.y * alpha;
+                                     q.x[i] = h + w.z * omega;
+                                     const double ri = w.s - w.t * omega;
+                                     q.r[i] = ri;
+                                     v[0] += ri * ri;
+                                     v[1] += w.h * ri;
+                                 },
+                                 [&](RsScalars &c, const double *t) {
+                                     const double rn = sqrt(t[0]) / c.bnorm;
+                                     if ((rn < c.tol) || (rn / c.init_res < c.rtol)) {
+                                         c.error = rn;
+                                         if (c.lead) hist[c.iter] = rn;
+                                         c.iter += 1;
+                                         c.done = 1;
+                                         return;
+                                     }
+                                     c.beta = (t[1] / c.rho) * (c.alpha / c.omega);
+                                     c.rho = t[1];
+                                     if (fabs(c.rho) > (1e-15 * c.bnorm)) {
+                                         c.restart = 0;
+                                     } else {
+                                         c.restart = 1;
+                                         c.restarts += 1;
+                                         c.rho = t[0];  // rh = r, then rh.r
+                                     }
+                                     if (bad(c.omega) || bad(c.beta)) c.breakdown = 1;
+                                     c.error = rn / c.bnorm;  // the loop guard divides by |b| twice (:171)
+                                     if (c.lead) hist[c.iter] = c.error;
+                                     c.iter += 1;
+                                     if (!(c.error > c.tol) || c.iter > c.max_it) c.done = 1;
+                                 });
+        }
+        if (sh->sc.done) break;
+        if (sh->sc.restart) {
+            rs_each<double>(q, [&](int64_t i, double &w) { w = q.r[i]; }, [&](int64_t i, double &w) {
+                b.rh[i] = w;
+                b.p[i] = w;
+            });
+        } else {
+            const double omega = sh->sc.omega, beta = sh->sc.beta;
+            rs_each<Rs4>(q, [&](int64_t i, Rs4 &w) { w = Rs4{q.r[i], b.p[i], b.v[i], 0.0}; },
+                            [&](int64_t i, Rs4 &w) { b.p[i] = w.a + (w.b - w.c * omega) * beta; });
+        }
+        rs_barrier();
+    }
+    rs_close(sh, S);
+}
+
+}  // namespace
+
 extern "C" fv_status fv_spmv(const fv_csr *A, const double *x, double *y, void *stream) {
     if (!A || !x || !y || x == y) return FV_ERR_INVALID;
     if (A->nrows == 0) return FV_OK;
@@ -665,6 +1046,49 @@ fv_status loop_until_done(const Workspace &w, cudaStream_t st, Body body, Solver
     return s;
 }
 
+// Whole iterations in one kernel per kRsIterations (k_resident_cg /
+// k_resident_bicgstab) when the preconditioner's sweeps are resident; `used` says
+// whether they ran.  vecs: the solver's vectors after r, in the kernel's order.
+template <bool BICG>
+fv_status loop_resident(const Workspace &w, const fv_csr *A, fv_precond *P, double *x, double *r, int G,
+                        double *const *vecs, cudaStream_t st, SolverState &h, bool &used) {
+    used = false;
+    const void *rec = nullptr;
+    int *err = nullptr;
+    const fv_resident *plan = P ? fv_precond_resident(P, &rec, &err) : nullptr;
+    // Up to where whole iterations in one cluster beat kernels on all SMs, us per
+    // iteration (resident / kernels): CG natural 32,768 rows 95 / 102, 45,000
+    // 132 / 126; CG in box order 65,522 rows 47 / 55, 96,800 57 / 55; BiCGStab
+    // natural 48,000 rows 155 / 180, 82,944 223 / 177; 2,048 rows 32 / 49.
+    const int64_t most = BICG ? 50000 : plan && plan->sorted ? 75000 : 36000;
+    if (!plan || A->nrows > most) return FV_OK;
+    const size_t smem = kRsBytes + fv_resident_smem(plan, sizeof(double));
+    int L = plan->C;  // CTAs: those of the sweeps, and more where the vectors need them
+    while (L < kResMaxCta && G > 2 * L) L *= 2;
+    if ((G + 2 * L - 1) / (2 * L) > kRsMaxPerHalf || G > kRsMaxBlocks) return FV_OK;
+    RsSystem q{A->nrows, G, L, A->row_ptr, A->cols, A->vals, x, r, w.S, err};
+    return fv_res_dispatch(plan->ml, plan->sets, [&](auto M, auto S) -> fv_status {
+        const fv_res_args a = fv_resident_args(plan, rec, sizeof(double));
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = fv_res_config(L, smem, st, &at);
+        auto run = [&](auto *k, auto... args) -> fv_status {
+            if (!fv_res_launchable(k, L, smem)) return FV_OK;
+            used = true;
+            while (true) {
+                fv_note_launch();
+                FV_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, a, q, args...));
+                FV_TRY(read_state(w, h, st));
+                if (h.done) return FV_OK;
+            }
+        };
+        if constexpr (BICG)
+            return run(k_resident_bicgstab<M(), S()>,
+                       RsBiVecs{vecs[0], vecs[1], vecs[2], vecs[3], vecs[4], vecs[5], vecs[6]});
+        else
+            return run(k_resident_cg<M(), S()>, vecs[0], vecs[1], vecs[2]);
+    });
+}
+
 }  // namespace
 
 extern "C" fv_status fv_cg(const fv_csr *A, fv_precond *P, const double *b, double *x, fv_solver_options opt,
@@ -700,7 +1124,10 @@ extern "C" fv_status fv_cg(const fv_csr *A, fv_precond *P, const double *b, doub
         FV_CUDA_TRY(cudaGetLastError());
         return FV_OK;
     };
-    if (s == FV_OK) s = loop_until_done(w, st, body, h);
+    bool resident = false;
+    double *const vecs[3] = {z, p, ap};
+    if (s == FV_OK) s = loop_resident<false>(w, A, P, x, r, G, vecs, st, h, resident);
+    if (s == FV_OK && !resident) s = loop_until_done(w, st, body, h);
     cudaEventRecord(e1, st);
     if (s == FV_OK) s = read_state(w, h, st);
     float ms = 0.f;
@@ -747,7 +1174,10 @@ extern "C" fv_status fv_bicgstab(const fv_csr *A, fv_precond *P, const double *b
         FV_CUDA_TRY(cudaGetLastError());
         return FV_OK;
     };
-    s = loop_until_done(w, st, body, h);
+    bool resident = false;
+    double *const vecs[7] = {rh, p, y, v, s_, z, t};
+    s = loop_resident<true>(w, A, P, x, r, G, vecs, st, h, resident);
+    if (s == FV_OK && !resident) s = loop_until_done(w, st, body, h);
     fv_note_launch(), k_bi_finish<<<G, RB, 0, st>>>(n, x, y, S);
     cudaEventRecord(e1, st);
     if (s == FV_OK) s = read_state(w, h, st);
@@ -792,7 +1222,7 @@ extern "C" fv_status fv_bicgstab_host(const fv_csr *A, fv_precond *P, const doub
 // sized device array that is created when this file's CUDA module is loaded on
 // a device (under lazy module loading, the CUDA 12 default: at the first
 // launch from, or symbol lookup in, this module on that device).  It launches
-// the same kernels in the same order as fv_cg, so its results are the same bits.
+// the iteration's kernels one by one; the results are fv_cg's bits.
 namespace {
 constexpr int64_t kNoAllocMaxRows = FV_NOALLOC_MAX_ROWS;
 constexpr int64_t kNoAllocMaxHist = FV_NOALLOC_MAX_ITERATIONS + 3;

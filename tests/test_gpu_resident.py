@@ -100,3 +100,31 @@ def test_resident_in_a_batch(fv, precision):
         info = BatchCG(A, mb.cell_offsets, 256).solve(P, b, x, precision=precision, solver="bicgstab")
         out.append((x.numpy(), info["iterations"].tolist()))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("dim,side,ordering", [(2, 2, None), (2, 22, None), (2, 23, "boxes"), (2, 130, None),
+                                               (2, 190, "boxes"), (3, 2, None), (3, 7, "boxes"), (3, 20, None)])
+def test_resident_solve_equals_kernels(fv, dim, side, ordering):
+    """Whole iterations in one cluster against the iteration's kernels (an explicit
+    schedule takes them): the same bits, the same history, at row counts around
+    the reduction blocks (1,024 rows), the cluster sizes and the limits, with the
+    iteration limit reached in the middle and past the iterations of one launch."""
+    case = diffusion_2d(fv, side, seed=63) if dim == 2 else convdiff_3d(fv, side, seed=64)
+    cls = fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper
+    solve = fv.conjugate_gradient if dim == 2 else fv.bi_conjugate_gradient_stab
+    A, b = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    P = cls.from_matrix(A, 0, ordering=ordering)
+    Q = cls.from_matrix(A, 0, ordering=ordering)
+    Q.schedule(1)
+    n = case["mesh"].n_cells
+    x0 = np.random.default_rng(9).standard_normal(n) * 1e-3
+    for tol, limit in ((1e-8, 2000), (0.0, 7), (1e-300, 300)):
+        got = []
+        for M in (P, Q):
+            x = fv.DistributedVector(x0)
+            info = solve(x, A, b, M, None, fv.LinearSolverOptions(tol, tol, limit))
+            got.append((x.numpy(), np.array(info.history), info.iterations, info.restarts, info.status,
+                        info.initial_residual, info.final_residual))
+        assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
+        assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
+        assert np.array_equal(got[0][2:], got[1][2:], equal_nan=True)
