@@ -209,6 +209,18 @@ __device__ __forceinline__ unsigned fv_pack_value(float v) {
     return b == FV_SENTINEL_U32 ? 0x7FC00000u : b;
 }
 
+// Reads *p; whether it holds a produced value.
+__device__ __forceinline__ bool fv_slot_ready(const double *p, double &v) {
+    unsigned long long b = fv_ld_relaxed_u64(p);
+    v = __longlong_as_double((long long)b);
+    return b != FV_SENTINEL_U64;
+}
+__device__ __forceinline__ bool fv_slot_ready(const float *p, float &v) {
+    unsigned b = fv_ld_relaxed_u32(p);
+    v = __uint_as_float(b);
+    return b != FV_SENTINEL_U32;
+}
+
 // Wait until *p holds a produced value.  Gives up (returns NaN and raises
 // FV_DEV_TIMEOUT in *err) after FV_WAIT_LIMIT_NS, or as soon as another
 // thread has raised an error, so one failure cannot cascade into long waits.

@@ -108,14 +108,24 @@ __global__ void k_res_bins(int64_t n, const double4 *__restrict__ cell, ResAxes 
     for (int k = threadIdx.x; k < 3 * kResBins; k += blockDim.x)
         if (cnt[k]) atomicAdd(&a->bin[k / kResBins][k % kResBins], cnt[k]);
 }
-// Equal numbers of rows per CTA along every axis (whole bins).  Three threads.
+// Equal numbers of rows per CTA along every axis (whole bins).  One warp per axis.
 __global__ void k_res_cuts(int64_t n, int C, ResAxes *a) {
-    const int d = threadIdx.x;
-    int64_t before = 0;
-    for (int k = 0; k < kResBins; ++k) {
-        const int32_t w = a->bin[d][k];
-        a->bin[d][k] = (int32_t)min((int64_t)C - 1, (2 * before + w) * C / (2 * n));
-        before += w;
+    const int d = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int per = kResBins / 32;
+    int32_t w[per], sum = 0;
+#pragma unroll
+    for (int k = 0; k < per; ++k) sum += w[k] = a->bin[d][lane * per + k];
+    int32_t before = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += t;
+    }
+    before -= sum;
+#pragma unroll
+    for (int k = 0; k < per; ++k) {
+        a->bin[d][lane * per + k] = (int32_t)min((int64_t)C - 1, (2 * (int64_t)before + w[k]) * C / (2 * n));
+        before += w[k];
     }
 }
 // The balanced candidate, and the rows of every (axis, CTA, level) of the slabs.
@@ -221,24 +231,24 @@ __global__ void k_res_keys(ResPattern a, const uint32_t *__restrict__ owner, uin
     }
 }
 
-// Readers of every item, steps of every key; a CTA's last key holds the empty
-// steps that make its number of steps a multiple of `sets`.
+// Readers of every item, steps of every key (but a CTA's last one, k_res_pad).
 __global__ void k_res_counts(int64_t items, const uint32_t *__restrict__ mask, int32_t *__restrict__ nread, int32_t nk,
-                             int32_t per_cta, const int32_t *__restrict__ first, int width, int sets,
+                             int32_t per_cta, const int32_t *__restrict__ first, int width,
                              int32_t *__restrict__ nstep) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= items) nread[i] = i < items ? __popc(mask[i]) : 0;
     if (i > nk) return;
-    auto steps = [&](int64_t k) { return (first[k + 1] - first[k] + width - 1) / width; };
-    if (i == nk) {
-        nstep[i] = 0;
-    } else if ((i + 1) % per_cta != 0) {
-        nstep[i] = steps(i);
-    } else {
-        int sum = 0;
-        for (int64_t k = i + 1 - per_cta; k < i; ++k) sum += steps(k);
-        nstep[i] = (sets - sum % sets) % sets;
-    }
+    if (i == nk) nstep[i] = 0;
+    else if ((i + 1) % per_cta != 0) nstep[i] = (first[i + 1] - first[i] + width - 1) / width;
+}
+// A CTA's last key holds the empty steps that make its number of steps a
+// multiple of `sets`.  One warp per CTA.
+__global__ void k_res_pad(int32_t per_cta, int sets, int32_t *__restrict__ nstep) {
+    const int64_t k0 = (int64_t)blockIdx.x * per_cta;
+    int sum = 0;
+    for (int k = threadIdx.x; k < per_cta - 1; k += 32) sum += nstep[k0 + k];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (threadIdx.x == 0) nstep[k0 + per_cta - 1] = (sets - sum % sets) % sets;
 }
 
 // Halo slots: an item read by CTA c takes the next free slot of c.
@@ -510,7 +520,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
             fv_note_launch(), k_res_axes_init<<<1, 256, 0, st>>>(ax);
             fv_note_launch(), k_res_extent<<<gs, 256, 0, st>>>(n, s.cell, ax);
             fv_note_launch(), k_res_bins<<<gs, 256, 0, st>>>(n, s.cell, ax);
-            fv_note_launch(), k_res_cuts<<<1, 3, 0, st>>>(n, C, ax);
+            fv_note_launch(), k_res_cuts<<<1, 96, 0, st>>>(n, C, ax);
         }
         fv_note_launch(), k_res_owner<<<grid(n), 256, 0, st>>>(n, C, a.nlev[0], s.fwd_order, s.fwd_level, lst, s.cell, ax,
                                                                owner, hist);
@@ -527,7 +537,8 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     sort(key, item, items, nk);
     fv_note_launch(), k_res_bounds<<<grid(items + 1), 256, 0, st>>>(items, (int32_t)nk, sorted, first);
     fv_note_launch(), k_res_counts<<<grid(cm), 256, 0, st>>>(items, mask, cnt, (int32_t)nk, a.keys(), first, width,
-                                                             sets, cnt2);
+                                                             cnt2);
+    fv_note_launch(), k_res_pad<<<C, 32, 0, st>>>(a.keys(), sets, cnt2);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(cubt, cub_bytes, cnt, poff, (int)(items + 1), st);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(cubt, cub_bytes, cnt2, soff, (int)(nk + 1), st);
     fv_note_launch(), k_res_halo<<<grid(items), 256, 0, st>>>(items, mask, poff, hc, hslot, a.keys(), C, soff,
