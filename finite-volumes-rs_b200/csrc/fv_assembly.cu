@@ -1152,7 +1152,7 @@ extern "C" fv_status fv_assemble(fv_mesh *m, const fv_terms_desc *terms, const f
         a->cols = m->cols;
         a->owns_pattern = false;
         a->mesh = m;
-        cudaError_t e = cudaMalloc(&a->vals, sizeof(double) * (a->nnz ? a->nnz : 1));
+        cudaError_t e = fv_block_alloc(&a->vals, sizeof(double) * (a->nnz ? a->nnz : 1));
         if (e != cudaSuccess) {
             delete a;
             fv_internal_set_cuda_error(e, "fv_assemble vals");

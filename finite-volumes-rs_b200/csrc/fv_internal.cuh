@@ -57,6 +57,18 @@ template <typename T>
 static inline cudaError_t fv_malloc_async(T **p, size_t bytes, cudaStream_t st) {
     return fv_malloc_async_raw(reinterpret_cast<void **>(p), bytes, st);
 }
+// Device memory of matrices and preconditioners (fv_pool.cu).  fv_block_alloc:
+// like cudaMalloc.  fv_blocks_free: the blocks of one object at once, null
+// entries allowed; fv_block_free: one block.  Both also take memory from
+// cudaMalloc, and memory from fv_block_alloc goes through them only.
+cudaError_t fv_block_alloc_raw(void **p, size_t bytes);
+template <typename T>
+static inline cudaError_t fv_block_alloc(T **p, size_t bytes) {
+    return fv_block_alloc_raw(reinterpret_cast<void **>(p), bytes);
+}
+void fv_blocks_free(void *const *blocks, int n);
+void fv_block_free(void *p);
+unsigned long long fv_current_context_id();  // 0 when unknown
 void fv_note_launch();
 void fv_note_launches(long long delta);  // graph replays add, captures (not run) subtract
 unsigned long long fv_launches_now();

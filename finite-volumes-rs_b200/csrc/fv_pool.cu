@@ -1,0 +1,164 @@
+// Device memory of matrices and preconditioners: freed blocks are kept for the
+// next object.
+//
+// A program that assembles, factorises and solves once per problem spent more
+// on cudaMalloc / cudaFree than on the factorisation: a block of a megabyte or
+// less costs 2-4 us each way, one of several megabytes 1-4 ms, because it is
+// mapped and unmapped every time (24,576 rows: 3-5 ms of an 8 ms solve).
+//
+// A block is handed out again only after the device has finished all work
+// submitted before it was freed: fv_blocks_free first allocates and frees 256
+// bytes, and that cudaFree waits for the device as every cudaFree of the blocks
+// did (measured: it returns when a kernel in flight on another, non-blocking
+// stream ends).  So a block from here may be used on any stream at once, like
+// memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per device, blocks
+// of at most kKeepBlock) and given back when an allocation fails.  Blocks belong
+// to the device, and to its context: when the context has been replaced
+// (cudaDeviceReset), what was kept is forgotten.
+#include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
+
+#include <map>
+#include <mutex>
+#include <unordered_map>
+
+#include "fv_internal.cuh"
+
+// Unique id of the calling thread's current context (cuCtxGetId, unique over
+// the process's life), or 0 when the driver does not provide it.
+unsigned long long fv_current_context_id() {
+    using GetCurrent = CUresult (*)(CUcontext *);
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = (GetCurrent)f;
+        f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = (GetId)f;
+        cudaGetLastError();
+    });
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
+}
+
+namespace {
+
+constexpr size_t kKeepBytes = 512u << 20, kKeepBlock = 64u << 20;
+
+struct Block {
+    size_t bytes;
+    int dev;
+    unsigned long long ctx;
+};
+struct Kept {
+    std::multimap<size_t, void *> by_size;
+    size_t bytes = 0;
+    unsigned long long ctx = 0;
+};
+std::mutex g_mu;
+std::unordered_map<void *, Block> g_live;  // blocks handed out that may be kept when freed
+Kept g_kept[64];
+
+// Everything kept on the current device goes back to the driver.
+void give_back(int dev) {
+    Kept &k = g_kept[dev];
+    for (auto &b : k.by_size) cudaFree(b.second);
+    k.by_size.clear();
+    k.bytes = 0;
+}
+
+}  // namespace
+
+cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
+    *p = nullptr;
+    int dev = -1;
+    const bool keep = bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    if (!keep) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation && dev >= 0 && dev < 64) {
+            std::lock_guard<std::mutex> g(g_mu);
+            cudaGetLastError();
+            give_back(dev);
+            e = cudaMalloc(p, bytes);
+        }
+        return e;
+    }
+    try {
+        const unsigned long long ctx = fv_current_context_id();
+        std::lock_guard<std::mutex> g(g_mu);
+        Kept &k = g_kept[dev];
+        if (k.ctx != ctx) {  // another context: its addresses mean nothing any more
+            k.by_size.clear();
+            k.bytes = 0;
+            k.ctx = ctx;
+        }
+        if (ctx != 0) {
+            auto it = k.by_size.lower_bound(bytes);
+            if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
+                g_live[it->second] = Block{it->first, dev, ctx};
+                *p = it->second;
+                k.bytes -= it->first;
+                k.by_size.erase(it);
+                return cudaSuccess;
+            }
+        }
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            give_back(dev);
+            e = cudaMalloc(p, bytes);
+        }
+        if (e == cudaSuccess && ctx != 0) g_live[*p] = Block{bytes, dev, ctx};
+        return e;
+    } catch (...) {  // host memory for the bookkeeping: plain memory then
+        return *p ? cudaSuccess : cudaMalloc(p, bytes);
+    }
+}
+
+void fv_block_free(void *p) {
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> g(g_mu);
+        g_live.erase(p);
+    }
+    cudaFree(p);
+}
+
+void fv_blocks_free(void *const *blocks, int n) {
+    int dev = -1;
+    void *fence = nullptr;
+    const bool idle = cudaGetDevice(&dev) == cudaSuccess && cudaMalloc(&fence, 256) == cudaSuccess &&
+                      cudaFree(fence) == cudaSuccess;  // waits for the device
+    if (!idle) cudaGetLastError();
+    for (int i = 0; i < n; ++i) {
+        if (!blocks[i]) continue;
+        bool kept = false;
+        if (idle) {
+            try {
+                std::lock_guard<std::mutex> g(g_mu);
+                auto it = g_live.find(blocks[i]);
+                if (it != g_live.end() && it->second.dev == dev) {
+                    const Block b = it->second;
+                    Kept &k = g_kept[b.dev];
+                    if (k.ctx == b.ctx && k.bytes + b.bytes <= kKeepBytes) {
+                        k.by_size.emplace(b.bytes, blocks[i]);
+                        k.bytes += b.bytes;
+                        g_live.erase(it);
+                        kept = true;
+                    }
+                }
+            } catch (...) {  // host memory for the bookkeeping: freed then
+            }
+        }
+        if (!kept) fv_block_free(blocks[i]);
+    }
+}

@@ -63,22 +63,13 @@ struct fv_symbolic {
 
 void fv_symbolic_free(fv_symbolic *s) {
     if (!s) return;
-    cudaFree(s->l_ptr);
-    cudaFree(s->l_col);
-    cudaFree(s->u_ptr);
-    cudaFree(s->u_col);
-    cudaFree(s->fwd_order);
-    cudaFree(s->bwd_order);
-    cudaFree(s->l_tpos);
-    cudaFree(s->d_fwd_level);
-    cudaFree(s->d_bwd_level);
+    void *blocks[19] = {s->l_ptr, s->l_col, s->u_ptr, s->u_col, s->fwd_order, s->bwd_order, s->l_tpos,
+                        s->d_fwd_level, s->d_bwd_level};
     for (int d = 0; d < 2; ++d) {
-        cudaFree(s->t_box_step[d]);
-        cudaFree(s->t_slot_row[d]);
-        cudaFree(s->t_slot_src[d]);
-        cudaFree(s->t_slot_ds[d]);
-        cudaFree(s->t_slot_next[d]);
+        void *tiles[5] = {s->t_box_step[d], s->t_slot_row[d], s->t_slot_src[d], s->t_slot_ds[d], s->t_slot_next[d]};
+        std::copy(tiles, tiles + 5, blocks + 9 + 5 * d);
     }
+    fv_blocks_free(blocks, 19);
     delete s;
 }
 
@@ -171,7 +162,7 @@ static fv_status resident_plan(fv_precond *P, const int32_t *perm, cudaStream_t 
     const fv_status s = fv_resident_build(q, st, &P->res);
     if (s == FV_ERR_ALLOC) return resident_no_memory(P);
     if (s != FV_OK || !P->res) return s;
-    const cudaError_t e = cudaMalloc(&P->res_rec, fv_resident_record_bytes(P->res, sizeof(double)));
+    const cudaError_t e = fv_block_alloc(&P->res_rec, fv_resident_record_bytes(P->res, sizeof(double)));
     if (e == cudaErrorMemoryAllocation) return resident_no_memory(P);
     FV_CUDA_TRY(e);
     return FV_OK;
@@ -287,7 +278,7 @@ static fv_status build_symbolic_impl(const fv_csr *A, cudaStream_t st, fv_symbol
     cudaError_t e = cudaSuccess;
     auto up_load = [&](int32_t **d, const std::vector<int32_t> &h, size_t cnt) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(d, sizeof(int32_t) * (cnt ? cnt : 1));
+        e = fv_block_alloc(d, sizeof(int32_t) * (cnt ? cnt : 1));
         if (e == cudaSuccess && cnt) e = cudaMemcpyAsync(*d, h.data(), sizeof(int32_t) * cnt, cudaMemcpyHostToDevice, st);
     };
     up_load(&s->l_ptr, lp, (size_t)n + 1);
@@ -370,7 +361,7 @@ static fv_status build_tiles_impl(fv_symbolic *s, const fv_csr *A, cudaStream_t 
     cudaError_t e = cudaSuccess;
     auto up_load = [&](int32_t **dp, const std::vector<int32_t> &h) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(dp, sizeof(int32_t) * (h.size() ? h.size() : 1));
+        e = fv_block_alloc(dp, sizeof(int32_t) * (h.size() ? h.size() : 1));
         if (e == cudaSuccess && h.size())
             e = cudaMemcpyAsync(*dp, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice, st);
     };
@@ -1392,8 +1383,8 @@ static fv_status tile_prepare(fv_precond *P, cudaStream_t st) {
     unsigned &seen = sizeof(T) == 8 ? P->t_rec64_epoch : P->t_rec32_version;
     for (int d = 0; d < 2; ++d) {
         if (!rec[d]) {
-            FV_CUDA_TRY(cudaMalloc(&rec[d], sizeof(TileRec<T>) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
-            FV_CUDA_TRY(cudaMalloc(&rhs[d], sizeof(T) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
+            FV_CUDA_TRY(fv_block_alloc(&rec[d], sizeof(TileRec<T>) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
+            FV_CUDA_TRY(fv_block_alloc(&rhs[d], sizeof(T) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
             seen = version - 1;
         }
     }
@@ -1679,8 +1670,8 @@ static fv_status build_symbolic_device(const fv_csr *A, cudaStream_t st, fv_symb
     cudaError_t e = fv_malloc_async(&dw, sizeof(int) * 8, st);
     if (e == cudaSuccess) e = fv_malloc_async(&ctrl, sizeof(unsigned) * 4, st);
     if (e == cudaSuccess) e = fv_malloc_async(&cnt, sizeof(int32_t) * 2 * (n + 1), st);
-    if (e == cudaSuccess) e = cudaMalloc(&s->l_ptr, sizeof(int32_t) * (n + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&s->u_ptr, sizeof(int32_t) * (n + 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&s->l_ptr, sizeof(int32_t) * (n + 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&s->u_ptr, sizeof(int32_t) * (n + 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(dw, 0, sizeof(int) * 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctrl, 0, sizeof(unsigned) * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int32_t) * 2 * (n + 1), st);
@@ -1711,12 +1702,12 @@ static fv_status build_symbolic_device(const fv_csr *A, cudaStream_t st, fv_symb
     s->max_lower = h[1];
     s->max_upper = h[2];
     s->max_row = h[3];
-    e = cudaMalloc(&s->l_col, sizeof(int32_t) * (nl ? nl : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&s->u_col, sizeof(int32_t) * (nu ? nu : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_fwd_level, sizeof(int32_t) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_bwd_level, sizeof(int32_t) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&s->fwd_order, sizeof(int32_t) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&s->bwd_order, sizeof(int32_t) * n);
+    e = fv_block_alloc(&s->l_col, sizeof(int32_t) * (nl ? nl : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&s->u_col, sizeof(int32_t) * (nu ? nu : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&s->d_fwd_level, sizeof(int32_t) * n);
+    if (e == cudaSuccess) e = fv_block_alloc(&s->d_bwd_level, sizeof(int32_t) * n);
+    if (e == cudaSuccess) e = fv_block_alloc(&s->fwd_order, sizeof(int32_t) * n);
+    if (e == cudaSuccess) e = fv_block_alloc(&s->bwd_order, sizeof(int32_t) * n);
     if (e == cudaSuccess) e = fv_malloc_async(&keys, sizeof(int32_t) * n, st);
     if (e == cudaSuccess) e = fv_malloc_async(&iota, sizeof(int32_t) * n, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_fwd_level, 0xFF, sizeof(int32_t) * n, st);
@@ -1766,7 +1757,7 @@ static fv_status build_symbolic_device(const fv_csr *A, cudaStream_t st, fv_symb
     }
     // transpose map (IC) when the pattern is structurally symmetric
     if (e == cudaSuccess && nl == nu) {
-        e = cudaMalloc(&s->l_tpos, sizeof(int32_t) * (nl ? nl : 1));
+        e = fv_block_alloc(&s->l_tpos, sizeof(int32_t) * (nl ? nl : 1));
         if (e == cudaSuccess) {
             fv_note_launch();
             k_sym_tpos<<<G, 256, 0, st>>>(n, s->l_ptr, s->l_col, s->u_ptr, s->u_col, s->l_tpos, dw);
@@ -1778,7 +1769,7 @@ static fv_status build_symbolic_device(const fv_csr *A, cudaStream_t st, fv_symb
     if (e != cudaSuccess) return fail(e, "symbolic (orders)");
     s->symmetric_pattern = nl == nu && !(h[0] & kSymAsym);
     if (!s->symmetric_pattern) {
-        cudaFree(s->l_tpos);
+        fv_block_free(s->l_tpos);
         s->l_tpos = nullptr;
     }
     cleanup();
@@ -1856,8 +1847,8 @@ extern "C" fv_status fv_diag_factor(const fv_csr *A, void *stream, fv_precond **
     P->kind = 3;
     P->n = A->nrows;
     P->A = A;
-    cudaError_t e = cudaMalloc(&P->dinv, sizeof(double) * P->n);
-    if (e == cudaSuccess) e = cudaMalloc(&P->err, sizeof(int));
+    cudaError_t e = fv_block_alloc(&P->dinv, sizeof(double) * P->n);
+    if (e == cudaSuccess) e = fv_block_alloc(&P->err, sizeof(int));
     if (e != cudaSuccess) {
         fv_internal_set_cuda_error(e, "fv_diag_factor");
         fv_precond_destroy(P);
@@ -1993,20 +1984,20 @@ fv_status fv_precond_make_f32(fv_precond *P, cudaStream_t st) {
     const fv_symbolic *s = P->sym;
     const int64_t n = P->n;
     if (P->kind == 3) {
-        if (!P->dinv32) FV_CUDA_TRY(cudaMalloc(&P->dinv32, sizeof(float) * n));
+        if (!P->dinv32) FV_CUDA_TRY(fv_block_alloc(&P->dinv32, sizeof(float) * n));
         fv_note_launch(), k_to_f32<<<148 * 8, 256, 0, st>>>(n, P->dinv, P->dinv32);
         FV_CUDA_TRY(cudaGetLastError());
         P->f32_version += 1;
         return FV_OK;
     }
     if (!P->l32) {
-        FV_CUDA_TRY(cudaMalloc(&P->l32, sizeof(float) * (s->nnz_l ? s->nnz_l : 1)));
-        FV_CUDA_TRY(cudaMalloc(&P->u32, sizeof(float) * (s->nnz_u ? s->nnz_u : 1)));
-        FV_CUDA_TRY(cudaMalloc(&P->dinv32, sizeof(float) * n));
-        FV_CUDA_TRY(cudaMalloc(&P->tmp32, sizeof(float) * n));
+        FV_CUDA_TRY(fv_block_alloc(&P->l32, sizeof(float) * (s->nnz_l ? s->nnz_l : 1)));
+        FV_CUDA_TRY(fv_block_alloc(&P->u32, sizeof(float) * (s->nnz_u ? s->nnz_u : 1)));
+        FV_CUDA_TRY(fv_block_alloc(&P->dinv32, sizeof(float) * n));
+        FV_CUDA_TRY(fv_block_alloc(&P->tmp32, sizeof(float) * n));
         FV_CUDA_TRY(cudaMemsetAsync(P->tmp32, 0xFF, sizeof(float) * n, st));
         if (P->perm) {
-            FV_CUDA_TRY(cudaMalloc(&P->zint32, sizeof(float) * n));
+            FV_CUDA_TRY(fv_block_alloc(&P->zint32, sizeof(float) * n));
             FV_CUDA_TRY(cudaMemsetAsync(P->zint32, 0xFF, sizeof(float) * n, st));
         }
     }
@@ -2017,7 +2008,7 @@ fv_status fv_precond_make_f32(fv_precond *P, cudaStream_t st) {
     FV_CUDA_TRY(cudaGetLastError());
     if (P->res) {
         if (!P->res_rec32 &&
-            cudaMalloc(&P->res_rec32, fv_resident_record_bytes(P->res, sizeof(float))) != cudaSuccess)
+            fv_block_alloc(&P->res_rec32, fv_resident_record_bytes(P->res, sizeof(float))) != cudaSuccess)
             cudaGetLastError();  // no memory: the other sweeps run
         if (P->res_rec32)
             FV_CUDA_TRY(fv_resident_records<float>(P->res, resident_src(P, P->perm), P->kind == 2, P->l32, P->u32, P->dinv32,
@@ -2130,31 +2121,15 @@ extern "C" fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t
 
 extern "C" fv_status fv_precond_destroy(fv_precond *P) {
     if (!P) return FV_OK;
-    cudaFree(P->l_val);
-    cudaFree(P->u_val);
-    cudaFree(P->diag);
-    cudaFree(P->dinv);
-    cudaFree(P->tmp);
-    cudaFree(P->done);
-    cudaFree(P->ctrl);
-    cudaFree(P->err);
-    cudaFree(P->l32);
-    cudaFree(P->u32);
-    cudaFree(P->dinv32);
-    cudaFree(P->tmp32);
-    cudaFree(P->amap);
-    cudaFree(P->perm);
-    cudaFree(P->zint);
-    cudaFree(P->zint32);
-    fv_resident_free(P->res);
-    cudaFree(P->res_rec);
-    cudaFree(P->res_rec32);
+    void *blocks[28] = {P->l_val, P->u_val, P->diag, P->dinv, P->tmp, P->done, P->ctrl, P->err, P->l32, P->u32,
+                        P->dinv32, P->tmp32, P->amap, P->perm, P->zint, P->zint32, P->res_rec, P->res_rec32};
+    if (P->res) blocks[18] = P->res->arena[0], blocks[19] = P->res->arena[1];
     for (int d = 0; d < 2; ++d) {
-        cudaFree(P->t_rec64[d]);
-        cudaFree(P->t_rec32[d]);
-        cudaFree(P->t_rhs64[d]);
-        cudaFree(P->t_rhs32[d]);
+        void *tiles[4] = {P->t_rec64[d], P->t_rec32[d], P->t_rhs64[d], P->t_rhs32[d]};
+        std::copy(tiles, tiles + 4, blocks + 20 + 4 * d);
     }
+    fv_blocks_free(blocks, 28);
+    delete P->res;
     fv_csr *F = P->fill;
     delete P;
     if (F) fv_csr_destroy(F);
@@ -2163,14 +2138,14 @@ extern "C" fv_status fv_precond_destroy(fv_precond *P) {
 
 static fv_status precond_alloc(fv_precond *P, cudaStream_t st) {
     const int64_t n = P->n;
-    FV_CUDA_TRY(cudaMalloc(&P->l_val, sizeof(double) * (P->sym->nnz_l ? P->sym->nnz_l : 1)));
-    FV_CUDA_TRY(cudaMalloc(&P->u_val, sizeof(double) * (P->sym->nnz_u ? P->sym->nnz_u : 1)));
-    FV_CUDA_TRY(cudaMalloc(&P->diag, sizeof(double) * n));
-    FV_CUDA_TRY(cudaMalloc(&P->dinv, sizeof(double) * n));
-    FV_CUDA_TRY(cudaMalloc(&P->tmp, sizeof(double) * n));
-    FV_CUDA_TRY(cudaMalloc(&P->done, sizeof(unsigned) * n));
-    FV_CUDA_TRY(cudaMalloc(&P->ctrl, sizeof(unsigned) * 8));
-    FV_CUDA_TRY(cudaMalloc(&P->err, sizeof(int)));
+    FV_CUDA_TRY(fv_block_alloc(&P->l_val, sizeof(double) * (P->sym->nnz_l ? P->sym->nnz_l : 1)));
+    FV_CUDA_TRY(fv_block_alloc(&P->u_val, sizeof(double) * (P->sym->nnz_u ? P->sym->nnz_u : 1)));
+    FV_CUDA_TRY(fv_block_alloc(&P->diag, sizeof(double) * n));
+    FV_CUDA_TRY(fv_block_alloc(&P->dinv, sizeof(double) * n));
+    FV_CUDA_TRY(fv_block_alloc(&P->tmp, sizeof(double) * n));
+    FV_CUDA_TRY(fv_block_alloc(&P->done, sizeof(unsigned) * n));
+    FV_CUDA_TRY(fv_block_alloc(&P->ctrl, sizeof(unsigned) * 8));
+    FV_CUDA_TRY(fv_block_alloc(&P->err, sizeof(int)));
     FV_CUDA_TRY(cudaMemsetAsync(P->tmp, 0xFF, sizeof(double) * n, st));
     FV_CUDA_TRY(cudaMemsetAsync(P->done, 0, sizeof(unsigned) * n, st));
     FV_CUDA_TRY(cudaMemsetAsync(P->ctrl, 0, sizeof(unsigned) * 8, st));
@@ -2394,10 +2369,10 @@ static fv_status fill_factor(const fv_csr *Ac, int kind, int level, cudaStream_t
     F->nnz = (int64_t)fcol.size();
     if (kind == 1) F->fill_mask = std::move(fill);
     int32_t *damap = nullptr;
-    cudaError_t e = cudaMalloc(&F->row_ptr, sizeof(int32_t) * (n + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&F->cols, sizeof(int32_t) * (F->nnz ? F->nnz : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&F->vals, sizeof(double) * (F->nnz ? F->nnz : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&damap, sizeof(int32_t) * (nnz ? nnz : 1));
+    cudaError_t e = fv_block_alloc(&F->row_ptr, sizeof(int32_t) * (n + 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&F->cols, sizeof(int32_t) * (F->nnz ? F->nnz : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&F->vals, sizeof(double) * (F->nnz ? F->nnz : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&damap, sizeof(int32_t) * (nnz ? nnz : 1));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(F->row_ptr, fptr.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && F->nnz)
@@ -2407,7 +2382,7 @@ static fv_status fill_factor(const fv_csr *Ac, int kind, int level, cudaStream_t
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         fv_internal_set_cuda_error(e, "fill pattern upload");
-        cudaFree(damap);
+        fv_block_free(damap);
         fv_csr_destroy(F);
         return e == cudaErrorMemoryAllocation ? FV_ERR_ALLOC : FV_ERR_CUDA;
     }
@@ -2422,7 +2397,7 @@ static fv_status fill_factor(const fv_csr *Ac, int kind, int level, cudaStream_t
     if (s == FV_OK) s = factor_common(F, kind, st, &P);
     if (s == FV_OK) P->schedule = 1;  // fill patterns keep the level chunks
     if (s != FV_OK) {
-        cudaFree(damap);
+        fv_block_free(damap);
         fv_csr_destroy(F);
         return s;
     }
@@ -2534,11 +2509,11 @@ static fv_status build_permuted(fv_csr *A, const int32_t *perm_host, cudaStream_
     void *scan_tmp = nullptr;
     size_t scan_bytes = 0;
     int hbad = 0;
-    cudaError_t e = cudaMalloc(&perm, sizeof(int32_t) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&B->row_ptr, sizeof(int32_t) * (n + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&B->cols, sizeof(int32_t) * (nnz ? nnz : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&B->vals, sizeof(double) * (nnz ? nnz : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&amap, sizeof(int32_t) * (nnz ? nnz : 1));
+    cudaError_t e = fv_block_alloc(&perm, sizeof(int32_t) * n);
+    if (e == cudaSuccess) e = fv_block_alloc(&B->row_ptr, sizeof(int32_t) * (n + 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&B->cols, sizeof(int32_t) * (nnz ? nnz : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&B->vals, sizeof(double) * (nnz ? nnz : 1));
+    if (e == cudaSuccess) e = fv_block_alloc(&amap, sizeof(int32_t) * (nnz ? nnz : 1));
     if (e == cudaSuccess) e = fv_malloc_async(&iperm, sizeof(int32_t) * n, st);
     if (e == cudaSuccess) e = fv_malloc_async(&len, sizeof(int32_t) * (n + 1), st);
     if (e == cudaSuccess) e = fv_malloc_async(&bad, sizeof(int), st);
@@ -2571,8 +2546,8 @@ static fv_status build_permuted(fv_csr *A, const int32_t *perm_host, cudaStream_
         if (e != cudaSuccess) fv_internal_set_cuda_error(e, "matrix permutation");
         if (hbad & 1) fv_internal_set_error_text("perm is not a permutation of 0..n-1");
         if (hbad & 2) fv_internal_set_error_text("a row has more than 32 entries");
-        cudaFree(perm);
-        cudaFree(amap);
+        fv_block_free(perm);
+        fv_block_free(amap);
         fv_csr_destroy(B);
         if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? FV_ERR_ALLOC : FV_ERR_CUDA;
         return (hbad & 2) ? FV_ERR_UNSUPPORTED : FV_ERR_INVALID;
@@ -2603,7 +2578,7 @@ static fv_status perm_factor_impl(const fv_csr *Ac, const int32_t *perm_host, in
     if (s == FV_OK) s = factor_common(B, kind, st, &P, perm);
     if (s == FV_OK) P->schedule = 1;  // the reordered sweeps have their own kernels (P->perm)
     if (s == FV_OK) {
-        e = cudaMalloc(&P->zint, sizeof(double) * n);
+        e = fv_block_alloc(&P->zint, sizeof(double) * n);
         if (e == cudaSuccess) e = cudaMemsetAsync(P->zint, 0xFF, sizeof(double) * n, st);
         if (e != cudaSuccess) {
             fv_internal_set_cuda_error(e, "reordered factorisation");
@@ -2613,8 +2588,8 @@ static fv_status perm_factor_impl(const fv_csr *Ac, const int32_t *perm_host, in
         }
     }
     if (s != FV_OK) {
-        cudaFree(perm);
-        cudaFree(amap);
+        fv_block_free(perm);
+        fv_block_free(amap);
         fv_csr_destroy(B);
         return s;
     }

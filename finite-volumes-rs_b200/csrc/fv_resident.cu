@@ -418,8 +418,7 @@ fv_res_args fv_resident_args(const fv_resident *p, const void *rec, size_t tb) {
 
 void fv_resident_free(fv_resident *p) {
     if (!p) return;
-    cudaFree(p->arena[0]);
-    cudaFree(p->arena[1]);
+    fv_blocks_free(p->arena, 2);
     delete p;
 }
 
@@ -472,7 +471,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     size_t cub_bytes = std::max(sort_bytes, scan_bytes);
     const size_t t_cub = tl.take(cub_bytes);
     char *plan = nullptr, *tmp = nullptr;
-    cudaError_t e = cudaMalloc((void **)&plan, pl.bytes);
+    cudaError_t e = fv_block_alloc(&plan, pl.bytes);
     p->arena[0] = plan;
     if (e == cudaSuccess) e = fv_malloc_async(&tmp, tl.bytes, st);
     auto fail = [&]() {
@@ -564,7 +563,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     Layout sl;
     const size_t s_item = sl.take(4 * p->nslots), s_dep = sl.take(2 * (size_t)p->ml * p->nslots),
                  s_push = sl.take(8 * p->nslots);
-    e = cudaMalloc(&p->arena[1], sl.bytes);
+    e = fv_block_alloc(&p->arena[1], sl.bytes);
     if (e != cudaSuccess) return fail();
     p->slot_item = (int32_t *)((char *)p->arena[1] + s_item);
     p->slot_dep = (uint16_t *)((char *)p->arena[1] + s_dep);

@@ -89,13 +89,9 @@ extern "C" fv_status fv_csr_download(const fv_csr *A, int32_t *row_ptr, int32_t 
 
 extern "C" fv_status fv_csr_destroy(fv_csr *A) {
     if (!A) return FV_OK;
-    if (A->owns_pattern) {
-        cudaFree(A->row_ptr);
-        cudaFree(A->cols);
-    }
-    cudaFree(A->vals);
-    cudaFree(A->perm);
-    cudaFree(A->perm_amap);
+    void *blocks[5] = {A->owns_pattern ? A->row_ptr : nullptr, A->owns_pattern ? A->cols : nullptr, A->vals, A->perm,
+                       A->perm_amap};
+    fv_blocks_free(blocks, 5);
     fv_symbolic_free(A->sym);
     delete A;
     return FV_OK;
@@ -1237,8 +1233,6 @@ constexpr size_t kNoAllocBytes =
 // device address.
 static __device__ __align__(256) unsigned char g_cg_noalloc_scratch[kNoAllocBytes];
 
-#include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
-
 #include <mutex>
 static std::mutex g_cg_noalloc_mu;
 struct NoAllocSlot {
@@ -1246,33 +1240,6 @@ struct NoAllocSlot {
     unsigned long long ctx_id = 0;  // unique id of the context the address belongs to (0: none yet)
 };
 static NoAllocSlot g_cg_noalloc_slot[256];
-
-// Unique id of the calling thread's current context (cuCtxGetId, unique over
-// the process's life), or 0 when the driver does not provide it.
-static unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext *);
-    using GetId = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = (GetCurrent)f;
-        f = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = (GetId)f;
-        cudaGetLastError();
-    });
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
-        return 0;
-    return id;
-}
 
 // Device address of the scratch array on the current device.  Set-up runs
 // once per device, with that device current: cudaGetSymbolAddress, checked.
@@ -1283,14 +1250,14 @@ static fv_status cg_noalloc_scratch(void **out) {
     int dev = -1;
     FV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 256) return FV_ERR_INVALID;
-    const unsigned long long ctx = current_context_id();  // 0 while no context is current on this thread
+    const unsigned long long ctx = fv_current_context_id();  // 0 while no context is current on this thread
     std::lock_guard<std::mutex> lock(g_cg_noalloc_mu);
     NoAllocSlot &slot = g_cg_noalloc_slot[dev];
     if (!slot.addr || ctx == 0 || slot.ctx_id != ctx) {
         void *p = nullptr;
         FV_CUDA_TRY(cudaGetSymbolAddress(&p, g_cg_noalloc_scratch));  // makes the primary context current
         slot.addr = p;
-        slot.ctx_id = current_context_id();
+        slot.ctx_id = fv_current_context_id();
     }
     *out = slot.addr;
     return FV_OK;
