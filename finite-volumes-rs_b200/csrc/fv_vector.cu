@@ -16,6 +16,54 @@ inline int vec_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 4));
 }
 
+constexpr int kMaxBlocks = 148 * 4;
+
+// The workspace of one host thread's reductions: per device the block partials
+// and the ticket (0 between calls), and the result in pinned host memory, which
+// the kernel writes.  A reduction returns after its stream has finished, so a
+// thread's next one never meets it in use.
+struct Workspace {
+    struct OnDevice {
+        double *partial = nullptr;  // kMaxBlocks values, then the ticket
+        unsigned long long ctx = 0;
+    };
+    OnDevice at[64];
+    double *result = nullptr;
+    ~Workspace() {
+        int dev = -1;
+        if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && at[dev].partial && at[dev].ctx != 0 &&
+            fv_current_context_id() == at[dev].ctx)
+            cudaFree(at[dev].partial);
+        if (result) cudaFreeHost(result);
+    }
+};
+
+// The thread's workspace on the current device, made on first use there (and
+// again after the device's context was replaced).
+fv_status workspace(cudaStream_t st, double *&partial, double *&result) {
+    thread_local Workspace w;
+    int dev = -1;
+    FV_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return FV_ERR_INVALID;
+    Workspace::OnDevice &d = w.at[dev];
+    const unsigned long long ctx = fv_current_context_id();
+    if (!d.partial || d.ctx != ctx) {
+        double *p = nullptr;
+        FV_CUDA_TRY(cudaMalloc(&p, sizeof(double) * (kMaxBlocks + 1)));
+        const cudaError_t e = cudaMemsetAsync(p, 0, sizeof(double) * (kMaxBlocks + 1), st);
+        if (e != cudaSuccess) {
+            cudaFree(p);
+            FV_CUDA_TRY(e);
+        }
+        d.partial = p;
+        d.ctx = fv_current_context_id();
+    }
+    if (!w.result) FV_CUDA_TRY(cudaHostAlloc((void **)&w.result, sizeof(double), cudaHostAllocPortable));
+    partial = d.partial;
+    result = w.result;
+    return FV_OK;
+}
+
 __device__ __forceinline__ double block_sum(double v, double *sm) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -27,23 +75,40 @@ __device__ __forceinline__ double block_sum(double v, double *sm) {
     return t;
 }
 
-// mode 0: sum x_i y_i; mode 1: sum x_i
-__global__ void __launch_bounds__(kVB) k_vec_partial(int64_t n, const double *__restrict__ x,
-                                                     const double *__restrict__ y, int mode,
-                                                     double *__restrict__ partial) {
-    __shared__ double sm[kVB / 32];
+// DOT: sum x_i y_i, else sum x_i.  One kernel: the last block to finish loads
+// the block partials together and adds them in block order (a second kernel's
+// single thread read them from L2 one after the other), and the result goes
+// straight to the host.  Bound by memory above some 10^6 entries, below by the
+// launch and the host's wait: dot of 10,007 entries 34 -> 22 us per call from
+// Python, of 1,000,003 entries 56 -> 24, of 8,000,000 entries 69 -> 41.
+template <bool DOT>
+__global__ void __launch_bounds__(kVB) k_vec_reduce(int64_t n, const double *__restrict__ x,
+                                                    const double *__restrict__ y, double *partial,
+                                                    double *__restrict__ out) {
+    __shared__ double sm[kVB / 32], all[kMaxBlocks];
+    __shared__ bool last;
+    unsigned *ticket = reinterpret_cast<unsigned *>(partial + kMaxBlocks);
     double acc = 0.0;
+#pragma unroll 4
     for (int64_t i = (int64_t)blockIdx.x * kVB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kVB)
-        acc += mode == 0 ? x[i] * y[i] : x[i];
+        acc += DOT ? x[i] * y[i] : x[i];
     const double t = block_sum(acc, sm);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t;
-}
-
-__global__ void k_vec_final(int nb, const double *__restrict__ partial, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double t = 0.0;
-    for (int b = 0; b < nb; ++b) t += partial[b];
-    *out = t;
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    for (int b = threadIdx.x; b < gridDim.x; b += kVB) all[b] = __ldcg(&partial[b]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int b = 0; b < gridDim.x; ++b) s += all[b];
+        *ticket = 0;
+        *out = s;
+        __threadfence_system();
+    }
 }
 
 // op 0: y += x; 1: y -= x; 2: y *= a; 3: y = 1 / y; 4: y = x
@@ -67,18 +132,16 @@ fv_status reduce(int64_t n, const double *x, const double *y, int mode, void *st
     }
     if (!x || (mode == 0 && !y)) return FV_ERR_INVALID;
     cudaStream_t st = fv_stream(stream);
-    const int G = vec_grid(n);
-    double *buf = nullptr;
-    FV_CUDA_TRY(fv_malloc_async(&buf, sizeof(double) * (G + 1), st));
+    double *partial = nullptr, *result = nullptr;
+    FV_TRY(workspace(st, partial, result));
     fv_note_launch();
-    k_vec_partial<<<G, kVB, 0, st>>>(n, x, y, mode, buf);
-    fv_note_launch();
-    k_vec_final<<<1, 32, 0, st>>>(G, buf, buf + G);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, buf + G, sizeof(double), cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(buf, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    FV_CUDA_TRY(e);
+    if (mode == 0)
+        k_vec_reduce<true><<<vec_grid(n), kVB, 0, st>>>(n, x, y, partial, result);
+    else
+        k_vec_reduce<false><<<vec_grid(n), kVB, 0, st>>>(n, x, y, partial, result);
+    FV_CUDA_TRY(cudaGetLastError());
+    FV_CUDA_TRY(cudaStreamSynchronize(st));
+    *out = *(volatile double *)result;
     return FV_OK;
 }
 
