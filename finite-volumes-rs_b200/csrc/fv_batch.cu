@@ -35,6 +35,8 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
                                    const fv_row_skip *rskip);
 fv_status fv_precond_make_f32(fv_precond *P, cudaStream_t st);
 fv_status fv_precond_check_error(fv_precond *P, cudaStream_t st);
+fv_status fv_precond_batch_prepare(fv_precond *P, int np, const int64_t *offsets, const int32_t *of_row, bool f32,
+                                   cudaStream_t st);
 
 namespace {
 
@@ -1024,6 +1026,7 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
     const int G = grid_of(B);
     const Tiles tl = tiles_of(B);
     if (!mixed) {
+        FV_TRY(fv_precond_batch_prepare(P, np, B->off.data(), B->row_prob, false, st));
         InnerVecs<double> v = carve<double>(B->vec, n, x);
         FV_CUDA_TRY(cudaMemcpyAsync(v.r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
         if (nseg) {
@@ -1038,6 +1041,7 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
         if (!B->a32) FV_CUDA_TRY(cudaMalloc(&B->a32, sizeof(float) * (B->A->nnz ? B->A->nnz : 1)));
         fv_note_launch(), k_to_f32b<<<148 * 8, 256, 0, st>>>(B->A->nnz, B->A->vals, B->a32);
         FV_TRY(fv_precond_make_f32(P, st));
+        FV_TRY(fv_precond_batch_prepare(P, np, B->off.data(), B->row_prob, true, st));
         InnerVecs<float> v = carve<float>(B->vec, n, nullptr);
         if (nseg) {
             const InnerVecs<float> u = carve<float>(from->vec, from->n, nullptr);

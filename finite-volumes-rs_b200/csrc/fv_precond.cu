@@ -120,6 +120,12 @@ struct fv_precond {
     fv_resident *res = nullptr;
     void *res_rec = nullptr, *res_rec32 = nullptr;
     bool explicit_schedule = false;
+    // the same for the problems of a batch on several clusters, made by the
+    // first batch run (fv_precond_batch_prepare); the records' versions
+    fv_resident *batch_res = nullptr;
+    bool batch_tried = false;
+    void *batch_rec = nullptr, *batch_rec32 = nullptr;
+    unsigned batch_rec_epoch = 0, batch_rec32_version = 0;
 };
 
 static fv_resident_src resident_src(const fv_precond *P, const int32_t *perm) {
@@ -144,9 +150,11 @@ static fv_resident_src resident_src(const fv_precond *P, const int32_t *perm) {
     return q;
 }
 
-static bool use_resident(const fv_precond *P) {
-    return P->res && !P->explicit_schedule && P->sweep_blocks == 0 && P->sweep_rpt == 0;
+// No schedule or launch shape was asked for explicitly.
+static bool default_sweeps(const fv_precond *P) {
+    return !P->explicit_schedule && P->sweep_blocks == 0 && P->sweep_rpt == 0;
 }
+static bool use_resident(const fv_precond *P) { return P->res && default_sweeps(P); }
 
 // The plan and its records are an optimisation: without memory for them the
 // other sweeps run.
@@ -1888,6 +1896,10 @@ fv_status fv_precond_apply_dev(fv_precond *P, const double *r, double *z, cudaSt
         FV_CUDA_TRY(cudaGetLastError());
         return FV_OK;
     }
+    if (rs.group && P->batch_rec && P->batch_rec_epoch == P->epoch && default_sweeps(P)) {
+        FV_CUDA_TRY(fv_resident_apply<double>(P->batch_res, P->batch_rec, r, z, skip, rs, P->err, st));
+        return FV_OK;
+    }
     if (use_resident(P)) {
         FV_CUDA_TRY(fv_resident_apply<double>(P->res, P->res_rec, r, z, skip, rs, P->err, st));
         return FV_OK;
@@ -2031,6 +2043,10 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
         return FV_OK;
     }
     if (!P->l32) return FV_ERR_INVALID;
+    if (rs.group && P->batch_rec32 && P->batch_rec32_version == P->f32_version && default_sweeps(P)) {
+        FV_CUDA_TRY(fv_resident_apply<float>(P->batch_res, P->batch_rec32, r, z, skip, rs, P->err, st));
+        return FV_OK;
+    }
     if (use_resident(P) && P->res_rec32) {
         FV_CUDA_TRY(fv_resident_apply<float>(P->res, P->res_rec32, r, z, skip, rs, P->err, st));
         return FV_OK;
@@ -2092,6 +2108,38 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
     return FV_OK;
 }
 
+// Before a batch run over these problems: the plan on several clusters (once) and
+// the records of the current factors in the run's precision.  Without a plan or
+// memory for it the other sweeps run.
+fv_status fv_precond_batch_prepare(fv_precond *P, int np, const int64_t *offsets, const int32_t *of_row, bool f32,
+                                   cudaStream_t st) {
+    if (P->kind == 3 || np < 2 || !default_sweeps(P)) return FV_OK;
+    if (!P->batch_tried) {
+        P->batch_tried = true;
+        const fv_resident_problems q{np, offsets, of_row};
+        const fv_status s = fv_resident_build(resident_src(P, P->perm), st, &P->batch_res, &q);
+        if (s != FV_OK && s != FV_ERR_ALLOC) return s;
+        if (s == FV_ERR_ALLOC) cudaGetLastError();
+    }
+    if (!P->batch_res) return FV_OK;
+    void *&rec = f32 ? P->batch_rec32 : P->batch_rec;
+    if (!rec && fv_block_alloc(&rec, fv_resident_record_bytes(P->batch_res, f32 ? sizeof(float) : sizeof(double))) !=
+                    cudaSuccess) {
+        cudaGetLastError();
+        rec = nullptr;
+        return FV_OK;
+    }
+    const fv_resident_src src = resident_src(P, P->perm);
+    if (f32) {
+        FV_CUDA_TRY(fv_resident_records<float>(P->batch_res, src, P->kind == 2, P->l32, P->u32, P->dinv32, rec, st));
+        P->batch_rec32_version = P->f32_version;
+    } else if (P->batch_rec_epoch != P->epoch) {
+        FV_CUDA_TRY(fv_resident_records<double>(P->batch_res, src, P->kind == 2, P->l_val, P->u_val, P->dinv, rec, st));
+        P->batch_rec_epoch = P->epoch;
+    }
+    return FV_OK;
+}
+
 extern "C" fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t *active, double *stats) {
     if (!P || request < -1 || request > 4) return FV_ERR_INVALID;
     if (P->kind == 3) {  // no sweeps to schedule
@@ -2121,14 +2169,18 @@ extern "C" fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t
 
 extern "C" fv_status fv_precond_destroy(fv_precond *P) {
     if (!P) return FV_OK;
-    void *blocks[28] = {P->l_val, P->u_val, P->diag, P->dinv, P->tmp, P->done, P->ctrl, P->err, P->l32, P->u32,
+    void *blocks[32] = {P->l_val, P->u_val, P->diag, P->dinv, P->tmp, P->done, P->ctrl, P->err, P->l32, P->u32,
                         P->dinv32, P->tmp32, P->amap, P->perm, P->zint, P->zint32, P->res_rec, P->res_rec32};
     if (P->res) blocks[18] = P->res->arena[0], blocks[19] = P->res->arena[1];
     for (int d = 0; d < 2; ++d) {
         void *tiles[4] = {P->t_rec64[d], P->t_rec32[d], P->t_rhs64[d], P->t_rhs32[d]};
         std::copy(tiles, tiles + 4, blocks + 20 + 4 * d);
     }
-    fv_blocks_free(blocks, 28);
+    if (P->batch_res) blocks[28] = P->batch_res->arena[0], blocks[29] = P->batch_res->arena[1];
+    blocks[30] = P->batch_rec;
+    blocks[31] = P->batch_rec32;
+    fv_blocks_free(blocks, 32);
+    delete P->batch_res;
     delete P->res;
     fv_csr *F = P->fill;
     delete P;

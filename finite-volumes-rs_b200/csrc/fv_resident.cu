@@ -1,7 +1,9 @@
 // Plans, records and launch of the resident sweeps (fv_resident.cuh).
 #include <algorithm>
 #include <cub/cub.cuh>
+#include <cstdint>
 #include <new>
+#include <vector>
 
 #include "fv_resident.cuh"
 
@@ -38,6 +40,31 @@ __global__ void k_res_level_start(int64_t n, int32_t nlev, const int32_t *__rest
 // to other CTAs only at the slabs' faces and only downstream, so a CTA lags its
 // neighbour instead of waiting on every level (24,576-row ILU(0) on 8 CTAs:
 // 1,024 halo slots per CTA instead of 9,065).
+//
+// A batch's problems (k_res_owner_batch): the same within each problem, over the
+// CTAs of the problem's cluster.
+__global__ void k_res_root_count(int64_t n, const int32_t *__restrict__ lstart, const int32_t *__restrict__ perm,
+                                 const int32_t *__restrict__ of_row, int32_t *__restrict__ root0,
+                                 int32_t *__restrict__ nroot) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= lstart[1]) return;
+    const int32_t q = of_row[perm ? perm[i] : i];
+    atomicMin(&root0[q], (int32_t)i);
+    atomicAdd(&nroot[q], 1);
+}
+__global__ void k_res_owner_batch(int64_t n, int C, const int32_t *__restrict__ perm,
+                                  const int32_t *__restrict__ of_row, const int32_t *__restrict__ cluster,
+                                  const int32_t *__restrict__ root0, const int32_t *__restrict__ nroot,
+                                  const int32_t *__restrict__ lp, const int32_t *__restrict__ lc,
+                                  uint32_t *__restrict__ owner) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int32_t q = of_row[perm ? perm[p] : p];
+    int r = (int)p;
+    for (int e = lp[r + 1]; e > lp[r]; e = lp[r + 1]) r = lc[e - 1];
+    const int64_t at = (int64_t)(r - root0[q]) * C / max(1, nroot[q]);
+    owner[p] = (uint32_t)(cluster[q] * C + (int)max((int64_t)0, min((int64_t)C - 1, at)));
+}
 __global__ void k_res_owner_sorted(int64_t n, int C, const int32_t *__restrict__ lstart,
                                    const int32_t *__restrict__ lp, const int32_t *__restrict__ lc,
                                    uint32_t *__restrict__ owner) {
@@ -217,8 +244,9 @@ struct ResPattern {
     int32_t nlev[2];
     __host__ __device__ int32_t keys() const { return nlev[0] + nlev[1] + 1; }
 };
-__global__ void k_res_keys(ResPattern a, const uint32_t *__restrict__ owner, uint32_t *__restrict__ key,
-                           uint32_t *__restrict__ mask) {
+// *bad: a dependency on another cluster (the plan does not apply).
+__global__ void k_res_keys(ResPattern a, int C, const uint32_t *__restrict__ owner, uint32_t *__restrict__ key,
+                           uint32_t *__restrict__ mask, int32_t *__restrict__ bad) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 2 * a.n) return;
     const int d = t >= a.n ? 1 : 0;
@@ -227,7 +255,9 @@ __global__ void k_res_keys(ResPattern a, const uint32_t *__restrict__ owner, uin
     key[t] = o * (uint32_t)a.keys() + (uint32_t)(a.level[d][i] + (d ? a.nlev[0] : 0));
     for (int e = a.ptr[d][i]; e < a.ptr[d][i + 1]; ++e) {
         const int32_t j = a.col[d][e];
-        if (owner[j] != o) atomicOr(&mask[d * a.n + j], 1u << o);
+        if (owner[j] == o) continue;
+        atomicOr(&mask[d * a.n + j], 1u << (o % C));
+        if (owner[j] / C != o / C) *bad = 1;
     }
 }
 
@@ -252,21 +282,23 @@ __global__ void k_res_pad(int32_t per_cta, int sets, int32_t *__restrict__ nstep
 }
 
 // Halo slots: an item read by CTA c takes the next free slot of c.
-__global__ void k_res_halo(int64_t items, const uint32_t *__restrict__ mask, const int32_t *__restrict__ poff,
-                           int32_t *__restrict__ hcount, uint16_t *__restrict__ hslot, int32_t per_cta, int C,
+__global__ void k_res_halo(int64_t n, const uint32_t *__restrict__ owner, const uint32_t *__restrict__ mask,
+                           const int32_t *__restrict__ poff, int32_t *__restrict__ hcount,
+                           uint16_t *__restrict__ hslot, int32_t per_cta, int C, int ctas,
                            const int32_t *__restrict__ soff, int32_t *__restrict__ step_ptr) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= C) step_ptr[i] = soff[i * per_cta];
-    if (i >= items) return;
+    if (i <= ctas) step_ptr[i] = soff[i * per_cta];
+    if (i >= 2 * n) return;
+    const uint32_t first = owner[i >= n ? i - n : i] / C * C;  // its cluster's first CTA
     int k = poff[i];
     for (uint32_t m = mask[i]; m; m &= m - 1) {
-        const int h = atomicAdd(&hcount[__ffs(m) - 1], 1);
+        const int h = atomicAdd(&hcount[first + __ffs(m) - 1], 1);
         hslot[k++] = (uint16_t)min(h, 65535);  // a count past the limit makes the plan inapplicable
     }
 }
 
 // The slot of the p-th item in key order, its dependencies and readers.
-__global__ void k_res_compose(ResPattern a, int ml, int width, int zero, const uint32_t *__restrict__ key,
+__global__ void k_res_compose(ResPattern a, int C, int ml, int width, int zero, const uint32_t *__restrict__ key,
                               const int32_t *__restrict__ item, const int32_t *__restrict__ first,
                               const int32_t *__restrict__ soff, const uint32_t *__restrict__ owner,
                               const uint16_t *__restrict__ slot_of, const uint32_t *__restrict__ mask,
@@ -292,7 +324,7 @@ __global__ void k_res_compose(ResPattern a, int ml, int width, int zero, const u
                 c = slot_of[j];
             } else {
                 const int64_t u = d * a.n + j;
-                c = (uint16_t)(hbase + hslot[poff[u] + __popc(mask[u] & ((1u << o) - 1u))]);
+                c = (uint16_t)(hbase + hslot[poff[u] + __popc(mask[u] & ((1u << (o % C)) - 1u))]);
                 meta |= kResHalo;
             }
         }
@@ -378,10 +410,50 @@ int res_group(const fv_resident *p, size_t tb) {
 }
 
 template <typename T>
-bool res_launchable(const fv_resident *p) {
+int res_launchable(const fv_resident *p) {
     return fv_res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
         return fv_res_launchable(k_resident_apply<T, M(), S()>, p->C, fv_resident_smem(p, sizeof(T)));
     });
+}
+
+constexpr int kResMaxCtas = 160;  // CTAs of all clusters
+
+// Shares the problems out over clusters: the cluster size whose fullest CTA has
+// the fewest rows, problems to the emptiest cluster in descending size.
+fv_status res_share_problems(const fv_resident_problems &q, int levels, int &C, int &width, int &clusters,
+                             std::vector<int32_t> &cluster) {
+    try {
+        std::vector<int> order(q.n);
+        for (int k = 0; k < q.n; ++k) order[k] = k;
+        auto rows = [&](int k) { return q.offsets[k + 1] - q.offsets[k]; };
+        std::sort(order.begin(), order.end(), [&](int x, int y) { return rows(x) != rows(y) ? rows(x) > rows(y) : x < y; });
+        int64_t best = INT64_MAX;
+        for (int c = 1; c <= kResMaxCta; c *= 2) {
+            // clusters resident at once with one CTA per SM (148 SMs; a cluster stays within a GPC)
+            const int most = c == 1 ? 148 : c == 2 ? 74 : c == 4 ? 33 : c == 8 ? 15 : 7;
+            const int k = std::min(most, q.n);
+            std::vector<int64_t> load(k, 0);
+            std::vector<int32_t> to(q.n);
+            for (int t : order) {
+                const int at = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+                load[at] += rows(t);
+                to[t] = at;
+            }
+            const int64_t full = (*std::max_element(load.begin(), load.end()) + c - 1) / c;
+            if (full < best - best / 8) {  // larger clusters hand more values over
+                best = full;
+                C = c;
+                clusters = k;
+                cluster = to;
+            }
+        }
+        width = 32;
+        const int64_t lw = best / std::max(1, levels);
+        while (width < 256 && 2 * lw > width) width *= 2;
+        return FV_OK;
+    } catch (const std::bad_alloc &) {
+        return FV_ERR_ALLOC;
+    }
 }
 
 // Arrays laid out in one allocation.
@@ -408,7 +480,7 @@ fv_res_args fv_resident_args(const fv_resident *p, const void *rec, size_t tb) {
     a.step_ptr = p->step_ptr;
     a.cta_ptr = p->cta_ptr;
     a.rows = p->nat ? p->nat : p->rows;
-    a.C = p->C;
+    a.C = p->C * p->clusters;
     a.cap = p->cap;
     a.halo = p->halo;
     a.width = p->width;
@@ -424,10 +496,13 @@ void fv_resident_free(fv_resident *p) {
 
 size_t fv_resident_record_bytes(const fv_resident *p, size_t tb) { return (size_t)p->nslots * res_rec_bytes(p->ml, tb); }
 
-fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out) {
+fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
+                            const fv_resident_problems *problems) {
     *out = nullptr;
     const int64_t n = s.n;
-    if (n <= 0 || n > 16 * 20000 || s.max_side > 6 || !s.fwd_level || !s.bwd_level) return FV_OK;
+    if (n <= 0 || n > (problems ? 148 : kResMaxCta) * 20000LL || s.max_side > 6 || !s.fwd_level || !s.bwd_level)
+        return FV_OK;
+    if (problems && !s.sorted) return FV_OK;
     // CTAs: enough shared memory for the rows, and as few as keep a level of a
     // CTA within 128 rows (natural order: more CTAs only add hand-offs) or as
     // many as leave it 32 (rows sorted by level: few, wide levels).  Measured as
@@ -439,10 +514,14 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
     while (C < kResMaxCta && (n > (int64_t)C * 18000 || lw > (int64_t)C * (s.sorted ? 32 : 128))) C *= 2;
     while (width < (s.sorted ? 256 : 128) && lw * (s.sorted ? 2 : 1) > (int64_t)C * width) width *= 2;
-    const int sets = width <= 128 ? 4 : 512 / width;
+    std::vector<int32_t> cluster;  // of every problem
+    int clusters = 1;
+    if (problems) FV_TRY(res_share_problems(*problems, s.n_fwd_levels, C, width, clusters, cluster));
+    const int sets = width <= 128 ? 4 : 512 / width, ctas = C * clusters;
     fv_resident *p = new (std::nothrow) fv_resident();
     if (!p) return FV_ERR_ALLOC;
     p->C = C;
+    p->clusters = clusters;
     p->width = width;
     p->sorted = s.sorted;
     p->sets = sets;
@@ -453,14 +532,14 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     a.col[0] = s.l_col, a.col[1] = s.u_col;
     a.level[0] = s.fwd_level, a.level[1] = s.bwd_level;
     a.nlev[0] = s.n_fwd_levels, a.nlev[1] = s.n_bwd_levels;
-    const int64_t items = 2 * n, nk = (int64_t)C * a.keys(), nnz = s.nnz_l + s.nnz_u;
+    const int64_t items = 2 * n, nk = (int64_t)ctas * a.keys(), nnz = s.nnz_l + s.nnz_u;
     const int64_t cm = std::max(items, nk) + 2;
     Layout pl, tl;
-    const size_t o_cta = pl.take(4 * (C + 1)), o_rows = pl.take(4 * n), o_nat = pl.take(s.perm ? 4 * n : 0),
-                 o_slot = pl.take(2 * n), o_sptr = pl.take(4 * (C + 1)), o_push = pl.take(4 * (nnz + 1));
+    const size_t o_cta = pl.take(4 * (ctas + 1)), o_rows = pl.take(4 * n), o_nat = pl.take(s.perm ? 4 * n : 0),
+                 o_slot = pl.take(2 * n), o_sptr = pl.take(4 * (ctas + 1)), o_push = pl.take(4 * (nnz + 1));
     const size_t t_owner = tl.take(4 * n), t_iota = tl.take(4 * items), t_key = tl.take(4 * items),
                  t_sorted = tl.take(4 * items), t_item = tl.take(4 * items), t_cnt = tl.take(4 * cm),
-                 t_cnt2 = tl.take(4 * cm), t_hc = tl.take(4 * kResMaxCta), t_axes = tl.take(sizeof(ResAxes)),
+                 t_cnt2 = tl.take(4 * cm), t_hc = tl.take(4 * (ctas + 1)), t_prob = tl.take(problems ? 12 * (size_t)problems->n : 0), t_axes = tl.take(sizeof(ResAxes)),
                  t_hist = tl.take(s.cell ? 12 * (size_t)C * a.nlev[0] : 0), t_lst = tl.take(4 * (a.nlev[0] + 2)),
                  t_mask = tl.take(4 * items), t_poff = tl.take(4 * (items + 1)), t_hslot = tl.take(2 * (nnz + 1)),
                  t_first = tl.take(4 * (nk + 1)), t_soff = tl.take(4 * (nk + 1));
@@ -504,11 +583,20 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
         if (e == cudaSuccess)
             e = cub::DeviceRadixSort::SortPairs(cubt, cub_bytes, k, sorted, iota, v, (int)m, 0, bits_of(keys), st);
     };
-    e = cudaMemsetAsync(hc, 0, 4 * kResMaxCta, st);
+    e = cudaMemsetAsync(hc, 0, 4 * (ctas + 1), st);  // the last entry: a dependency between clusters
     if (e == cudaSuccess) e = cudaMemsetAsync(mask, 0, 4 * items, st);
     fv_note_launch(), k_res_level_start<<<grid(n + 1), 256, 0, st>>>(n, a.nlev[0], s.fwd_order, s.fwd_level, lst);
     fv_note_launch(), k_res_iota<<<grid(items), 256, 0, st>>>(items, iota);
-    if (s.sorted) {
+    if (problems) {
+        const int np = problems->n;
+        int32_t *root0 = i32(t_prob), *nroot = root0 + np, *dcl = root0 + 2 * np;
+        if (e == cudaSuccess) e = cudaMemsetAsync(root0, 0x7F, 4 * (size_t)np, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(nroot, 0, 4 * (size_t)np, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dcl, cluster.data(), 4 * (size_t)np, cudaMemcpyHostToDevice, st);
+        fv_note_launch(), k_res_root_count<<<grid(n), 256, 0, st>>>(n, lst, s.perm, problems->of_row, root0, nroot);
+        fv_note_launch(), k_res_owner_batch<<<grid(n), 256, 0, st>>>(n, C, s.perm, problems->of_row, dcl, root0, nroot,
+                                                                     s.l_ptr, s.l_col, owner);
+    } else if (s.sorted) {
         fv_note_launch(), k_res_owner_sorted<<<grid(n), 256, 0, st>>>(n, C, lst, s.l_ptr, s.l_col, owner);
     } else {
         int32_t *hist = i32(t_hist);
@@ -529,32 +617,33 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
             fv_note_launch(), k_res_pick<<<grid(n), 256, 0, st>>>(n, s.cell, ax, owner);
         }
     }
-    sort(owner, p->rows, n, C);
-    fv_note_launch(), k_res_bounds<<<grid(n + 1), 256, 0, st>>>(n, C, sorted, p->cta_ptr);
+    sort(owner, p->rows, n, ctas);
+    fv_note_launch(), k_res_bounds<<<grid(n + 1), 256, 0, st>>>(n, ctas, sorted, p->cta_ptr);
     fv_note_launch(), k_res_slots<<<grid(n), 256, 0, st>>>(n, p->rows, owner, p->cta_ptr, s.perm, p->slot_of, p->nat);
-    fv_note_launch(), k_res_keys<<<grid(items), 256, 0, st>>>(a, owner, key, mask);
+    fv_note_launch(), k_res_keys<<<grid(items), 256, 0, st>>>(a, C, owner, key, mask, hc + ctas);
     sort(key, item, items, nk);
     fv_note_launch(), k_res_bounds<<<grid(items + 1), 256, 0, st>>>(items, (int32_t)nk, sorted, first);
     fv_note_launch(), k_res_counts<<<grid(cm), 256, 0, st>>>(items, mask, cnt, (int32_t)nk, a.keys(), first, width,
                                                              cnt2);
-    fv_note_launch(), k_res_pad<<<C, 32, 0, st>>>(a.keys(), sets, cnt2);
+    fv_note_launch(), k_res_pad<<<ctas, 32, 0, st>>>(a.keys(), sets, cnt2);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(cubt, cub_bytes, cnt, poff, (int)(items + 1), st);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(cubt, cub_bytes, cnt2, soff, (int)(nk + 1), st);
-    fv_note_launch(), k_res_halo<<<grid(items), 256, 0, st>>>(items, mask, poff, hc, hslot, a.keys(), C, soff,
-                                                              p->step_ptr);
-    int32_t h_cta[kResMaxCta + 1], h_hc[kResMaxCta], h_sptr[kResMaxCta + 1];
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_sptr, p->step_ptr, 4 * (C + 1), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_cta, p->cta_ptr, 4 * (C + 1), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_hc, hc, 4 * kResMaxCta, cudaMemcpyDeviceToHost, st);
+    fv_note_launch(), k_res_halo<<<grid(std::max<int64_t>(items, ctas + 1)), 256, 0, st>>>(
+                          n, owner, mask, poff, hc, hslot, a.keys(), C, ctas, soff, p->step_ptr);
+    int32_t h_cta[kResMaxCtas + 1], h_hc[kResMaxCtas + 1], h_sptr[kResMaxCtas + 1];
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_sptr, p->step_ptr, 4 * (ctas + 1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_cta, p->cta_ptr, 4 * (ctas + 1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_hc, hc, 4 * (ctas + 1), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail();
-    for (int c = 0; c < C; ++c) {
+    for (int c = 0; c < ctas; ++c) {
         p->cap = std::max(p->cap, h_cta[c + 1] - h_cta[c]);
         p->halo = std::max(p->halo, h_hc[c]);
     }
-    p->nslots = (int64_t)h_sptr[C] * width;
-    const bool fits = p->cap + p->halo + 2 < 65536 && res_launchable<double>(p) && res_launchable<float>(p);
+    p->nslots = (int64_t)h_sptr[ctas] * width;
+    const bool fits = !h_hc[ctas] && p->cap + p->halo + 2 < 65536 && res_launchable<double>(p) > 0 &&
+                      res_launchable<float>(p) > 0;
     if (!fits) {
         cudaFreeAsync(tmp, st);
         fv_resident_free(p);
@@ -569,7 +658,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     p->slot_dep = (uint16_t *)((char *)p->arena[1] + s_dep);
     p->slot_push = (uint32_t *)((char *)p->arena[1] + s_push);
     e = cudaMemsetAsync(p->slot_item, 0xFF, 4 * p->nslots, st);
-    fv_note_launch(), k_res_compose<<<grid(items), 256, 0, st>>>(a, p->ml, width, p->cap, sorted, item, first, soff,
+    fv_note_launch(), k_res_compose<<<grid(items), 256, 0, st>>>(a, C, p->ml, width, p->cap, sorted, item, first, soff,
                                                                  owner, p->slot_of, mask, poff, hslot, p->slot_item,
                                                                  p->slot_dep, p->slot_push, p->push);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -595,7 +684,7 @@ cudaError_t fv_resident_apply(const fv_resident *p, const void *rec, const T *r,
                               const fv_row_skip &rs, int *err, cudaStream_t st) {
     return fv_res_dispatch(p->ml, p->sets, [&](auto M, auto S) {
         cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = fv_res_config(p->C, fv_resident_smem(p, sizeof(T)), st, &at);
+        const cudaLaunchConfig_t cfg = fv_res_config(p->C, fv_resident_smem(p, sizeof(T)), st, &at, p->clusters);
         fv_note_launch();
         const cudaError_t e = cudaLaunchKernelEx(&cfg, k_resident_apply<T, M(), S()>,
                                                  fv_resident_args(p, rec, sizeof(T)), r, z, skip, rs, err);

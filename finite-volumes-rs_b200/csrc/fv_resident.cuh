@@ -60,20 +60,22 @@ constexpr size_t kResSmem = 226 * 1024;  // dynamic shared memory of a CTA (1 KB
 constexpr int kResBuffers = 4;
 constexpr int kResGroupBytes = 16 * 1024;
 
-// The plan of an apply.  Every CTA has one list of steps, the levels of its
+// The plan of an apply: one cluster for a system, or several clusters, each with
+// some of the independent problems of a batch.  Every CTA has one list of steps, the levels of its
 // rows forward and then backward; a level is one or more steps of `width`
 // slots, one row per thread, and every step ends with a barrier.
 struct fv_resident {
-    int C = 0, width = 0, sets = 0, ml = 0;  // CTAs, rows per step, thread sets (below), entries per record
+    int C = 0, clusters = 1;       // CTAs per cluster, clusters
+    int width = 0, sets = 0, ml = 0;  // rows per step, thread sets (below), entries per record
     int32_t cap = 0;               // most rows of a CTA
     int32_t halo = 0;              // most halo slots of a CTA
     int64_t nslots = 0;            // slots of all steps
     bool sorted = false;           // rows sorted by forward level
-    int32_t *cta_ptr = nullptr;    // [C + 1] first entry of a CTA in `rows`
+    int32_t *cta_ptr = nullptr;    // [clusters * C + 1] first entry of a CTA in `rows`
     int32_t *rows = nullptr;       // slot k of CTA c holds row rows[cta_ptr[c] + k]
     int32_t *nat = nullptr;        // the same rows in the caller's numbering (null: no permutation)
     uint16_t *slot_of = nullptr;   // the slot of every row in its CTA
-    int32_t *step_ptr = nullptr;   // [C + 1] first step of every CTA
+    int32_t *step_ptr = nullptr;   // [clusters * C + 1] first step of every CTA
     uint32_t *push = nullptr;      // further push targets, rank << 16 | slot
     int32_t *slot_item = nullptr;  // row (forward) or n + row (backward) of every slot, -1: idle
     uint16_t *slot_dep = nullptr;  // [ml] per slot
@@ -296,7 +298,7 @@ struct fv_res_args {
     const uint4 *rec;
     const uint32_t *push;
     const int32_t *step_ptr, *cta_ptr, *rows;  // rows: in the caller's numbering
-    int C, cap, halo, width, group;
+    int C, cap, halo, width, group;            // C: CTAs of all clusters
 };
 fv_res_args fv_resident_args(const fv_resident *p, const void *rec, size_t value_bytes);
 // Dynamic shared memory of a CTA for values of this size; the kernels run
@@ -324,7 +326,7 @@ struct fv_res_cta {
     __device__ __forceinline__ fv_res_cta(const fv_res_args &args, unsigned char *smem, unsigned long long *mbar)
         : a(args), buf(reinterpret_cast<uint4 *>(smem)), bars(mbar) {
         xs = reinterpret_cast<T *>(buf + kResBuffers * a.group * a.width * PL);
-        const unsigned c = fv_cluster_rank();
+        const unsigned c = blockIdx.x;  // cluster * C + rank
         const bool mine = c < (unsigned)a.C;
         const int r0 = mine ? a.cta_ptr[c] : 0, s0 = mine ? a.step_ptr[c] : 0;
         nr = mine ? a.cta_ptr[c + 1] - r0 : 0;
@@ -385,10 +387,11 @@ auto fv_res_dispatch(int ml, int sets, F &&f) {
     return by_sets(std::integral_constant<int, 6>());
 }
 
-// Launch configuration of a plan's kernels on one cluster of C CTAs (at: storage for its attribute).
-inline cudaLaunchConfig_t fv_res_config(int C, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
+// Launch configuration of a plan's kernels on clusters of C CTAs (at: storage for its attribute).
+inline cudaLaunchConfig_t fv_res_config(int C, size_t smem, cudaStream_t st, cudaLaunchAttribute *at,
+                                        int clusters = 1) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(C);
+    cfg.gridDim = dim3(C * clusters);
     cfg.blockDim = dim3(kResThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -400,19 +403,19 @@ inline cudaLaunchConfig_t fv_res_config(int C, size_t smem, cudaStream_t st, cud
     return cfg;
 }
 
-// Sets a kernel's launch attributes; false when the GPU cannot run such a cluster of it.
+// Sets a kernel's launch attributes; how many such clusters of it the GPU runs at once.
 template <class K>
-bool fv_res_launchable(K *k, int C, size_t smem) {
-    if (smem > kResSmem) return false;
+int fv_res_launchable(K *k, int C, size_t smem) {
+    if (smem > kResSmem) return 0;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = fv_res_config(C, smem, nullptr, &at);
     int nc = 0;
     const bool ok =
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) == cudaSuccess &&
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess && nc >= 1;
+        cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess;
     if (!ok) cudaGetLastError();
-    return ok;
+    return ok ? nc : 0;
 }
 
 // The symbolic side of a factor a plan is built from (all arrays on the device).
@@ -429,7 +432,15 @@ struct fv_resident_src {
 
 // The plan for a factor, or null when the resident sweeps do not apply (too
 // many rows or entries per row, or a shape the level-chunk sweeps serve better).
-fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out);
+// Problems of a batch: nothing couples rows of different ones.
+struct fv_resident_problems {
+    int n = 0;
+    const int64_t *offsets = nullptr;  // host, [n + 1]: the caller's rows of every problem
+    const int32_t *of_row = nullptr;   // device: the problem of every row, in the caller's numbering
+};
+// problems (optional): several clusters, each with whole problems; rows sorted by level only.
+fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
+                            const fv_resident_problems *problems = nullptr);
 void fv_resident_free(fv_resident *p);
 
 // Records of the factor's current values (rec: fv_resident_record_bytes of

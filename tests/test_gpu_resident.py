@@ -82,24 +82,35 @@ def test_resident_without_a_mesh_and_long_rows(fv, m, kind):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_resident_in_a_batch(fv, precision):
-    """Problems that converge at different iterations: converged rows are skipped the same way."""
+@pytest.mark.parametrize("sides,ordering", [((3, 9, 5), None), ((3, 9, 5), "boxes"), ((2, 1, 2, 3, 1), "boxes"),
+                                            (tuple(range(2, 20)), "boxes"), ((21, 4), "boxes")])
+def test_resident_in_a_batch(fv, precision, sides, ordering):
+    """Problems that converge at different iterations, on one cluster or several:
+    converged rows are skipped the same way; again after new values."""
     from fvb200.batch import BatchCG, MeshBatch
-    meshes = [fv.Mesh.cube(s, 0.15, 70 + s) for s in (3, 9, 5)]
+    meshes = [fv.Mesh.cube(s, 0.15, 70 + s) for s in sides]
     f = [m.fields(70, 0.1, 0.5, velocity=(1.0, 0.5, 0.25), source_uniform=True) for m in meshes]
     mb = MeshBatch(meshes)
     kf, fl, sc = (mb.face_field([q[0] for q in f]), mb.face_field([q[1] for q in f]), mb.cell_field([q[2] for q in f]))
     bc = (np.zeros(mb.n_boundary_faces), np.zeros(mb.n_boundary_faces))
-    A, b = fv.assemble(fv.convection(fv.Upwind(fl), fl) - fv.laplacian(fv.Orthogonal(), kf) - fv.source(sc), bc, mb)
-    out = []
-    for explicit in (False, True):
-        P = fv.IncompleteLowerUpper.from_matrix(A, 0)
-        if explicit:
-            P.schedule(1)
-        x = fv.DistributedVector.from_size(mb.n_cells)
-        info = BatchCG(A, mb.cell_offsets, 256).solve(P, b, x, precision=precision, solver="bicgstab")
-        out.append((x.numpy(), info["iterations"].tolist()))
-    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+    A = None
+    P = []
+    for scale in (1.0, 2.5):
+        eq = fv.convection(fv.Upwind(fl), fl) - fv.laplacian(fv.Orthogonal(), kf * scale) - fv.source(sc)
+        A, b = fv.assemble(eq, bc, mb, lhs=A)
+        out = []
+        for k, explicit in enumerate((False, True)):
+            if len(P) < 2:
+                P.append(fv.IncompleteLowerUpper.from_matrix(A, 0, ordering=ordering,
+                                                             offsets=mb.cell_offsets if ordering else None))
+                if explicit:
+                    P[k].schedule(1)
+            else:
+                P[k].refactor()
+            x = fv.DistributedVector.from_size(mb.n_cells)
+            info = BatchCG(A, mb.cell_offsets, 256).solve(P[k], b, x, precision=precision, solver="bicgstab")
+            out.append((x.numpy(), info["iterations"].tolist()))
+        assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
 
 
 @pytest.mark.parametrize("dim,side,ordering", [(2, 2, None), (2, 22, None), (2, 23, "boxes"), (2, 130, None),
