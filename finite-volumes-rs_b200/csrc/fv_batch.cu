@@ -35,6 +35,7 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
                                    const fv_row_skip *rskip);
 fv_status fv_precond_make_f32(fv_precond *P, cudaStream_t st);
 fv_status fv_precond_check_error(fv_precond *P, cudaStream_t st);
+unsigned long long fv_precond_version(const fv_precond *P);
 fv_status fv_precond_batch_prepare(fv_precond *P, int np, const int64_t *offsets, const int32_t *of_row, bool f32,
                                    cudaStream_t st);
 
@@ -698,10 +699,27 @@ struct fv_batch {
     std::vector<BProb> hs;       // the problems' state as of the end of the last begin / advance
     int64_t *seg = nullptr;      // carried-over segments (kb_adopt)
     int32_t *resume = nullptr;   // carried-over problems (kb_resume)
+    // one group of iterations of the run as a graph, replayed on a stream of its own
+    cudaGraphExec_t graph = nullptr;
+    cudaStream_t graph_stream = nullptr;
+    cudaEvent_t graph_event = nullptr, graph_flag = nullptr;
+    long long graph_launches = 0;
+    unsigned long long graph_version = 0;  // of the preconditioner it was captured with
+    BGlobal *flag = nullptr;               // pinned
 };
+
+static void drop_graph(fv_batch *B) {
+    if (B->graph) cudaGraphExecDestroy(B->graph);
+    B->graph = nullptr;
+}
 
 extern "C" fv_status fv_batch_destroy(fv_batch *B) {
     if (!B) return FV_OK;
+    drop_graph(B);
+    if (B->graph_event) cudaEventDestroy(B->graph_event);
+    if (B->graph_flag) cudaEventDestroy(B->graph_flag);
+    if (B->graph_stream) cudaStreamDestroy(B->graph_stream);
+    if (B->flag) cudaFreeHost(B->flag);
     cudaFree(B->tile_prob);
     cudaFree(B->row_prob);
     cudaFree(B->tile_row0);
@@ -1006,6 +1024,7 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
     }
     const int nfresh = np - (int)list.size();
     B->run = false;
+    drop_graph(B);
     FV_TRY(ensure_bytes(B->vec, B->vec_bytes, mixed ? sizeof(float) * 10 * (size_t)n : sizeof(double) * 9 * (size_t)n));
     FV_CUDA_TRY(cudaMemcpyAsync(B->S, hs.data(), sizeof(BProb) * np, cudaMemcpyHostToDevice, st));
     BGlobal g0{nfresh, nfresh == 0 ? 1 : 0, {0, 0}};
@@ -1068,6 +1087,75 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
     return FV_OK;
 }
 
+// Groups of iterations -- body(stream) enqueues one -- until every problem is
+// done or max_iterations are launched.  A group is captured once per run and
+// replayed (its 20-70 kernels of 3-20 us, launched one by one, left 2.4 us
+// between two), and the next replay is queued before the host looks at the
+// previous one's flag; a replay after the last problem is done finds every
+// kernel's problems done and changes nothing.  Plain launches where capture fails.
+template <class Body>
+fv_status run_groups(fv_batch *B, int group, int64_t max_iterations, cudaStream_t st, bool done, Body body) {
+    if (done || max_iterations <= 0) return FV_OK;
+    if (!B->flag && cudaHostAlloc((void **)&B->flag, sizeof(BGlobal), cudaHostAllocPortable) != cudaSuccess)
+        B->flag = nullptr;
+    if (!B->graph_stream && cudaStreamCreateWithFlags(&B->graph_stream, cudaStreamNonBlocking) != cudaSuccess)
+        B->graph_stream = nullptr;
+    for (cudaEvent_t *e : {&B->graph_event, &B->graph_flag})
+        if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) *e = nullptr;
+    cudaGetLastError();
+    cudaStream_t cs = B->graph_stream;
+    const unsigned long long version = fv_precond_version(B->P);
+    const bool able = B->flag && cs && B->graph_event && B->graph_flag && version != 0;
+    if (B->graph && B->graph_version != version) drop_graph(B);  // new factors or another schedule since
+    if (able && !B->graph) {
+        const unsigned long long c0 = fv_launches_now();
+        if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            const fv_status bs = body(cs);
+            cudaGraph_t g = nullptr;
+            const cudaError_t e = cudaStreamEndCapture(cs, &g);
+            if (bs != FV_OK || e != cudaSuccess || !g || cudaGraphInstantiate(&B->graph, g, 0) != cudaSuccess)
+                B->graph = nullptr;
+            if (g) cudaGraphDestroy(g);
+        }
+        B->graph_launches = (long long)(fv_launches_now() - c0);
+        B->graph_version = version;
+        fv_note_launches(-B->graph_launches);  // captured, not run
+        cudaGetLastError();
+    }
+    if (!able || !B->graph) {
+        for (int64_t it = 0; !done && it < max_iterations; it += group) {
+            FV_TRY(body(st));
+            B->launched += group;
+            FV_TRY(wait_all_done(B, st, done));
+        }
+        return FV_OK;
+    }
+    FV_CUDA_TRY(cudaEventRecord(B->graph_event, st));
+    FV_CUDA_TRY(cudaStreamWaitEvent(cs, B->graph_event, 0));
+    auto replay = [&]() -> fv_status {
+        FV_CUDA_TRY(cudaGraphLaunch(B->graph, cs));
+        fv_note_launches(B->graph_launches);
+        return FV_OK;
+    };
+    fv_status s = replay();
+    for (int64_t it = group; s == FV_OK; it += group) {
+        B->launched += group;
+        cudaError_t e = cudaMemcpyAsync(B->flag, B->G, sizeof(BGlobal), cudaMemcpyDeviceToHost, cs);
+        if (e == cudaSuccess) e = cudaEventRecord(B->graph_flag, cs);
+        const bool more = it < max_iterations;
+        if (e == cudaSuccess && more) s = replay();
+        if (e == cudaSuccess) e = cudaEventSynchronize(B->graph_flag);
+        if (e != cudaSuccess) {
+            fv_internal_set_cuda_error(e, "batch iterations");
+            s = FV_ERR_CUDA;
+        }
+        if (s != FV_OK || !more || ((volatile BGlobal *)B->flag)->all_done) break;
+    }
+    // what the caller's stream does next comes after the replays
+    if (cudaEventRecord(B->graph_event, cs) == cudaSuccess) cudaStreamWaitEvent(st, B->graph_event, 0);
+    return s;
+}
+
 // Up to max_iterations more iterations (whole groups) until every problem is
 // done; the problems that retired get their result, and the state is read back.
 fv_status run_advance(fv_batch *B, int64_t max_iterations, cudaStream_t st) {
@@ -1078,22 +1166,20 @@ fv_status run_advance(fv_batch *B, int64_t max_iterations, cudaStream_t st) {
     bool done = true;
     for (const BProb &q : B->hs) done = done && q.done;
     const int group = B->bicg ? kGroupBiCG : kGroupCG;
-    int64_t it = 0;
+    int64_t counted = 0;  // run_groups counts the iterations
     if (B->mixed) {
         InnerVecs<float> v = carve<float>(B->vec, n, nullptr);
         const MixedArgs mx{MixedCfg{1, B->opt.outer_tolerance, B->opt.inner_relative_tolerance}, B->x, B->b};
-        for (; !done && it < max_iterations; it += group) {
-            FV_TRY(inner_group<float>(B->bicg, B, B->P, B->a32, v, G, tl, st, B->launched, mx));
-            FV_TRY(wait_all_done(B, st, done));
-        }
+        FV_TRY(run_groups(B, group, max_iterations, st, done, [&](cudaStream_t q) {
+            return inner_group<float>(B->bicg, B, B->P, B->a32, v, G, tl, q, counted, mx);
+        }));
         fv_note_launch(), kb_finalize<float><<<G, TB, 0, st>>>(tl, v.d, nullptr, B->x, B->S);
     } else {
         InnerVecs<double> v = carve<double>(B->vec, n, B->x);
         const MixedArgs none{MixedCfg{0, 0.0, 0.0}, nullptr, nullptr};
-        for (; !done && it < max_iterations; it += group) {
-            FV_TRY(inner_group<double>(B->bicg, B, B->P, B->A->vals, v, G, tl, st, B->launched, none));
-            FV_TRY(wait_all_done(B, st, done));
-        }
+        FV_TRY(run_groups(B, group, max_iterations, st, done, [&](cudaStream_t q) {
+            return inner_group<double>(B->bicg, B, B->P, B->A->vals, v, G, tl, q, counted, none);
+        }));
         fv_note_launch(), kb_finalize<double><<<G, TB, 0, st>>>(tl, v.d, B->bicg ? v.y : nullptr, nullptr, B->S);
     }
     fv_note_launch(), kb_mark_fin<<<(B->np + 255) / 256, 256, 0, st>>>(B->np, B->S);

@@ -2108,6 +2108,19 @@ fv_status fv_precond_apply_dev_f32(fv_precond *P, const float *r, float *z, cuda
     return FV_OK;
 }
 
+// Changes when an apply would launch something else: new factors, another schedule or launch shape.
+// 0: the applies may allocate or refresh records (box tiles), so they are not captured.
+unsigned long long fv_precond_version(const fv_precond *P) {
+    if (P->kind != 3 && use_tiles(P)) return 0;
+    unsigned long long h = P->epoch + 1;
+    for (unsigned long long v : {(unsigned long long)P->f32_version, (unsigned long long)P->schedule,
+                                 (unsigned long long)P->explicit_schedule, (unsigned long long)P->sweep_blocks,
+                                 (unsigned long long)P->sweep_rpt, (unsigned long long)(size_t)P->batch_rec,
+                                 (unsigned long long)(size_t)P->batch_rec32})
+        h = h * 1000003ULL + v;
+    return h ? h : 1;
+}
+
 // Before a batch run over these problems: the plan on several clusters (once) and
 // the records of the current factors in the run's precision.  Without a plan or
 // memory for it the other sweeps run.
