@@ -325,7 +325,6 @@ __global__ void k_res_compose(ResPattern a, int C, int ml, int width, int zero, 
             } else {
                 const int64_t u = d * a.n + j;
                 c = (uint16_t)(hbase + hslot[poff[u] + __popc(mask[u] & ((1u << (o % C)) - 1u))]);
-                meta |= kResHalo;
             }
         }
         slot_dep[s * ml + q] = c;
@@ -496,9 +495,15 @@ void fv_resident_free(fv_resident *p) {
 
 size_t fv_resident_record_bytes(const fv_resident *p, size_t tb) { return (size_t)p->nslots * res_rec_bytes(p->ml, tb); }
 
-fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
-                            const fv_resident_problems *problems) {
+// How to go on when the shared memory of eight thread sets' buffers and the rows
+// does not fit: the rows over twice the CTAs (65,522-row IC(0), 362 levels: 131 ->
+// 114 us per apply), else four sets.
+enum class ResTry { kFirst, kMoreCtas, kFewerSets };
+
+static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
+                           const fv_resident_problems *problems, ResTry attempt, bool &full) {
     *out = nullptr;
+    full = false;
     const int64_t n = s.n;
     if (n <= 0 || n > (problems ? 148 : kResMaxCta) * 20000LL || s.max_side > 6 || !s.fwd_level || !s.bwd_level)
         return FV_OK;
@@ -513,11 +518,17 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     int C = 1, width = 32;
     const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
     while (C < kResMaxCta && (n > (int64_t)C * 18000 || lw > (int64_t)C * (s.sorted ? 32 : 128))) C *= 2;
+    if (attempt == ResTry::kMoreCtas && C < kResMaxCta) C *= 2;
     while (width < (s.sorted ? 256 : 128) && lw * (s.sorted ? 2 : 1) > (int64_t)C * width) width *= 2;
     std::vector<int32_t> cluster;  // of every problem
     int clusters = 1;
     if (problems) FV_TRY(res_share_problems(*problems, s.n_fwd_levels, C, width, clusters, cluster));
-    const int sets = width <= 128 ? 4 : 512 / width, ctas = C * clusters;
+    const int ml = s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6, ctas = C * clusters;
+    // Thread sets: with four, the unpacking of a record (some 500 cycles) sets the
+    // pace of a 100-cycle step; eight of up to 64 threads hide it.  Four -> eight,
+    // us per apply in natural order: 8,192-row IC(0), 128 levels, 62 -> 51;
+    // 131,072 rows, 512 levels, 158 -> 149.
+    const int sets = width > 64 ? 512 / width : attempt == ResTry::kFewerSets ? 4 : 8;
     fv_resident *p = new (std::nothrow) fv_resident();
     if (!p) return FV_ERR_ALLOC;
     p->C = C;
@@ -525,7 +536,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     p->width = width;
     p->sorted = s.sorted;
     p->sets = sets;
-    p->ml = s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6;
+    p->ml = ml;
     ResPattern a;
     a.n = n;
     a.ptr[0] = s.l_ptr, a.ptr[1] = s.u_ptr;
@@ -645,6 +656,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     const bool fits = !h_hc[ctas] && p->cap + p->halo + 2 < 65536 && res_launchable<double>(p) > 0 &&
                       res_launchable<float>(p) > 0;
     if (!fits) {
+        full = sets == 8;
         cudaFreeAsync(tmp, st);
         fv_resident_free(p);
         return FV_OK;
@@ -666,6 +678,14 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
     cudaFreeAsync(tmp, st);
     *out = p;
     return FV_OK;
+}
+
+fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
+                            const fv_resident_problems *problems) {
+    bool full;
+    FV_TRY(res_build(s, st, out, problems, ResTry::kFirst, full));
+    if (full && !problems) FV_TRY(res_build(s, st, out, problems, ResTry::kMoreCtas, full));
+    return full ? res_build(s, st, out, problems, ResTry::kFewerSets, full) : FV_OK;
 }
 
 template <typename T>

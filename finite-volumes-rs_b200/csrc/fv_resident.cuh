@@ -9,12 +9,12 @@
 // of their shared memory (st.shared::cluster), where the consumer polls its own
 // copy.  The vector is updated in place: right-hand side, forward result and
 // backward result occupy the same slot, so nothing but the factor's records
-// streams from memory.  A level costs 0.13-0.15 us: operands from shared
+// streams from memory.  A level costs 0.11-0.13 us: operands from shared
 // memory (30 cycles), the row's FP64 chain (40), one store and one barrier.
 //
 // Measured per apply (both sweeps; level chunks -> resident): 131,072-row IC(0)
-// in natural order (512 levels) 790 -> 150 us, 24,576-row ILU(0) (64 levels)
-// 140 -> 38 us, 196,608-row ILU(0) (128 levels) 247 -> 62 us; 65,522-row IC(0)
+// in natural order (512 levels) 790 -> 125 us, 24,576-row ILU(0) (64 levels)
+// 140 -> 28 us, 196,608-row ILU(0) (128 levels) 247 -> 52 us; 65,522-row IC(0)
 // in box order (18 wide levels; consecutive rows -> resident) 42 -> 25 us.
 //
 // Rows are computed with the operations of k_sweep in the same order, so the
@@ -33,10 +33,10 @@
 // unit), the shared-memory slots of its dependencies and its own, the first
 // remote reader of its value (rank << 16 | slot) and
 //   meta = offset of further readers in the push table << 8 | their number << 4
-//          | kResPush | kResHalo
+//          | kResPush
 // Unused entries have value 0 and read the slot that holds 0 (x - 0 * 0 keeps
 // every x, signed zeros included); idle lanes of a step write the slot after it.
-enum : uint32_t { kResHalo = 1, kResPush = 2 };
+enum : uint32_t { kResPush = 1 };
 template <typename T, int ML>
 struct __align__(16) fv_res_rec {
     T val[ML];
@@ -207,7 +207,7 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
         __device__ Stage() {}
     };
     Stage u;
-    unsigned a_self = 0, a_push = 0, a_dep[ML], slow = 0;
+    unsigned a_self = 0, a_push = 0, a_dep[ML], halo_deps = 0, slow = 0;
     // the set's next step: steps left of its group, that group's successor, its record's address
     int left = 0, g = 0, todo = nsteps / S;
     unsigned src = 0;
@@ -250,8 +250,12 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
         a_self = xbase + u.r.self * (unsigned)sizeof(T);
 #pragma unroll
         for (int q = 0; q < ML; ++q) a_dep[q] = xbase + u.r.dep[q] * (unsigned)sizeof(T);
-        slow = __any_sync(0xffffffffu, (u.r.meta & (kResHalo | kResPush)) != 0);
-        if (slow) a_push = fv_mapa(xbase + (u.r.push0 & 0xFFFFu) * (unsigned)sizeof(T), u.r.push0 >> 16);
+        // formed here for every row: a branch around them costs a level 0.015 us
+        a_push = fv_mapa(xbase + (u.r.push0 & 0xFFFFu) * (unsigned)sizeof(T), u.r.push0 >> 16);
+        halo_deps = 0;
+#pragma unroll
+        for (int q = 0; q < ML; ++q) halo_deps |= u.r.dep[q] >= halo0 ? 1u << q : 0u;
+        slow = __any_sync(0xffffffffu, halo_deps != 0);
     };
     if (threadIdx.x == 0)
         for (int g = 0; g < kResBuffers; ++g) copy(g);
@@ -262,28 +266,28 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
 #pragma unroll
         for (int q = 0; q < ML; ++q) fv_lds(a_dep[q], xv[q]);
         fv_lds(a_self, x);
-        if (slow) {
-            if (u.r.meta & kResHalo) {
+        if (slow) {  // a row of this warp reads another CTA's values
+            unsigned wait = 0;
+#pragma unroll
+            for (int q = 0; q < ML; ++q) wait |= (fv_is_sentinel(xv[q]) ? halo_deps : 0u) & (1u << q);
+            if (wait) {
 #pragma unroll
                 for (int q = 0; q < ML; ++q)
-                    if (u.r.dep[q] >= halo0 && fv_is_sentinel(xv[q])) xv[q] = fv_halo_value<T>(a_dep[q], err);
+                    if ((wait >> q) & 1u) xv[q] = fv_halo_value<T>(a_dep[q], err);
             }
+        }
 #pragma unroll
-            for (int q = 0; q < ML; ++q) x = x - u.r.val[q] * xv[q];
-            x = u.r.d * x;
-            fv_sts(a_self, x);
-            if (u.r.meta & kResPush) {
-                fv_push(a_push, x);
+        for (int q = 0; q < ML; ++q) x = x - u.r.val[q] * xv[q];
+        x = u.r.d * x;
+        fv_sts(a_self, x);
+        if (u.r.meta & kResPush) {
+            fv_push(a_push, x);
+            if (u.r.meta & 0xF0u) {
                 for (uint32_t e = u.r.meta >> 8, last = e + ((u.r.meta >> 4) & 15u); e < last; ++e) {
                     const uint32_t t = __ldg(&push[e]);
                     fv_push(fv_mapa(xbase + (t & 0xFFFFu) * (unsigned)sizeof(T), t >> 16), x);
                 }
             }
-        } else {
-#pragma unroll
-            for (int q = 0; q < ML; ++q) x = x - u.r.val[q] * xv[q];
-            x = u.r.d * x;
-            fv_sts(a_self, x);
         }
         if (S > 1) end_own();
         fetch();
@@ -378,6 +382,7 @@ struct fv_res_cta {
 template <typename F>
 auto fv_res_dispatch(int ml, int sets, F &&f) {
     auto by_sets = [&](auto M) {
+        if (sets == 8) return f(M, std::integral_constant<int, 8>());
         if (sets == 4) return f(M, std::integral_constant<int, 4>());
         if (sets == 2) return f(M, std::integral_constant<int, 2>());
         return f(M, std::integral_constant<int, 1>());

@@ -139,3 +139,13 @@ def test_resident_solve_equals_kernels(fv, dim, side, ordering):
         assert np.array_equal(got[0][0], got[1][0], equal_nan=True)
         assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
         assert np.array_equal(got[0][2:], got[1][2:], equal_nan=True)
+
+
+@pytest.mark.parametrize("side", [128, 181, 362, 392])
+def test_resident_where_shared_memory_fills(fv, side):
+    """Long natural orders whose rows and eight sets' buffers fit, fit on twice the
+    CTAs, fit the largest cluster, or leave four sets: the same bits."""
+    case = diffusion_2d(fv, side, seed=65)
+    A, _ = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    P, Q = _pair(fv, fv.IncompleteCholesky, A)
+    _same_apply(fv, P, Q, case["mesh"].n_cells)
