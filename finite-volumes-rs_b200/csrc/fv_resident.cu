@@ -523,7 +523,9 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     std::vector<int32_t> cluster;  // of every problem
     int clusters = 1;
     if (problems) FV_TRY(res_share_problems(*problems, s.n_fwd_levels, C, width, clusters, cluster));
-    const int ml = s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6, ctas = C * clusters;
+    // entries per record: a padded one costs a dependent subtraction (131,072-row
+    // IC(0) in natural order with 3 and 2 per side: 149 and 140 us per apply)
+    const int ml = s.max_side <= 2 ? 2 : s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6, ctas = C * clusters;
     // Thread sets: with four, the unpacking of a record (some 500 cycles) sets the
     // pace of a 100-cycle step; eight of up to 64 threads hide it.  Four -> eight,
     // us per apply in natural order: 8,192-row IC(0), 128 levels, 62 -> 51;

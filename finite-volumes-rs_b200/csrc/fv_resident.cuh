@@ -13,7 +13,7 @@
 // memory (30 cycles), the row's FP64 chain (40), one store and one barrier.
 //
 // Measured per apply (both sweeps; level chunks -> resident): 131,072-row IC(0)
-// in natural order (512 levels) 790 -> 125 us, 24,576-row ILU(0) (64 levels)
+// in natural order (512 levels) 790 -> 117 us, 24,576-row ILU(0) (64 levels)
 // 140 -> 28 us, 196,608-row ILU(0) (128 levels) 247 -> 52 us; 65,522-row IC(0)
 // in box order (18 wide levels; consecutive rows -> resident) 42 -> 25 us.
 //
@@ -45,7 +45,7 @@ struct __align__(16) fv_res_rec {
     uint16_t self;
     uint32_t push0, meta;
 };
-static_assert(sizeof(fv_res_rec<double, 3>) == 48 && sizeof(fv_res_rec<double, 4>) == 64 &&
+static_assert(sizeof(fv_res_rec<double, 2>) == 48 && sizeof(fv_res_rec<double, 3>) == 48 && sizeof(fv_res_rec<double, 4>) == 64 &&
                   sizeof(fv_res_rec<double, 6>) == 80 && sizeof(fv_res_rec<float, 3>) == 32,
               "record sizes are multiples of 16");
 
@@ -387,6 +387,7 @@ auto fv_res_dispatch(int ml, int sets, F &&f) {
         if (sets == 2) return f(M, std::integral_constant<int, 2>());
         return f(M, std::integral_constant<int, 1>());
     };
+    if (ml == 2) return by_sets(std::integral_constant<int, 2>());
     if (ml == 3) return by_sets(std::integral_constant<int, 3>());
     if (ml == 4) return by_sets(std::integral_constant<int, 4>());
     return by_sets(std::integral_constant<int, 6>());
