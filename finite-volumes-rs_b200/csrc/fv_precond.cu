@@ -1389,12 +1389,21 @@ static fv_status tile_prepare(fv_precond *P, cudaStream_t st) {
     T **rhs = reinterpret_cast<T **>(sizeof(T) == 8 ? (void **)P->t_rhs64 : (void **)P->t_rhs32);
     const unsigned version = sizeof(T) == 8 ? P->epoch : P->f32_version;
     unsigned &seen = sizeof(T) == 8 ? P->t_rec64_epoch : P->t_rec32_version;
-    for (int d = 0; d < 2; ++d) {
-        if (!rec[d]) {
-            FV_CUDA_TRY(fv_block_alloc(&rec[d], sizeof(TileRec<T>) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
-            FV_CUDA_TRY(fv_block_alloc(&rhs[d], sizeof(T) * (s->t_nslots[d] ? s->t_nslots[d] : 1)));
-            seen = version - 1;
+    if (!rec[0] || !rhs[0] || !rec[1] || !rhs[1]) {
+        // Not while the stream is captured, where cudaMalloc fails but a kept
+        // block would be handed out: the solve then runs without a graph.
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        FV_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) {
+            fv_internal_set_cuda_error(cudaErrorStreamCaptureUnsupported, "box tiles' first apply");
+            return FV_ERR_CUDA;
         }
+        for (int d = 0; d < 2; ++d) {
+            const int64_t slots = s->t_nslots[d] ? s->t_nslots[d] : 1;
+            if (!rec[d]) FV_CUDA_TRY(fv_block_alloc(&rec[d], sizeof(TileRec<T>) * slots));
+            if (!rhs[d]) FV_CUDA_TRY(fv_block_alloc(&rhs[d], sizeof(T) * slots));
+        }
+        seen = version - 1;
     }
     if (seen != version) {
         const T *lv, *uv, *dv;

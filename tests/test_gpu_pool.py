@@ -44,3 +44,23 @@ def test_blocks_reused_across_threads_and_streams(fv):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("n", [6, 12])
+def test_kept_blocks_are_not_taken_while_a_solve_is_captured(fv, n):
+    """Box tiles allocate at their first apply, which a solve captures: blocks kept
+    from an earlier object must not be handed out there, in part or in whole."""
+    case = convdiff_3d(fv, n, seed=6)
+    A, b = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    opts = fv.LinearSolverOptions(1e-10, 1e-10, 2000)
+    got = []
+    for req in (1, 2, 2, 2):
+        P = fv.IncompleteLowerUpper.from_matrix(A, 0)
+        P.schedule(req)
+        for _ in range(2):
+            x = fv.DistributedVector.from_size(A.nrows())
+            fv.bi_conjugate_gradient_stab(x, A, b, P, None, opts)
+            got.append(x.numpy())
+        P.close()
+    for x in got[1:]:
+        assert np.array_equal(x, got[0])
