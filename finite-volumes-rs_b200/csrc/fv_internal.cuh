@@ -221,16 +221,66 @@ __device__ __forceinline__ unsigned fv_pack_value(float v) {
     return b == FV_SENTINEL_U32 ? 0x7FC00000u : b;
 }
 
-// Reads *p; whether it holds a produced value.
-__device__ __forceinline__ bool fv_slot_ready(const double *p, double &v) {
-    unsigned long long b = fv_ld_relaxed_u64(p);
-    v = __longlong_as_double((long long)b);
-    return b != FV_SENTINEL_U64;
+__device__ __forceinline__ bool fv_is_sentinel(double v) {
+    return (unsigned long long)__double_as_longlong(v) == FV_SENTINEL_U64;
 }
-__device__ __forceinline__ bool fv_slot_ready(const float *p, float &v) {
-    unsigned b = fv_ld_relaxed_u32(p);
+__device__ __forceinline__ bool fv_is_sentinel(float v) { return __float_as_uint(v) == FV_SENTINEL_U32; }
+__device__ __forceinline__ double fv_sentinel(double) { return __longlong_as_double(-1LL); }
+__device__ __forceinline__ float fv_sentinel(float) { return __uint_as_float(FV_SENTINEL_U32); }
+
+// Reads *p into v where v is still the sentinel; no branch, so that the polls of
+// a row's slots are in flight together.
+__device__ __forceinline__ void fv_slot_poll(const double *p, double &v) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    asm volatile("{\n.reg .pred q;\nsetp.eq.u64 q, %0, 0xFFFFFFFFFFFFFFFF;\n@q ld.relaxed.gpu.global.u64 %0, [%1];\n}"
+                 : "+l"(b)
+                 : "l"(p)
+                 : "memory");
+    v = __longlong_as_double((long long)b);
+}
+__device__ __forceinline__ void fv_slot_poll(const unsigned *p, unsigned &v) {
+    asm volatile("{\n.reg .pred q;\nsetp.eq.u32 q, %0, 0xFFFFFFFF;\n@q ld.relaxed.gpu.global.u32 %0, [%1];\n}"
+                 : "+r"(v)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void fv_slot_poll(const float *p, float &v) {
+    unsigned b = __float_as_uint(v);
+    fv_slot_poll(reinterpret_cast<const unsigned *>(p), b);
     v = __uint_as_float(b);
-    return b != FV_SENTINEL_U32;
+}
+
+// xv[q] = x[c[q]] where xv[q] holds the sentinel, once all are produced.  Gives up (NaN for the missing
+// ones, FV_DEV_TIMEOUT in *err) after FV_WAIT_LIMIT_NS, or as soon as another
+// thread has raised an error.
+template <int N, typename T>
+__device__ __forceinline__ void fv_wait_slots(const T *x, const int (&c)[N], T (&xv)[N], int *err) {
+    unsigned long long t0 = 0;
+    for (unsigned it = 0;; ++it) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) fv_slot_poll(&x[c[q]], xv[q]);
+        bool pending = false;
+#pragma unroll
+        for (int q = 0; q < N; ++q) pending |= fv_is_sentinel(xv[q]);
+        if (!pending) return;
+        if ((it & 255u) == 255u) {
+            if (!t0) t0 = fv_globaltimer();
+            if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
+                if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
+#pragma unroll
+                for (int q = 0; q < N; ++q)
+                    if (fv_is_sentinel(xv[q])) xv[q] = T(NAN);
+                return;
+            }
+        }
+    }
+}
+// The first m of them.
+template <int N, typename T>
+__device__ __forceinline__ void fv_wait_slots(const T *x, const int (&c)[N], int m, T (&xv)[N], int *err) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) xv[q] = q < m ? fv_sentinel(T(0)) : T(0);
+    fv_wait_slots(x, c, xv, err);
 }
 
 // Wait until *p holds a produced value.  Gives up (returns NaN and raises

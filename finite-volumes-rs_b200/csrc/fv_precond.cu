@@ -512,8 +512,9 @@ __global__ void __launch_bounds__(128) k_ilu0(int64_t n, const int32_t *__restri
 // mutually adjacent cells that is u_ki alone -- and then polls just those and
 // the u_kk, all together.  A level costs one store and one L2 read (flags:
 // fence, flag store, flag read, value read).  1.57M rows, 256 levels: 1.24 ms
-// with flags and all of U_k loaded, 0.59 ms this way; 5.3M rows in box order (28
-// levels): 0.79 -> 0.28 ms.
+// with flags and all of U_k loaded, 0.36 ms this way; 5.3M rows in box order (28
+// levels): 0.79 -> 0.22 ms.  (The polls of a round have no branch between them:
+// one after the other they cost 0.59 and 0.28 ms.)
 template <int MAXR>
 __global__ void __launch_bounds__(128) k_ilu0s(int64_t n, const int32_t *__restrict__ order,
                                                const int32_t *__restrict__ a_ptr, const double *__restrict__ a_val,
@@ -560,29 +561,32 @@ __global__ void __launch_bounds__(128) k_ilu0s(int64_t n, const int32_t *__restr
                     }
             }
         }
-        // poll (bounded): bit q of pend_d the pivots, bit q * MAXR + p of pend_u the entries
-        double dk[MAXR], uv[MAXR][MAXR];
-        unsigned pend_d = 0;
-        unsigned long long pend_u = 0;
+        // the pivots and entries of the dependencies: all polls of a round in flight together (bounded)
+        double dk[MAXR - 1], uv[MAXR - 1][MAXR];
+        const double none = fv_sentinel(0.0);
 #pragma unroll
-        for (int q = 0; q < MAXR - 1; ++q)
-            if (q < nl) {
-                pend_d |= 1u << q;
+        for (int q = 0; q < MAXR - 1; ++q) {
+            dk[q] = q < nl ? none : 0.0;
 #pragma unroll
-                for (int p = q + 1; p < MAXR; ++p)
-                    if (pos[q][p] >= 0) pend_u |= 1ULL << (q * MAXR + p);
-            }
+            for (int p = q + 1; p < MAXR; ++p) uv[q][p] = q < nl && pos[q][p] >= 0 ? none : 0.0;
+        }
         unsigned long long t0 = 0;
-        for (unsigned it = 0; pend_d | pend_u; ++it) {
+        for (unsigned it = 0;; ++it) {
 #pragma unroll
             for (int q = 0; q < MAXR - 1; ++q) {
-                if (((pend_d >> q) & 1u) && fv_slot_ready(&diag[c[q]], dk[q])) pend_d &= ~(1u << q);
+                fv_slot_poll(&diag[c[q]], dk[q]);
 #pragma unroll
-                for (int p = q + 1; p < MAXR; ++p)
-                    if (((pend_u >> (q * MAXR + p)) & 1u) && fv_slot_ready(&u_val[pos[q][p]], uv[q][p]))
-                        pend_u &= ~(1ULL << (q * MAXR + p));
+                for (int p = q + 1; p < MAXR; ++p) fv_slot_poll(&u_val[pos[q][p]], uv[q][p]);
             }
-            if ((it & 255u) == 255u && (pend_d | pend_u)) {
+            bool pending = false;
+#pragma unroll
+            for (int q = 0; q < MAXR - 1; ++q) {
+                pending |= fv_is_sentinel(dk[q]);
+#pragma unroll
+                for (int p = q + 1; p < MAXR; ++p) pending |= fv_is_sentinel(uv[q][p]);
+            }
+            if (!pending) break;
+            if ((it & 255u) == 255u) {
                 if (!t0) t0 = fv_globaltimer();
                 if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
                     if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(128) k_ic0(int64_t n, const int32_t *__restric
 // k_ic0 for short rows, with the values as their own readiness like k_ilu0s:
 // l_val and dinv start as sentinels, a row polls dinv_j of its dependencies and
 // the l_jk with k in its own pattern (none on a mesh without triangles of
-// mutually adjacent cells).  131,072 rows, 512 levels: 1.41 -> 0.49 ms.
+// mutually adjacent cells).  131,072 rows, 512 levels: 1.41 -> 0.30 ms.
 template <int MAXR>
 __global__ void __launch_bounds__(128) k_ic0s(int64_t n, const int32_t *__restrict__ order,
                                               const int32_t *__restrict__ a_ptr, const double *__restrict__ a_val,
@@ -726,26 +730,30 @@ __global__ void __launch_bounds__(128) k_ic0s(int64_t n, const int32_t *__restri
             }
         }
         double dj[ML], lv[ML][ML];
-        unsigned pend_d = 0, pend_l = 0;
+        const double none = fv_sentinel(0.0);
 #pragma unroll
-        for (int q = 0; q < ML; ++q)
-            if (q < nl) {
-                pend_d |= 1u << q;
+        for (int q = 0; q < ML; ++q) {
+            dj[q] = q < nl ? none : 0.0;
 #pragma unroll
-                for (int p = 0; p < q; ++p)
-                    if (pos[q][p] >= 0) pend_l |= 1u << (q * ML + p);
-            }
+            for (int p = 0; p < q; ++p) lv[q][p] = q < nl && pos[q][p] >= 0 ? none : 0.0;
+        }
         unsigned long long t0 = 0;
-        for (unsigned it = 0; pend_d | pend_l; ++it) {
+        for (unsigned it = 0;; ++it) {
 #pragma unroll
             for (int q = 0; q < ML; ++q) {
-                if (((pend_d >> q) & 1u) && fv_slot_ready(&dinv[c[q]], dj[q])) pend_d &= ~(1u << q);
+                fv_slot_poll(&dinv[c[q]], dj[q]);
 #pragma unroll
-                for (int p = 0; p < q; ++p)
-                    if (((pend_l >> (q * ML + p)) & 1u) && fv_slot_ready(&l_val[pos[q][p]], lv[q][p]))
-                        pend_l &= ~(1u << (q * ML + p));
+                for (int p = 0; p < q; ++p) fv_slot_poll(&l_val[pos[q][p]], lv[q][p]);
             }
-            if ((it & 255u) == 255u && (pend_d | pend_l)) {
+            bool pending = false;
+#pragma unroll
+            for (int q = 0; q < ML; ++q) {
+                pending |= fv_is_sentinel(dj[q]);
+#pragma unroll
+                for (int p = 0; p < q; ++p) pending |= fv_is_sentinel(lv[q][p]);
+            }
+            if (!pending) break;
+            if ((it & 255u) == 255u) {
                 if (!t0) t0 = fv_globaltimer();
                 if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
                     if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
@@ -817,8 +825,11 @@ __global__ void k_count_dropped(int64_t nl, const double *__restrict__ l_val, in
 //
 // Everything a row needs apart from its dependencies' values (its position in
 // the level order, row bounds, columns, coefficients, rhs, 1/diagonal) is
-// loaded before the first wait, and all dependencies are polled together, so
-// the critical path from one level to the next is one store plus one L2 read.
+// loaded before the first wait, and all dependencies are polled together
+// (fv_wait_slots), so the critical path from one level to the next is one store
+// plus one L2 read.  With a branch after every poll their round trips added up:
+// 1.57M-row ILU(0) of 256 levels 256 -> 203 us per sweep, 131,072-row IC(0) of
+// 512 levels 811 -> 591 us per apply.
 // MAXL bounds the off-diagonal count of a row on the swept side; rows are
 // held in registers.
 // The permutation of a reordered factorisation (fv_ilu0_factor_perm and
@@ -862,28 +873,7 @@ __global__ void __launch_bounds__(256) k_sweep(int64_t n, const int32_t *__restr
             }
         T s = rhs[pm.gather ? nat : i];
         const T d = UNIT ? T(1) : __ldg(&dinv[i]);
-        unsigned pending = 0;
-#pragma unroll
-        for (int q = 0; q < MAXL; ++q)
-            if (q < m && !fv_slot_ready(&x[c[q]], xv[q])) pending |= 1u << q;
-        if (pending) {
-            const unsigned long long t0 = fv_globaltimer();
-            for (unsigned it = 1; pending; ++it) {
-#pragma unroll
-                for (int q = 0; q < MAXL; ++q)
-                    if ((pending >> q) & 1u)
-                        if (fv_slot_ready(&x[c[q]], xv[q])) pending &= ~(1u << q);
-                if (pending && (it & 255u) == 0) {
-                    if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
-                        if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
-#pragma unroll
-                        for (int q = 0; q < MAXL; ++q)
-                            if ((pending >> q) & 1u) xv[q] = T(NAN);
-                        pending = 0;
-                    }
-                }
-            }
-        }
+        fv_wait_slots(x, c, m, xv, err);
 #pragma unroll
         for (int q = 0; q < MAXL; ++q)
             if (q < m) s = s - v[q] * xv[q];
@@ -958,28 +948,7 @@ __global__ void __launch_bounds__(256) k_sweep_pf(int64_t n, const int32_t *__re
         if (have_next) sweep_stage<T, UNIT, MAXL>(b, next, n, order, ptr, col, val, dinv, rhs, rs, pm);
         if (a.live) {
             T xv[MAXL];
-            unsigned pending = 0;
-#pragma unroll
-            for (int q = 0; q < MAXL; ++q)
-                if (q < a.m && !fv_slot_ready(&x[a.c[q]], xv[q])) pending |= 1u << q;
-            if (pending) {
-                const unsigned long long t0 = fv_globaltimer();
-                for (unsigned it = 1; pending; ++it) {
-#pragma unroll
-                    for (int q = 0; q < MAXL; ++q)
-                        if ((pending >> q) & 1u)
-                            if (fv_slot_ready(&x[a.c[q]], xv[q])) pending &= ~(1u << q);
-                    if (pending && (it & 255u) == 0) {
-                        if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
-                            if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
-#pragma unroll
-                            for (int q = 0; q < MAXL; ++q)
-                                if ((pending >> q) & 1u) xv[q] = T(NAN);
-                            pending = 0;
-                        }
-                    }
-                }
-            }
+            fv_wait_slots(x, a.c, a.m, xv, err);
             T s = a.s;
 #pragma unroll
             for (int q = 0; q < MAXL; ++q)
@@ -1074,28 +1043,7 @@ __global__ void __launch_bounds__(256, RPT == 1 ? 5 : 1) k_sweep_seq(int64_t n, 
         for (int q = 0; q < RPT; ++q) {
             if (m[q] < 0) continue;
             T xv[MAXL];
-            unsigned pending = 0;
-#pragma unroll
-            for (int t = 0; t < MAXL; ++t)
-                if (t < m[q] && !fv_slot_ready(&x[c[q][t]], xv[t])) pending |= 1u << t;
-            if (pending) {
-                const unsigned long long t0 = fv_globaltimer();
-                for (unsigned it = 1; pending; ++it) {
-#pragma unroll
-                    for (int t = 0; t < MAXL; ++t)
-                        if ((pending >> t) & 1u)
-                            if (fv_slot_ready(&x[c[q][t]], xv[t])) pending &= ~(1u << t);
-                    if (pending && (it & 255u) == 0) {
-                        if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
-                            if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
-#pragma unroll
-                            for (int t = 0; t < MAXL; ++t)
-                                if ((pending >> t) & 1u) xv[t] = T(NAN);
-                            pending = 0;
-                        }
-                    }
-                }
-            }
+            fv_wait_slots(x, c[q], m[q], xv, err);
             T s = sr[q];
 #pragma unroll
             for (int t = 0; t < MAXL; ++t)
@@ -1321,30 +1269,9 @@ __global__ void __launch_bounds__(kTileWarps * 32) k_sweep_tiled(int64_t nb, con
             issue(st + kTileDepth, bi);
             if (r.row >= 0) {
                 T xv[FV_TILE_MAXL];
-                unsigned pending = 0;
 #pragma unroll
-                for (int q = 0; q < FV_TILE_MAXL; ++q) {
-                    xv[q] = T(0);
-                    if (r.ds[q] >= 0 && !fv_slot_ready(&x[r.ds[q]], xv[q])) pending |= 1u << q;
-                }
-                if (pending) {
-                    const unsigned long long t0 = fv_globaltimer();
-                    for (unsigned it = 1; pending; ++it) {
-#pragma unroll
-                        for (int q = 0; q < FV_TILE_MAXL; ++q)
-                            if ((pending >> q) & 1u)
-                                if (fv_slot_ready(&x[r.ds[q]], xv[q])) pending &= ~(1u << q);
-                        if (pending && (it & 255u) == 0) {
-                            if (*(volatile int *)err || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) {
-                                if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
-#pragma unroll
-                                for (int q = 0; q < FV_TILE_MAXL; ++q)
-                                    if ((pending >> q) & 1u) xv[q] = T(NAN);
-                                pending = 0;
-                            }
-                        }
-                    }
-                }
+                for (int q = 0; q < FV_TILE_MAXL; ++q) xv[q] = r.ds[q] >= 0 ? fv_sentinel(T(0)) : T(0);
+                fv_wait_slots(x, r.ds, xv, err);
                 T s = rh;
 #pragma unroll
                 for (int q = 0; q < FV_TILE_MAXL; ++q)
@@ -1531,7 +1458,7 @@ __global__ void k_sym_split(int64_t n, const int32_t *__restrict__ ptr, const in
 // for the upper part), so a chunk's rows depend on each other: rows of at most
 // MAXL entries poll the dependencies outside the chunk together and pass the
 // levels inside it through shuffles, so a chunk costs one hand-off through L2
-// where a level did (131,072 rows of 512 levels: 1.51 -> 0.19 ms).  Longer rows
+// where a level did (131,072 rows of 512 levels: 1.51 -> 0.17 ms).  Longer rows
 // (MAXL = 0) wait for one dependency after the other.  Bounded waits as in the
 // sweeps.
 template <int MAXL>
@@ -1557,10 +1484,12 @@ __global__ void __launch_bounds__(256) k_sym_levels(int64_t n, int upper, const 
         };
         if constexpr (MAXL > 0) {
             int c[MAXL], src[MAXL];
-            unsigned pending = 0, inside = 0;
+            unsigned v[MAXL], inside = 0, outside = 0;  // v: levels of the rows outside the chunk, the sentinel until known
 #pragma unroll
             for (int q = 0; q < MAXL; ++q) {
                 src[q] = 0;
+                c[q] = 0;
+                v[q] = 0;
                 if (q < m) {
                     c[q] = __ldg(&col[k0 + q]);
                     const int64_t at = (upper ? n - 1 - c[q] : (int64_t)c[q]) - chunk * 32;  // below 32: an earlier row
@@ -1568,22 +1497,22 @@ __global__ void __launch_bounds__(256) k_sym_levels(int64_t n, int upper, const 
                         src[q] = (int)at;
                         inside |= 1u << q;
                     } else {
-                        pending |= 1u << q;
+                        v[q] = FV_SENTINEL_U32;
+                        outside |= 1u << q;
                     }
                 }
             }
-            for (unsigned it = 0; pending; ++it) {
+            for (unsigned it = 0;; ++it) {
 #pragma unroll
-                for (int q = 0; q < MAXL; ++q)
-                    if ((pending >> q) & 1u) {
-                        const unsigned v = fv_ld_relaxed_u32(&level[c[q]]);
-                        if (v != 0xFFFFFFFFu) {
-                            lev = max(lev, (int)v + 1);
-                            pending &= ~(1u << q);
-                        }
-                    }
-                if (pending && gave_up(it)) break;
+                for (int q = 0; q < MAXL; ++q) fv_slot_poll(reinterpret_cast<const unsigned *>(&level[c[q]]), v[q]);
+                bool pending = false;
+#pragma unroll
+                for (int q = 0; q < MAXL; ++q) pending |= v[q] == FV_SENTINEL_U32;
+                if (!pending || gave_up(it)) break;
             }
+#pragma unroll
+            for (int q = 0; q < MAXL; ++q)
+                if ((outside >> q) & 1u) lev = max(lev, (int)v[q] + 1);
             __syncwarp();
             bool known = inside == 0;
             unsigned mask = __ballot_sync(0xffffffffu, known);
@@ -1592,10 +1521,10 @@ __global__ void __launch_bounds__(256) k_sym_levels(int64_t n, int upper, const 
                 bool all = true;
 #pragma unroll
                 for (int q = 0; q < MAXL; ++q) {
-                    const int v = __shfl_sync(0xffffffffu, lev, src[q]);
+                    const int at = __shfl_sync(0xffffffffu, lev, src[q]);
                     if ((inside >> q) & 1u) {
                         all = all && ((mask >> src[q]) & 1u);
-                        best = max(best, v + 1);
+                        best = max(best, at + 1);
                     }
                 }
                 if (!known && all) {
@@ -2294,12 +2223,16 @@ static fv_status factor_common(const fv_csr *Ac, int kind, cudaStream_t st, fv_p
         FV_CUDA_TRY(cudaMemsetAsync(P->done, 0, sizeof(unsigned) * n, st));
         P->epoch = 1;
     }
-    // 128-thread blocks: as many as the level chunks run, or all that fit where
-    // the levels are few and wide (rows sorted by level)
-    const int G = P->contiguous ? (int)std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, 148 * 16))
-                                : sweep_grid(n) * 2;
-    const int32_t *order = P->contiguous ? nullptr : sym->fwd_order;
+    // 128-thread blocks: all that fit where the levels are few and wide (rows
+    // sorted by level); else, for short rows, the chunks of two levels, since
+    // further pollers only slow the frontier's reads (1.57M rows of 256 levels: 363
+    // us with 148 blocks, 380 with 296, 441 with 592, 562 with 1,184; 131,072 rows
+    // of 512 levels: 297, 311, 341, 352)
     const int mr = sym->max_row;
+    const int64_t two_levels = std::max<int64_t>(148, n / std::max(1, sym->n_fwd_levels) * 2 / 128);
+    const int64_t chunk_blocks = mr <= 6 ? std::min<int64_t>(two_levels, sweep_grid(n) * 2) : sweep_grid(n) * 2;
+    const int G = (int)(P->contiguous ? std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, 148 * 16)) : chunk_blocks);
+    const int32_t *order = P->contiguous ? nullptr : sym->fwd_order;
     if (mr <= 6) {  // the short-row kernels' values are their own readiness
         double *polled = kind == 2 ? P->u_val : P->l_val;
         const int64_t np = kind == 2 ? sym->nnz_u : sym->nnz_l;

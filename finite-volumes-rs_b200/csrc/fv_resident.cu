@@ -508,13 +508,18 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     if (n <= 0 || n > (problems ? 148 : kResMaxCta) * 20000LL || s.max_side > 6 || !s.fwd_level || !s.bwd_level)
         return FV_OK;
     if (problems && !s.sorted) return FV_OK;
+    // Rows sorted by level in one cluster: few wide levels, which more than 5,000
+    // rows a CTA take longer than consecutive rows on all SMs.  us per apply with
+    // 23 of launch and check, resident against consecutive: 32,768-row IC(0) 40 52,
+    // 65,522 rows 50 55, 131,072 rows 60 49; ILU(0) 24,576 rows 47 62, 82,944 62 62.
+    if (s.sorted && !problems && n > kResMaxCta * 5000LL) return FV_OK;
     // CTAs: enough shared memory for the rows, and as few as keep a level of a
     // CTA within 128 rows (natural order: more CTAs only add hand-offs) or as
     // many as leave it 32 (rows sorted by level: few, wide levels).  Measured as
     // us per apply, the launch and its status check (23 us) included:
     // 48,000-row ILU(0), natural, C x width: 4x128 84, 8x128 84, 16x64 96,
-    // 16x32 100 (level chunks 209); 32,768-row IC(0), sorted: 16x256 36, 16x128
-    // 38, 8x128 46, 8x64 48 (consecutive rows 58).
+    // 16x32 100; 32,768-row IC(0), sorted: 16x256 36, 16x128
+    // 38, 8x128 46, 8x64 48 (consecutive rows 52).
     int C = 1, width = 32;
     const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
     while (C < kResMaxCta && (n > (int64_t)C * 18000 || lw > (int64_t)C * (s.sorted ? 32 : 128))) C *= 2;

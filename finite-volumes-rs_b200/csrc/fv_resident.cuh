@@ -13,9 +13,9 @@
 // memory (30 cycles), the row's FP64 chain (40), one store and one barrier.
 //
 // Measured per apply (both sweeps; level chunks -> resident): 131,072-row IC(0)
-// in natural order (512 levels) 790 -> 117 us, 24,576-row ILU(0) (64 levels)
-// 140 -> 28 us, 196,608-row ILU(0) (128 levels) 247 -> 52 us; 65,522-row IC(0)
-// in box order (18 wide levels; consecutive rows -> resident) 42 -> 25 us.
+// in natural order (512 levels) 568 -> 117 us, 24,576-row ILU(0) (64 levels)
+// 100 -> 28 us, 196,608-row ILU(0) (128 levels) 190 -> 52 us; 65,522-row IC(0)
+// in box order (18 wide levels; consecutive rows -> resident) 32 -> 27 us.
 //
 // Rows are computed with the operations of k_sweep in the same order, so the
 // results are the same bits.
@@ -113,12 +113,6 @@ __device__ __forceinline__ bool fv_halo_ready(unsigned addr, float &v) {
     v = __uint_as_float(b);
     return b != FV_SENTINEL_U32;
 }
-__device__ __forceinline__ bool fv_is_sentinel(double v) {
-    return (unsigned long long)__double_as_longlong(v) == FV_SENTINEL_U64;
-}
-__device__ __forceinline__ bool fv_is_sentinel(float v) { return __float_as_uint(v) == FV_SENTINEL_U32; }
-__device__ __forceinline__ double fv_sentinel(double) { return __longlong_as_double(-1LL); }
-__device__ __forceinline__ float fv_sentinel(float) { return __uint_as_float(FV_SENTINEL_U32); }
 
 // The value of a halo slot, waited for (bounded like fv_wait_value).
 template <typename T>

@@ -1055,7 +1055,8 @@ fv_status loop_resident(const Workspace &w, const fv_csr *A, fv_precond *P, doub
     // Up to where whole iterations in one cluster beat kernels on all SMs, us per
     // iteration (resident / kernels): CG natural 32,768 rows 95 / 102, 45,000
     // 132 / 126; CG in box order 65,522 rows 47 / 55, 96,800 57 / 55; BiCGStab
-    // natural 48,000 rows 155 / 180, 82,944 223 / 177; 2,048 rows 32 / 49.
+    // natural 48,000 rows 155 / 180, 82,944 223 / 177; 2,048 rows 32 / 49 (with
+    // sweeps of 0.14 us per level on both sides, now 0.11).
     const int64_t most = BICG ? 50000 : plan && plan->sorted ? 75000 : 36000;
     if (!plan || A->nrows > most) return FV_OK;
     const size_t smem = kRsBytes + fv_resident_smem(plan, sizeof(double));

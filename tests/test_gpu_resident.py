@@ -149,3 +149,13 @@ def test_resident_where_shared_memory_fills(fv, side):
     A, _ = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
     P, Q = _pair(fv, fv.IncompleteCholesky, A)
     _same_apply(fv, P, Q, case["mesh"].n_cells)
+
+
+@pytest.mark.parametrize("side", [200, 201])
+def test_resident_up_to_its_rows_in_level_order(fv, side):
+    """80,000 rows sorted by level and just above: the cluster's sweeps, then
+    consecutive rows on all SMs; the same bits."""
+    case = diffusion_2d(fv, side, seed=66)
+    A, _ = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    P, Q = _pair(fv, fv.IncompleteCholesky, A.permuted(fv.order_boxes(A)[0]))
+    _same_apply(fv, P, Q, case["mesh"].n_cells)
