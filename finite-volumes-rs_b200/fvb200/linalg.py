@@ -384,7 +384,9 @@ class Preconditioner:
         return fl, bl, nf.value, nb.value
 
     def schedule(self, request: int = -1):
-        """Sweep schedule: request -1 = query, 0 or 1 = level chunks (default),
+        """Sweep schedule.  Without a request, systems that fit one cluster's
+        shared memory are swept there; a request (0 included) takes the kernels
+        it names: -1 = query, 0 or 1 = level chunks (default of larger systems),
         2 = box tiles (matrices assembled on a mesh), 3 = level chunks with
         the next chunk prefetched, 4 = consecutive rows (the default when the
         rows are sorted by level, e.g. a matrix permuted by order_boxes'

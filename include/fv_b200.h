@@ -352,8 +352,11 @@ fv_status fv_precond_export(const fv_precond *P, int64_t *nnz, int32_t *row_ptr,
 /* Level schedules: level of every row in the forward (lower) and backward (upper) DAG. */
 fv_status fv_precond_levels(const fv_precond *P, int32_t *fwd_level, int32_t *bwd_level,
                             int32_t *n_fwd_levels, int32_t *n_bwd_levels, void *stream);
-/* Sweep schedule of P.  request: -1 query only; 0 or 1 level chunks (the
- * default for rows not sorted by level); 2 box tiles, available when the
+/* Sweep schedule of P.  Without a request, systems that fit one thread-block
+ * cluster's shared memory (up to 320,000 rows, 80,000 sorted by level) are swept
+ * there; a request, 0 included, takes the kernels it names from then on.
+ * request: -1 query only (the schedule of larger systems); 0 or 1 level chunks
+ * (their default for rows not sorted by level); 2 box tiles, available when the
  * matrix was assembled on a mesh whose box order exists (FV_ERR_UNSUPPORTED
  * otherwise); 3 level chunks with each warp loading its next chunk's rows
  * before waiting on the current one; 4 consecutive rows in index order, block
