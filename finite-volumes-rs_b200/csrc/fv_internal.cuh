@@ -69,6 +69,7 @@ static inline cudaError_t fv_block_alloc(T **p, size_t bytes) {
 void fv_blocks_free(void *const *blocks, int n);
 void fv_block_free(void *p);
 unsigned long long fv_current_context_id();  // 0 when unknown
+unsigned long long fv_bound_context_id();    // the current device's context, made current first; 0 when unknown
 void fv_note_launch();
 void fv_note_launches(long long delta);  // graph replays add, captures (not run) subtract
 unsigned long long fv_launches_now();

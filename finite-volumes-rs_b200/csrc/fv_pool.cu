@@ -50,6 +50,13 @@ unsigned long long fv_current_context_id() {
     return id;
 }
 
+// The same, once the current device's context is current on this thread: a
+// thread that has made no call yet which needs one has none.
+unsigned long long fv_bound_context_id() {
+    const unsigned long long id = fv_current_context_id();
+    return id != 0 || cudaFree(nullptr) != cudaSuccess ? id : fv_current_context_id();
+}
+
 namespace {
 
 constexpr size_t kKeepBytes = 512u << 20, kKeepBlock = 64u << 20;

@@ -4,6 +4,9 @@
 // order, so a result depends only on n and the data), and the elementwise
 // updates +=, -=, *= (scalar), inv and set, which are exact.
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <vector>
 
 #include "fv_internal.cuh"
 
@@ -18,50 +21,50 @@ inline int vec_grid(int64_t n) {
 
 constexpr int kMaxBlocks = 148 * 4;
 
-// The workspace of one host thread's reductions: per device the block partials
-// and the ticket (0 between calls), and the result in pinned host memory, which
-// the kernel writes.  A reduction returns after its stream has finished, so a
-// thread's next one never meets it in use.
+// The workspace of a reduction: the block partials and the ticket (0 between
+// uses), and the result in pinned host memory, which the kernel writes.  Both
+// belong to the context they were made in (cudaDeviceReset frees them), so free
+// ones wait under its id: at most as many as reductions ran at once.  A reduction
+// returns its workspace after its stream has finished, so no two meet in one.
 struct Workspace {
-    struct OnDevice {
-        double *partial = nullptr;  // kMaxBlocks values, then the ticket
-        unsigned long long ctx = 0;
-    };
-    OnDevice at[64];
+    double *partial = nullptr;  // kMaxBlocks values, then the ticket
     double *result = nullptr;
-    ~Workspace() {
-        int dev = -1;
-        if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && at[dev].partial && at[dev].ctx != 0 &&
-            fv_current_context_id() == at[dev].ctx)
-            cudaFree(at[dev].partial);
-        if (result) cudaFreeHost(result);
-    }
 };
+std::mutex g_mu;
+std::map<unsigned long long, std::vector<Workspace>> g_free;
 
-// The thread's workspace on the current device, made on first use there (and
-// again after the device's context was replaced).
-fv_status workspace(cudaStream_t st, double *&partial, double *&result) {
-    thread_local Workspace w;
-    int dev = -1;
-    FV_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return FV_ERR_INVALID;
-    Workspace::OnDevice &d = w.at[dev];
-    const unsigned long long ctx = fv_current_context_id();
-    if (!d.partial || d.ctx != ctx) {
-        double *p = nullptr;
-        FV_CUDA_TRY(cudaMalloc(&p, sizeof(double) * (kMaxBlocks + 1)));
-        const cudaError_t e = cudaMemsetAsync(p, 0, sizeof(double) * (kMaxBlocks + 1), st);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            FV_CUDA_TRY(e);
+void destroy(Workspace &w) {
+    cudaFree(w.partial);
+    cudaFreeHost(w.result);
+}
+
+cudaError_t take_workspace(unsigned long long ctx, cudaStream_t st, Workspace &w) {
+    if (ctx != 0) {
+        std::lock_guard<std::mutex> g(g_mu);
+        auto it = g_free.find(ctx);
+        if (it != g_free.end() && !it->second.empty()) {
+            w = it->second.back();
+            it->second.pop_back();
+            return cudaSuccess;
         }
-        d.partial = p;
-        d.ctx = fv_current_context_id();
     }
-    if (!w.result) FV_CUDA_TRY(cudaHostAlloc((void **)&w.result, sizeof(double), cudaHostAllocPortable));
-    partial = d.partial;
-    result = w.result;
-    return FV_OK;
+    cudaError_t e = cudaMalloc(&w.partial, sizeof(double) * (kMaxBlocks + 1));
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&w.result, sizeof(double), cudaHostAllocPortable);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.partial, 0, sizeof(double) * (kMaxBlocks + 1), st);
+    if (e != cudaSuccess) destroy(w);
+    return e;
+}
+
+void return_workspace(unsigned long long ctx, Workspace &w) {
+    if (ctx != 0) {
+        try {
+            std::lock_guard<std::mutex> g(g_mu);
+            g_free[ctx].push_back(w);
+            return;
+        } catch (...) {  // host memory for the list: freed then
+        }
+    }
+    destroy(w);
 }
 
 __device__ __forceinline__ double block_sum(double v, double *sm) {
@@ -132,16 +135,22 @@ fv_status reduce(int64_t n, const double *x, const double *y, int mode, void *st
     }
     if (!x || (mode == 0 && !y)) return FV_ERR_INVALID;
     cudaStream_t st = fv_stream(stream);
-    double *partial = nullptr, *result = nullptr;
-    FV_TRY(workspace(st, partial, result));
+    const unsigned long long ctx = fv_bound_context_id();
+    Workspace w;
+    FV_CUDA_TRY(take_workspace(ctx, st, w));
     fv_note_launch();
     if (mode == 0)
-        k_vec_reduce<true><<<vec_grid(n), kVB, 0, st>>>(n, x, y, partial, result);
+        k_vec_reduce<true><<<vec_grid(n), kVB, 0, st>>>(n, x, y, w.partial, w.result);
     else
-        k_vec_reduce<false><<<vec_grid(n), kVB, 0, st>>>(n, x, y, partial, result);
-    FV_CUDA_TRY(cudaGetLastError());
-    FV_CUDA_TRY(cudaStreamSynchronize(st));
-    *out = *(volatile double *)result;
+        k_vec_reduce<false><<<vec_grid(n), kVB, 0, st>>>(n, x, y, w.partial, w.result);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        destroy(w);
+        FV_CUDA_TRY(e);
+    }
+    *out = *(volatile double *)w.result;
+    return_workspace(ctx, w);
     return FV_OK;
 }
 

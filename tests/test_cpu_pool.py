@@ -1,0 +1,93 @@
+"""Memory that outlives a call -- the blocks of matrices and preconditioners,
+the workspace of the reductions -- against a fake CUDA runtime (fake_cuda.cpp),
+where a context can be replaced, memory can run out and queued work can be seen."""
+import ctypes as C
+import subprocess
+import threading
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+CSRC = ROOT / "finite-volumes-rs_b200" / "csrc"
+MB = 1 << 20
+
+
+@pytest.fixture(scope="module")
+def lib_path(tmp_path_factory):
+    from fvb200.build import INCLUDE, _nvcc
+    d = tmp_path_factory.mktemp("fake")
+    objs = []
+    for src in (CSRC / "fv_pool.cu", CSRC / "fv_vector.cu"):
+        objs.append(str(d / (src.stem + ".o")))
+        subprocess.run([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1", "--extended-lambda",
+                        "-Xcompiler", "-fPIC", "-I", str(INCLUDE), "-I", str(CSRC), "-c", str(src), "-o", objs[-1]],
+                       check=True)
+    out = d / "libfake.so"
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic,--no-undefined", "-I",
+                    "/usr/local/cuda/include", str(ROOT / "tests" / "fake_cuda.cpp"), *objs, "-o", str(out)], check=True)
+    return out
+
+
+MALLOCS, FREES, SYNCS, BAD = range(4)
+
+
+@pytest.fixture
+def cu(lib_path, tmp_path):
+    """The library of its own: nothing kept from another test."""
+    own = tmp_path / "lib.so"
+    own.write_bytes(lib_path.read_bytes())
+    L = C.CDLL(str(own))
+    L.pool_alloc.restype = C.c_void_p
+    L.pool_alloc.argtypes = [C.c_size_t]
+    L.pool_free.argtypes = [C.c_void_p]
+    L.fake_use.argtypes = L.fake_busy.argtypes = [C.c_void_p]
+    L.fake_count.restype = C.c_longlong
+    L.fake_used.restype = L.fake_capacity.restype = C.c_size_t
+    L.fake_capacity.argtypes = [C.c_size_t]
+    L.fv_vec_sum.argtypes = [C.c_int64, C.c_void_p, C.c_void_p, C.POINTER(C.c_double)]
+    L.fake_reset()
+    return L
+
+
+def _sum(L, n):
+    out = C.c_double(-1.0)
+    assert L.fv_vec_sum(n, C.c_void_p(16), None, C.byref(out)) == 0
+    return out.value
+
+
+@pytest.mark.parametrize("device", [0, 1])
+def test_reductions_after_a_context_was_replaced(cu, device):
+    """The partials and the pinned result belong to their device's context."""
+    assert _sum(cu, 1000) == 1000.0
+    cu.fake_device(device)
+    assert _sum(cu, 1001) == 1001.0
+    cu.fake_device(0)
+    cu.fake_replace_context()
+    cu.fake_device(device)
+    assert _sum(cu, 1002) == 1002.0
+    cu.fake_device(0)
+    assert _sum(cu, 1003) == 1003.0
+    assert cu.fake_count(BAD) == 0
+
+
+@pytest.mark.parametrize("ids", [True, False])
+def test_reductions_on_short_lived_threads_take_no_more_memory(cu, ids):
+    cu.fake_no_context_ids(not ids)
+    for device in (0, 1):
+        cu.fake_device(device)
+        assert _sum(cu, 5) == 5.0
+    used = []
+    for k in range(4):
+        def work():
+            for device in (0, 1):
+                cu.fake_device(device)
+                assert _sum(cu, 7 + k) == 7.0 + k
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        used.append([])
+        for device in (0, 1):
+            cu.fake_device(device)
+            used[-1].append(cu.fake_used())
+    assert used[0] == used[3] and cu.fake_count(BAD) == 0
