@@ -88,7 +88,8 @@ void give_back(int dev) {
 cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
     *p = nullptr;
     int dev = -1;
-    const bool keep = bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    const unsigned long long ctx = fv_bound_context_id();  // 0 (unknown): nothing is taken or kept
+    const bool keep = ctx != 0 && bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
     if (!keep) {
         cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaErrorMemoryAllocation && dev >= 0 && dev < 64) {
@@ -100,7 +101,6 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
         return e;
     }
     try {
-        const unsigned long long ctx = fv_current_context_id();
         std::lock_guard<std::mutex> g(g_mu);
         Kept &k = g_kept[dev];
         if (k.ctx != ctx) {  // another context: its addresses mean nothing any more
@@ -108,15 +108,13 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
             k.bytes = 0;
             k.ctx = ctx;
         }
-        if (ctx != 0) {
-            auto it = k.by_size.lower_bound(bytes);
-            if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
-                g_live[it->second] = Block{it->first, dev, ctx};
-                *p = it->second;
-                k.bytes -= it->first;
-                k.by_size.erase(it);
-                return cudaSuccess;
-            }
+        auto it = k.by_size.lower_bound(bytes);
+        if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
+            g_live[it->second] = Block{it->first, dev, ctx};
+            *p = it->second;
+            k.bytes -= it->first;
+            k.by_size.erase(it);
+            return cudaSuccess;
         }
         cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaErrorMemoryAllocation) {
@@ -124,7 +122,7 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
             give_back(dev);
             e = cudaMalloc(p, bytes);
         }
-        if (e == cudaSuccess && ctx != 0) g_live[*p] = Block{bytes, dev, ctx};
+        if (e == cudaSuccess) g_live[*p] = Block{bytes, dev, ctx};
         return e;
     } catch (...) {  // host memory for the bookkeeping: plain memory then
         return *p ? cudaSuccess : cudaMalloc(p, bytes);

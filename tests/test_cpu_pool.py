@@ -91,3 +91,23 @@ def test_reductions_on_short_lived_threads_take_no_more_memory(cu, ids):
             cu.fake_device(device)
             used[-1].append(cu.fake_used())
     assert used[0] == used[3] and cu.fake_count(BAD) == 0
+
+
+def test_kept_blocks_serve_a_thread_without_a_context(cu):
+    """A host thread's first call: no context is current on it yet, the kept blocks are still the device's."""
+    cu.pool_free(cu.pool_alloc(8 * MB))
+    got = []
+    t = threading.Thread(target=lambda: got.append(cu.pool_alloc(8 * MB)))
+    t.start()
+    t.join()
+    assert cu.fake_used() == 8 * MB  # the kept block, not a second one
+    cu.pool_free(got[0])
+    assert cu.pool_alloc(8 * MB) == got[0] and cu.fake_used() == 8 * MB
+    assert cu.fake_count(BAD) == 0
+
+
+def test_nothing_is_kept_when_contexts_are_unknown(cu):
+    cu.fake_no_context_ids(1)
+    for _ in range(3):
+        cu.pool_free(cu.pool_alloc(MB))
+    assert cu.fake_used() == 0 and cu.fake_count(BAD) == 0
