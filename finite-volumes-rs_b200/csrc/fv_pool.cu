@@ -11,10 +11,11 @@
 // bytes, and that cudaFree waits for the device as every cudaFree of the blocks
 // did (measured: it returns when a kernel in flight on another, non-blocking
 // stream ends).  So a block from here may be used on any stream at once, like
-// memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per device, blocks
+// memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per context, blocks
 // of at most kKeepBlock) and given back when an allocation fails.  Blocks belong
-// to the device, and to its context: when the context has been replaced
-// (cudaDeviceReset), what was kept is forgotten.
+// to the context they were made in and are handed out, kept and freed in that one
+// only: when it has been replaced (cudaDeviceReset), its addresses mean nothing
+// any more, or something else.
 #include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
 
 #include <map>
@@ -63,24 +64,22 @@ constexpr size_t kKeepBytes = 512u << 20, kKeepBlock = 64u << 20;
 
 struct Block {
     size_t bytes;
-    int dev;
     unsigned long long ctx;
 };
 struct Kept {
     std::multimap<size_t, void *> by_size;
     size_t bytes = 0;
-    unsigned long long ctx = 0;
 };
 std::mutex g_mu;
-std::unordered_map<void *, Block> g_live;  // blocks handed out that may be kept when freed
-Kept g_kept[64];
+std::unordered_map<void *, Block> g_live;     // blocks handed out that may be kept when freed
+std::map<unsigned long long, Kept> g_kept;    // by context
 
-// Everything kept on the current device goes back to the driver.
-void give_back(int dev) {
-    Kept &k = g_kept[dev];
-    for (auto &b : k.by_size) cudaFree(b.second);
-    k.by_size.clear();
-    k.bytes = 0;
+// Everything kept in the current context goes back to the driver.
+void give_back(unsigned long long ctx) {
+    auto it = g_kept.find(ctx);
+    if (it == g_kept.end()) return;
+    for (auto &b : it->second.by_size) cudaFree(b.second);
+    g_kept.erase(it);
 }
 
 }  // namespace
@@ -89,28 +88,23 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
     *p = nullptr;
     int dev = -1;
     const unsigned long long ctx = fv_bound_context_id();  // 0 (unknown): nothing is taken or kept
-    const bool keep = ctx != 0 && bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    const bool keep = ctx != 0 && bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess;
     if (!keep) {
         cudaError_t e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation && dev >= 0 && dev < 64) {
+        if (e == cudaErrorMemoryAllocation && dev >= 0) {
             std::lock_guard<std::mutex> g(g_mu);
             cudaGetLastError();
-            give_back(dev);
+            give_back(ctx);
             e = cudaMalloc(p, bytes);
         }
         return e;
     }
     try {
         std::lock_guard<std::mutex> g(g_mu);
-        Kept &k = g_kept[dev];
-        if (k.ctx != ctx) {  // another context: its addresses mean nothing any more
-            k.by_size.clear();
-            k.bytes = 0;
-            k.ctx = ctx;
-        }
+        Kept &k = g_kept[ctx];
         auto it = k.by_size.lower_bound(bytes);
         if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
-            g_live[it->second] = Block{it->first, dev, ctx};
+            g_live[it->second] = Block{it->first, ctx};
             *p = it->second;
             k.bytes -= it->first;
             k.by_size.erase(it);
@@ -119,10 +113,10 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
         cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            give_back(dev);
+            give_back(ctx);
             e = cudaMalloc(p, bytes);
         }
-        if (e == cudaSuccess) g_live[*p] = Block{bytes, dev, ctx};
+        if (e == cudaSuccess) g_live[*p] = Block{bytes, ctx};
         return e;
     } catch (...) {  // host memory for the bookkeeping: plain memory then
         return *p ? cudaSuccess : cudaMalloc(p, bytes);
@@ -139,9 +133,9 @@ void fv_block_free(void *p) {
 }
 
 void fv_blocks_free(void *const *blocks, int n) {
-    int dev = -1;
+    const unsigned long long ctx = fv_bound_context_id();
     void *fence = nullptr;
-    const bool idle = cudaGetDevice(&dev) == cudaSuccess && cudaMalloc(&fence, 256) == cudaSuccess &&
+    const bool idle = ctx != 0 && cudaMalloc(&fence, 256) == cudaSuccess &&
                       cudaFree(fence) == cudaSuccess;  // waits for the device
     if (!idle) cudaGetLastError();
     for (int i = 0; i < n; ++i) {
@@ -151,12 +145,12 @@ void fv_blocks_free(void *const *blocks, int n) {
             try {
                 std::lock_guard<std::mutex> g(g_mu);
                 auto it = g_live.find(blocks[i]);
-                if (it != g_live.end() && it->second.dev == dev) {
-                    const Block b = it->second;
-                    Kept &k = g_kept[b.dev];
-                    if (k.ctx == b.ctx && k.bytes + b.bytes <= kKeepBytes) {
-                        k.by_size.emplace(b.bytes, blocks[i]);
-                        k.bytes += b.bytes;
+                if (it != g_live.end() && it->second.ctx == ctx) {
+                    const size_t bytes = it->second.bytes;
+                    Kept &k = g_kept[ctx];
+                    if (k.bytes + bytes <= kKeepBytes) {
+                        k.by_size.emplace(bytes, blocks[i]);
+                        k.bytes += bytes;
                         g_live.erase(it);
                         kept = true;
                     }

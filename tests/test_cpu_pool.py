@@ -111,3 +111,19 @@ def test_nothing_is_kept_when_contexts_are_unknown(cu):
     for _ in range(3):
         cu.pool_free(cu.pool_alloc(MB))
     assert cu.fake_used() == 0 and cu.fake_count(BAD) == 0
+
+
+def test_addresses_of_a_replaced_context(cu):
+    """What was live or kept in a context that is gone says nothing about the same
+    addresses in the next one."""
+    first = cu.pool_alloc(MB)
+    cu.pool_free(cu.pool_alloc(2 * MB))
+    cu.fake_replace_context()
+    large = cu.pool_alloc(100 * MB)
+    assert large == first
+    cu.pool_free(large)  # not a block of 1 MB to be kept
+    assert cu.fake_used() == 0
+    p = cu.pool_alloc(2 * MB)
+    assert cu.fake_used() == 2 * MB
+    cu.pool_free(p)
+    assert cu.fake_count(BAD) == 0
