@@ -74,49 +74,44 @@ std::mutex g_mu;
 std::unordered_map<void *, Block> g_live;     // blocks handed out that may be kept when freed
 std::map<unsigned long long, Kept> g_kept;    // by context
 
-// Everything kept in the current context goes back to the driver.
-void give_back(unsigned long long ctx) {
-    auto it = g_kept.find(ctx);
-    if (it == g_kept.end()) return;
+}  // namespace
+
+// Everything kept in the current context goes back to the driver; whether that was anything.
+bool fv_blocks_give_back() {
+    std::lock_guard<std::mutex> g(g_mu);
+    auto it = g_kept.find(fv_bound_context_id());
+    if (it == g_kept.end() || it->second.by_size.empty()) return false;
     for (auto &b : it->second.by_size) cudaFree(b.second);
     g_kept.erase(it);
+    return true;
 }
-
-}  // namespace
 
 cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
     *p = nullptr;
-    int dev = -1;
     const unsigned long long ctx = fv_bound_context_id();  // 0 (unknown): nothing is taken or kept
-    const bool keep = ctx != 0 && bytes <= kKeepBlock && cudaGetDevice(&dev) == cudaSuccess;
-    if (!keep) {
-        cudaError_t e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation && dev >= 0) {
-            std::lock_guard<std::mutex> g(g_mu);
-            cudaGetLastError();
-            give_back(ctx);
-            e = cudaMalloc(p, bytes);
-        }
-        return e;
-    }
+    const bool keep = ctx != 0 && bytes <= kKeepBlock;
     try {
-        std::lock_guard<std::mutex> g(g_mu);
-        Kept &k = g_kept[ctx];
-        auto it = k.by_size.lower_bound(bytes);
-        if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
-            g_live[it->second] = Block{it->first, ctx};
-            *p = it->second;
-            k.bytes -= it->first;
-            k.by_size.erase(it);
-            return cudaSuccess;
+        if (keep) {
+            std::lock_guard<std::mutex> g(g_mu);
+            Kept &k = g_kept[ctx];
+            auto it = k.by_size.lower_bound(bytes);
+            if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
+                g_live[it->second] = Block{it->first, ctx};
+                *p = it->second;
+                k.bytes -= it->first;
+                k.by_size.erase(it);
+                return cudaSuccess;
+            }
         }
         cudaError_t e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation) {
+        if (e == cudaErrorMemoryAllocation && fv_blocks_give_back()) {
             cudaGetLastError();
-            give_back(ctx);
             e = cudaMalloc(p, bytes);
         }
-        if (e == cudaSuccess) g_live[*p] = Block{bytes, ctx};
+        if (e == cudaSuccess && keep) {
+            std::lock_guard<std::mutex> g(g_mu);
+            g_live[*p] = Block{bytes, ctx};
+        }
         return e;
     } catch (...) {  // host memory for the bookkeeping: plain memory then
         return *p ? cudaSuccess : cudaMalloc(p, bytes);

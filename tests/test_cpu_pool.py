@@ -127,3 +127,15 @@ def test_addresses_of_a_replaced_context(cu):
     assert cu.fake_used() == 2 * MB
     cu.pool_free(p)
     assert cu.fake_count(BAD) == 0
+
+
+@pytest.mark.parametrize("mb", [30, 100])
+def test_kept_blocks_are_given_back_when_memory_runs_out(cu, mb):
+    cu.fake_capacity(120 * MB)
+    blocks = [cu.pool_alloc(10 * MB) for _ in range(10)]
+    for p in blocks:
+        cu.pool_free(p)
+    assert cu.fake_used() == 100 * MB
+    assert cu.pool_alloc(mb * MB)
+    assert cu.fake_used() == mb * MB and cu.fake_count(BAD) == 0
+    assert not cu.pool_alloc(121 * MB)
