@@ -814,23 +814,6 @@ cudaError_t fv_mesh_launch_grad_coeffs(fv_mesh *m, int *dbad, cudaStream_t st) {
 #include <mutex>
 static std::atomic<unsigned long long> g_launches{0};
 
-cudaError_t fv_malloc_async_raw(void **p, size_t bytes, cudaStream_t st) {
-    static std::atomic<bool> configured[64];
-    static std::mutex mu;
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev].load()) {
-        std::lock_guard<std::mutex> g(mu);
-        if (!configured[dev].load()) {
-            cudaMemPool_t pool;
-            if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-                uint64_t keep = UINT64_MAX;
-                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            }
-            configured[dev].store(true);
-        }
-    }
-    return cudaMallocAsync(p, bytes, st);
-}
 void fv_note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void fv_note_launches(long long delta) { g_launches.fetch_add((unsigned long long)delta, std::memory_order_relaxed); }
 unsigned long long fv_launches_now() { return g_launches.load(std::memory_order_relaxed); }
@@ -960,13 +943,13 @@ static fv_status mesh_upload_impl(const fv_mesh_desc *d, void *stream, fv_mesh *
     m->ncf = ncf;
     cudaStream_t st = fv_stream(stream);
     cudaError_t e = cudaSuccess;
-    e = cudaMalloc(&m->face_cells, sizeof(int2) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_area, sizeof(double) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->bface_center, sizeof(double4) * bfc.size());
-    if (e == cudaSuccess) e = cudaMalloc(&m->cell, sizeof(double4) * N);
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_face, sizeof(int32_t) * (ncf ? ncf : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_other, sizeof(int32_t) * (ncf ? ncf : 1));
+    e = fv_device_malloc(&m->face_cells, sizeof(int2) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_area, sizeof(double) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->bface_center, sizeof(double4) * bfc.size());
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cell, sizeof(double4) * N);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_face, sizeof(int32_t) * (ncf ? ncf : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_other, sizeof(int32_t) * (ncf ? ncf : 1));
     if (e == cudaSuccess) e = cudaMemcpyAsync(m->face_cells, fc.data(), sizeof(int2) * F, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m->face_area, d->face_area, sizeof(double) * F, cudaMemcpyHostToDevice, st);
@@ -979,7 +962,7 @@ static fv_status mesh_upload_impl(const fv_mesh_desc *d, void *stream, fv_mesh *
         e = cudaMemcpyAsync(m->cf_face, cff.data(), sizeof(int32_t) * ncf, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && ncf)
         e = cudaMemcpyAsync(m->cf_other, cfo.data(), sizeof(int32_t) * ncf, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && padf) e = cudaMalloc(&m->cf_pad, sizeof(int2) * N * padf);
+    if (e == cudaSuccess && padf) e = fv_device_malloc(&m->cf_pad, sizeof(int2) * N * padf);
     if (e == cudaSuccess && padf)
         e = cudaMemcpyAsync(m->cf_pad, pad.data(), sizeof(int2) * N * padf, cudaMemcpyHostToDevice, st);
     // normals, all face centres and the mesh-order cell faces: gradient
@@ -996,13 +979,13 @@ static fv_status mesh_upload_impl(const fv_mesh_desc *d, void *stream, fv_mesh *
             fc4[f] = make_double4(p[0], p[1], dim == 3 ? p[2] : 0.0, 0.0);
         }
         const int64_t ng = d->cell_face_ptr[N];
-        e = cudaMalloc(&m->face_normal, sizeof(double4) * F);
-        if (e == cudaSuccess) e = cudaMalloc(&m->face_center, sizeof(double4) * F);
-        if (e == cudaSuccess) e = cudaMalloc(&m->gcf_ptr, sizeof(int32_t) * (N + 1));
-        if (e == cudaSuccess) e = cudaMalloc(&m->gcf_face, sizeof(int32_t) * (ng ? ng : 1));
-        if (e == cudaSuccess) e = cudaMalloc(&m->gcoef, sizeof(double4) * (ng ? ng : 1));
-        if (e == cudaSuccess) e = cudaMalloc(&m->gdiag, sizeof(double4) * N);
-        if (e == cudaSuccess) e = cudaMalloc(&dbad, sizeof(int));
+        e = fv_device_malloc(&m->face_normal, sizeof(double4) * F);
+        if (e == cudaSuccess) e = fv_device_malloc(&m->face_center, sizeof(double4) * F);
+        if (e == cudaSuccess) e = fv_device_malloc(&m->gcf_ptr, sizeof(int32_t) * (N + 1));
+        if (e == cudaSuccess) e = fv_device_malloc(&m->gcf_face, sizeof(int32_t) * (ng ? ng : 1));
+        if (e == cudaSuccess) e = fv_device_malloc(&m->gcoef, sizeof(double4) * (ng ? ng : 1));
+        if (e == cudaSuccess) e = fv_device_malloc(&m->gdiag, sizeof(double4) * N);
+        if (e == cudaSuccess) e = fv_device_malloc(&dbad, sizeof(int));
         if (e == cudaSuccess) e = cudaMemsetAsync(dbad, 0, sizeof(int), st);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(m->face_normal, fn4.data(), sizeof(double4) * F, cudaMemcpyHostToDevice, st);
@@ -1060,7 +1043,7 @@ static fv_status build_pattern(fv_mesh *m, cudaStream_t st) {
     const int B = 256;
     const unsigned G = (unsigned)((N + B - 1) / B);
     int32_t *len = nullptr;
-    FV_CUDA_TRY(cudaMalloc(&m->row_ptr, sizeof(int32_t) * (N + 1)));
+    FV_CUDA_TRY(fv_device_malloc(&m->row_ptr, sizeof(int32_t) * (N + 1)));
     FV_CUDA_TRY(fv_malloc_async(&len, sizeof(int32_t) * (N + 1), st));
     FV_CUDA_TRY(cudaMemsetAsync(len + N, 0, sizeof(int32_t), st));
     const int mf = m->maxf;
@@ -1082,7 +1065,7 @@ static fv_status build_pattern(fv_mesh *m, cudaStream_t st) {
     cudaFreeAsync(tmp, st);
     cudaFreeAsync(len, st);
     m->nnz = nnz;
-    FV_CUDA_TRY(cudaMalloc(&m->cols, sizeof(int32_t) * (nnz ? nnz : 1)));
+    FV_CUDA_TRY(fv_device_malloc(&m->cols, sizeof(int32_t) * (nnz ? nnz : 1)));
     if (mf <= 4)
         fv_note_launch(), k_row_fill<4><<<G, B, 0, st>>>(N, m->cf_ptr, m->cf_other, m->row_ptr, m->cols);
     else if (mf <= 8)
@@ -1103,8 +1086,8 @@ static fv_status ensure_orth_geometry(fv_mesh *m, cudaStream_t st) {
     if (m->face_geo && m->cell_vol) return FV_OK;
     double2 *geo = nullptr;
     double *vol = nullptr;
-    cudaError_t e = cudaMalloc(&geo, sizeof(double2) * (m->n_faces ? m->n_faces : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&vol, sizeof(double) * (m->n_cells ? m->n_cells : 1));
+    cudaError_t e = fv_device_malloc(&geo, sizeof(double2) * (m->n_faces ? m->n_faces : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&vol, sizeof(double) * (m->n_cells ? m->n_cells : 1));
     if (e == cudaSuccess && m->n_faces) {
         const unsigned G = (unsigned)std::min<int64_t>((m->n_faces + 255) / 256, 148 * 16);
         if (m->dim == 2)

@@ -777,7 +777,7 @@ static fv_status batch_create_impl(const fv_csr *A, int32_t n_problems, const in
     cudaError_t e = cudaSuccess;
     auto up = [&](int32_t **d, const std::vector<int32_t> &h) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(d, sizeof(int32_t) * h.size());
+        e = fv_device_malloc(d, sizeof(int32_t) * h.size());
         if (e == cudaSuccess) e = cudaMemcpyAsync(*d, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice, st);
     };
     up(&B->tile_prob, tp);
@@ -785,9 +785,9 @@ static fv_status batch_create_impl(const fv_csr *A, int32_t n_problems, const in
     up(&B->tile_row1, r1);
     up(&B->ptile, pt);
     up(&B->row_prob, rp);
-    if (e == cudaSuccess) e = cudaMalloc(&B->S, sizeof(BProb) * n_problems);
-    if (e == cudaSuccess) e = cudaMalloc(&B->G, sizeof(BGlobal));
-    if (e == cudaSuccess) e = cudaMalloc(&B->partial, sizeof(double) * B->ntiles * kMaxTileSums);
+    if (e == cudaSuccess) e = fv_device_malloc(&B->S, sizeof(BProb) * n_problems);
+    if (e == cudaSuccess) e = fv_device_malloc(&B->G, sizeof(BGlobal));
+    if (e == cudaSuccess) e = fv_device_malloc(&B->partial, sizeof(double) * B->ntiles * kMaxTileSums);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         fv_internal_set_cuda_error(e, "fv_batch_create");
@@ -963,7 +963,7 @@ fv_status ensure_bytes(void *&p, size_t &have, size_t need) {
     cudaFree(p);
     p = nullptr;
     have = 0;
-    FV_CUDA_TRY(cudaMalloc(&p, need));
+    FV_CUDA_TRY(fv_device_malloc(&p, need));
     have = need;
     return FV_OK;
 }
@@ -1034,8 +1034,8 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
         cudaFree(B->resume);
         B->seg = nullptr;
         B->resume = nullptr;
-        FV_CUDA_TRY(cudaMalloc(&B->seg, sizeof(int64_t) * seg.size()));
-        FV_CUDA_TRY(cudaMalloc(&B->resume, sizeof(int32_t) * list.size()));
+        FV_CUDA_TRY(fv_device_malloc(&B->seg, sizeof(int64_t) * seg.size()));
+        FV_CUDA_TRY(fv_device_malloc(&B->resume, sizeof(int32_t) * list.size()));
         FV_CUDA_TRY(cudaMemcpyAsync(B->seg, seg.data(), sizeof(int64_t) * seg.size(), cudaMemcpyHostToDevice, st));
         FV_CUDA_TRY(
             cudaMemcpyAsync(B->resume, list.data(), sizeof(int32_t) * list.size(), cudaMemcpyHostToDevice, st));
@@ -1057,7 +1057,7 @@ fv_status run_begin(fv_batch *B, fv_precond *P, bool bicg, const double *b, doub
         }
         FV_TRY(inner_start<double>(bicg, B, P, v, G, tl, st));
     } else {
-        if (!B->a32) FV_CUDA_TRY(cudaMalloc(&B->a32, sizeof(float) * (B->A->nnz ? B->A->nnz : 1)));
+        if (!B->a32) FV_CUDA_TRY(fv_device_malloc(&B->a32, sizeof(float) * (B->A->nnz ? B->A->nnz : 1)));
         fv_note_launch(), k_to_f32b<<<148 * 8, 256, 0, st>>>(B->A->nnz, B->A->vals, B->a32);
         FV_TRY(fv_precond_make_f32(P, st));
         FV_TRY(fv_precond_batch_prepare(P, np, B->off.data(), B->row_prob, true, st));

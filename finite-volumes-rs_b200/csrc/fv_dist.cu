@@ -299,7 +299,7 @@ extern "C" fv_status fv_csr_square_block(const fv_csr *A, void *stream, fv_csr *
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
     fv_status rc = FV_OK;
-    cudaError_t e = cudaMalloc(&s->row_ptr, sizeof(int32_t) * (n + 1));
+    cudaError_t e = fv_device_malloc(&s->row_ptr, sizeof(int32_t) * (n + 1));
     if (e == cudaSuccess) e = fv_malloc_async(&cnt, sizeof(int32_t) * (n + 1), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (n + 1), st);
     if (e == cudaSuccess && n > 0) {
@@ -314,8 +314,8 @@ extern "C" fv_status fv_csr_square_block(const fv_csr *A, void *stream, fv_csr *
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) {
         s->nnz = nnz;
-        e = cudaMalloc(&s->cols, sizeof(int32_t) * (nnz ? nnz : 1));
-        if (e == cudaSuccess) e = cudaMalloc(&s->vals, sizeof(double) * (nnz ? nnz : 1));
+        e = fv_device_malloc(&s->cols, sizeof(int32_t) * (nnz ? nnz : 1));
+        if (e == cudaSuccess) e = fv_device_malloc(&s->vals, sizeof(double) * (nnz ? nnz : 1));
     }
     if (e == cudaSuccess && n > 0) {
         fv_note_launch(), kd_square_fill<<<vec_grid(n), DB, 0, st>>>(n, A->row_ptr, A->cols, A->vals, s->row_ptr,
@@ -349,10 +349,10 @@ extern "C" fv_status fv_dist_create(const fv_csr *A, int64_t n_ghost, const int3
     D->n_send = n_send;
     if (comm) D->comm = *comm;
     const int G = dot_grid(D->n_own);
-    cudaError_t e = cudaMalloc(&D->send_idx, sizeof(int32_t) * (n_send ? n_send : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&D->send, sizeof(double) * (n_send ? n_send : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&D->part, sizeof(double) * kMaxDots * G);
-    if (e == cudaSuccess) e = cudaMalloc(&D->sums, sizeof(double) * kMaxDots);
+    cudaError_t e = fv_device_malloc(&D->send_idx, sizeof(int32_t) * (n_send ? n_send : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&D->send, sizeof(double) * (n_send ? n_send : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&D->part, sizeof(double) * kMaxDots * G);
+    if (e == cudaSuccess) e = fv_device_malloc(&D->sums, sizeof(double) * kMaxDots);
     if (e == cudaSuccess) e = cudaMallocHost(&D->host, sizeof(double) * kMaxDots);
     if (e == cudaSuccess && n_send)
         e = cudaMemcpy(D->send_idx, send_idx, sizeof(int32_t) * n_send, cudaMemcpyHostToDevice);

@@ -57,6 +57,13 @@ template <typename T>
 static inline cudaError_t fv_malloc_async(T **p, size_t bytes, cudaStream_t st) {
     return fv_malloc_async_raw(reinterpret_cast<void **>(p), bytes, st);
 }
+// cudaMalloc for what lives long or is made once; like fv_malloc_async it takes
+// memory kept for matrices and preconditioners back before it fails.
+cudaError_t fv_device_malloc_raw(void **p, size_t bytes);
+template <typename T>
+static inline cudaError_t fv_device_malloc(T **p, size_t bytes) {
+    return fv_device_malloc_raw(reinterpret_cast<void **>(p), bytes);
+}
 // Device memory of matrices and preconditioners (fv_pool.cu).  fv_block_alloc:
 // like cudaMalloc.  fv_blocks_free: the blocks of one object at once, null
 // entries allowed; fv_block_free: one block.  Both also take memory from

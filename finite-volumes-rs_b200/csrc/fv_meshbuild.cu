@@ -697,7 +697,7 @@ fv_status finish(Scratch &sc, fv_mesh *m, int64_t L, int *d_flags, int64_t n_nod
     int32_t *cnt = sc.get<int32_t>((size_t)N + 1);
     int *d_maxf = d_flags + 1;
     if (e == cudaSuccess) e = sc.err;
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt + N, 0, sizeof(int32_t), st);
     if (e == cudaSuccess) {
         fv_note_launch();
@@ -720,9 +720,9 @@ fv_status finish(Scratch &sc, fv_mesh *m, int64_t L, int *d_flags, int64_t n_nod
     m->maxf = maxf;
     m->ncf = ncf;
     m->padf = maxf <= 4 ? 4 : (maxf <= 8 ? 8 : 0);
-    e = cudaMalloc(&m->cf_face, sizeof(int32_t) * (ncf ? ncf : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_other, sizeof(int32_t) * (ncf ? ncf : 1));
-    if (e == cudaSuccess && m->padf) e = cudaMalloc(&m->cf_pad, sizeof(int2) * N * m->padf);
+    e = fv_device_malloc(&m->cf_face, sizeof(int32_t) * (ncf ? ncf : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_other, sizeof(int32_t) * (ncf ? ncf : 1));
+    if (e == cudaSuccess && m->padf) e = fv_device_malloc(&m->cf_pad, sizeof(int2) * N * m->padf);
     if (e == cudaSuccess) {
         fv_note_launch();
         k_cf_fill<<<blocks(N), kB, 0, st>>>(N, m->gcf_ptr, m->gcf_face, m->face_cells, m->cf_ptr, m->cf_face,
@@ -732,8 +732,8 @@ fv_status finish(Scratch &sc, fv_mesh *m, int64_t L, int *d_flags, int64_t n_nod
 
     // gradient coefficients (compute.rs:155-203) over the mesh-order cell faces
     int *d_gbad = d_flags + 2;
-    if (e == cudaSuccess) e = cudaMalloc(&m->gcoef, sizeof(double4) * (L ? L : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->gdiag, sizeof(double4) * N);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->gcoef, sizeof(double4) * (L ? L : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->gdiag, sizeof(double4) * N);
     if (e == cudaSuccess) e = fv_mesh_launch_grad_coeffs(m, d_gbad, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_flags, d_flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -795,7 +795,7 @@ extern "C" fv_status fv_mesh_build_elements(int32_t dim, int64_t n_nodes, const 
     unsigned long long *d_counts = sc.get<unsigned long long>(2);
     int32_t *nf = sc.get<int32_t>((size_t)n_elems + 1);
     if (e == cudaSuccess) e = sc.err;
-    if (e == cudaSuccess) e = cudaMalloc(&efp, sizeof(int32_t) * (n_elems + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&efp, sizeof(int32_t) * (n_elems + 1));
     fv_mesh *m = new fv_mesh();
     m->gcf_ptr = efp;
     auto give_up = [&](fv_status s) {
@@ -897,13 +897,13 @@ extern "C" fv_status fv_mesh_build_elements(int32_t dim, int64_t n_nodes, const 
     int32_t *face_src = sc.get<int32_t>((size_t)F), *face_len = sc.get<int32_t>((size_t)F + 1);
     int32_t *fnp = sc.get<int32_t>((size_t)F + 1), *fnodes = sc.get<int32_t>((size_t)F * W);
     if (sc.err != cudaSuccess) return give_up(fail(sc.err, "fv_mesh_build_elements (faces)"));
-    e = cudaMalloc(&m->face_cells, sizeof(int2) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_area, sizeof(double) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_normal, sizeof(double4) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_center, sizeof(double4) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->cell, sizeof(double4) * n_elems);
-    if (e == cudaSuccess) e = cudaMalloc(&m->gcf_face, sizeof(int32_t) * L);
-    if (e == cudaSuccess) e = cudaMalloc(&m->bface_center, sizeof(double4) * (F - n_int > 0 ? F - n_int : 1));
+    e = fv_device_malloc(&m->face_cells, sizeof(int2) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_area, sizeof(double) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_normal, sizeof(double4) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_center, sizeof(double4) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cell, sizeof(double4) * n_elems);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->gcf_face, sizeof(int32_t) * L);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->bface_center, sizeof(double4) * (F - n_int > 0 ? F - n_int : 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(face_len + F, 0, sizeof(int32_t), st);
     if (e == cudaSuccess) {
         fv_note_launch();
@@ -991,14 +991,14 @@ extern "C" fv_status fv_mesh_build_faces(int32_t dim, int64_t n_nodes, const dou
     m->n_cells = N;
     m->n_faces = F;
     m->n_bfaces = n_tagged;
-    if (e == cudaSuccess) e = cudaMalloc(&m->gcf_ptr, sizeof(int32_t) * (N + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->gcf_face, sizeof(int32_t) * (L ? L : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_cells, sizeof(int2) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_area, sizeof(double) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_normal, sizeof(double4) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_center, sizeof(double4) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->cell, sizeof(double4) * N);
-    if (e == cudaSuccess) e = cudaMalloc(&m->bface_center, sizeof(double4) * (n_tagged ? n_tagged : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->gcf_ptr, sizeof(int32_t) * (N + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->gcf_face, sizeof(int32_t) * (L ? L : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_cells, sizeof(int2) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_area, sizeof(double) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_normal, sizeof(double4) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_center, sizeof(double4) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cell, sizeof(double4) * N);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->bface_center, sizeof(double4) * (n_tagged ? n_tagged : 1));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m->gcf_ptr, cell_face_ptr, sizeof(int32_t) * (N + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && L)
@@ -1165,14 +1165,14 @@ static fv_status mesh_concat_impl(const fv_mesh *const *parts, int32_t n_parts, 
     m->maxf = maxf;
     m->padf = maxf <= 4 ? 4 : (maxf <= 8 ? 8 : 0);
     m->ncf = NCF;
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_cells, sizeof(int2) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->face_area, sizeof(double) * F);
-    if (e == cudaSuccess) e = cudaMalloc(&m->bface_center, sizeof(double4) * (TB ? TB : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cell, sizeof(double4) * N);
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_face, sizeof(int32_t) * (NCF ? NCF : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&m->cf_other, sizeof(int32_t) * (NCF ? NCF : 1));
-    if (e == cudaSuccess && m->padf) e = cudaMalloc(&m->cf_pad, sizeof(int2) * N * m->padf);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_cells, sizeof(int2) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->face_area, sizeof(double) * F);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->bface_center, sizeof(double4) * (TB ? TB : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cell, sizeof(double4) * N);
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_ptr, sizeof(int32_t) * (N + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_face, sizeof(int32_t) * (NCF ? NCF : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&m->cf_other, sizeof(int32_t) * (NCF ? NCF : 1));
+    if (e == cudaSuccess && m->padf) e = fv_device_malloc(&m->cf_pad, sizeof(int2) * N * m->padf);
     if (e == cudaSuccess) {
         CatPtrs q;
         q.face_cells = reinterpret_cast<const int2 *const *>(d_ptrs + 0 * P);

@@ -12,12 +12,13 @@
 // did (measured: it returns when a kernel in flight on another, non-blocking
 // stream ends).  So a block from here may be used on any stream at once, like
 // memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per context, blocks
-// of at most kKeepBlock) and given back when an allocation fails.  Blocks belong
-// to the context they were made in and are handed out, kept and freed in that one
+// of at most kKeepBlock) and given back when an allocation of this library fails.
+// Blocks belong to the context they were made in and are handed out, kept and freed in that one
 // only: when it has been replaced (cudaDeviceReset), its addresses mean nothing
 // any more, or something else.
 #include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -77,13 +78,46 @@ std::map<unsigned long long, Kept> g_kept;    // by context
 }  // namespace
 
 // Everything kept in the current context goes back to the driver; whether that was anything.
-bool fv_blocks_give_back() {
+static bool give_back() {
     std::lock_guard<std::mutex> g(g_mu);
     auto it = g_kept.find(fv_bound_context_id());
     if (it == g_kept.end() || it->second.by_size.empty()) return false;
     for (auto &b : it->second.by_size) cudaFree(b.second);
     g_kept.erase(it);
     return true;
+}
+
+// An allocation, made again after kept memory was given back when there is none left.
+template <class F>
+static cudaError_t with_kept_memory(F alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && give_back()) {
+        cudaGetLastError();
+        e = alloc();
+    }
+    return e;
+}
+
+cudaError_t fv_device_malloc_raw(void **p, size_t bytes) {
+    return with_kept_memory([&] { return cudaMalloc(p, bytes); });
+}
+
+cudaError_t fv_malloc_async_raw(void **p, size_t bytes, cudaStream_t st) {
+    static std::atomic<bool> configured[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev].load()) {
+        std::lock_guard<std::mutex> g(mu);
+        if (!configured[dev].load()) {
+            cudaMemPool_t pool;
+            if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+                uint64_t keep = UINT64_MAX;
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            }
+            configured[dev].store(true);
+        }
+    }
+    return with_kept_memory([&] { return cudaMallocAsync(p, bytes, st); });
 }
 
 cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
@@ -103,11 +137,7 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
                 return cudaSuccess;
             }
         }
-        cudaError_t e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation && fv_blocks_give_back()) {
-            cudaGetLastError();
-            e = cudaMalloc(p, bytes);
-        }
+        const cudaError_t e = fv_device_malloc_raw(p, bytes);
         if (e == cudaSuccess && keep) {
             std::lock_guard<std::mutex> g(g_mu);
             g_live[*p] = Block{bytes, ctx};

@@ -49,9 +49,9 @@ extern "C" fv_status fv_csr_create_host(int64_t nrows, int64_t ncols, const int3
     a->nrows = nrows;
     a->ncols = ncols;
     a->nnz = nnz;
-    cudaError_t e = cudaMalloc(&a->row_ptr, sizeof(int32_t) * (nrows + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&a->cols, sizeof(int32_t) * (nnz ? nnz : 1));
-    if (e == cudaSuccess) e = cudaMalloc(&a->vals, sizeof(double) * (nnz ? nnz : 1));
+    cudaError_t e = fv_device_malloc(&a->row_ptr, sizeof(int32_t) * (nrows + 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&a->cols, sizeof(int32_t) * (nnz ? nnz : 1));
+    if (e == cudaSuccess) e = fv_device_malloc(&a->vals, sizeof(double) * (nnz ? nnz : 1));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(a->row_ptr, row_ptr, sizeof(int32_t) * (nrows + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(a->cols, cols, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, st);

@@ -48,7 +48,7 @@ cudaError_t take_workspace(unsigned long long ctx, cudaStream_t st, Workspace &w
             return cudaSuccess;
         }
     }
-    cudaError_t e = cudaMalloc(&w.partial, sizeof(double) * (kMaxBlocks + 1));
+    cudaError_t e = fv_device_malloc(&w.partial, sizeof(double) * (kMaxBlocks + 1));
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&w.result, sizeof(double), cudaHostAllocPortable);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.partial, 0, sizeof(double) * (kMaxBlocks + 1), st);
     if (e != cudaSuccess) destroy(w);

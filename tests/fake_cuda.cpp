@@ -73,7 +73,10 @@ CUresult get_id(CUcontext c, unsigned long long *id) {
 // What the tested files take from the rest of the library, and what the test calls in them.
 void fv_note_launch() {}
 void fv_internal_set_cuda_error(cudaError_t, const char *) {}
+void fv_internal_set_error_text(const char *) {}
 cudaError_t fv_block_alloc_raw(void **p, size_t bytes);
+cudaError_t fv_device_malloc_raw(void **p, size_t bytes);
+cudaError_t fv_malloc_async_raw(void **p, size_t bytes, cudaStream_t st);
 void fv_blocks_free(void *const *blocks, int n);
 
 extern "C" {
@@ -82,6 +85,14 @@ extern "C" {
 void *pool_alloc(size_t bytes) {
     void *p = nullptr;
     return fv_block_alloc_raw(&p, bytes) == cudaSuccess ? p : nullptr;
+}
+void *device_alloc(size_t bytes) {
+    void *p = nullptr;
+    return fv_device_malloc_raw(&p, bytes) == cudaSuccess ? p : nullptr;
+}
+void *stream_alloc(size_t bytes) {
+    void *p = nullptr;
+    return fv_malloc_async_raw(&p, bytes, nullptr) == cudaSuccess ? p : nullptr;
 }
 void pool_free(void *p) { fv_blocks_free(&p, 1); }
 void fake_reset() {
@@ -164,6 +175,11 @@ cudaError_t cudaFree(void *p) {
     g.device.erase(it);
     return cudaSuccess;
 }
+cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t *p, int) {
+    *p = nullptr;
+    return cudaSuccess;
+}
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
 cudaError_t cudaMallocAsync(void **p, size_t bytes, cudaStream_t) { return cudaMalloc(p, bytes); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned) {

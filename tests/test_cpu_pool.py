@@ -139,3 +139,17 @@ def test_kept_blocks_are_given_back_when_memory_runs_out(cu, mb):
     assert cu.pool_alloc(mb * MB)
     assert cu.fake_used() == mb * MB and cu.fake_count(BAD) == 0
     assert not cu.pool_alloc(121 * MB)
+
+
+@pytest.mark.parametrize("allocator", ["device_alloc", "stream_alloc"])
+def test_the_other_allocations_get_kept_blocks_back_too(cu, allocator):
+    """Meshes, batches and distributed systems (device_alloc), the solvers' and the
+    factorisation's workspaces (stream_alloc)."""
+    cu.fake_capacity(120 * MB)
+    for p in [cu.pool_alloc(10 * MB) for _ in range(10)]:
+        cu.pool_free(p)
+    f = getattr(cu, allocator)
+    f.restype, f.argtypes = C.c_void_p, [C.c_size_t]
+    assert f(90 * MB)
+    assert cu.fake_used() == 90 * MB and cu.fake_count(BAD) == 0
+    assert not f(31 * MB)
