@@ -12,8 +12,8 @@
 // did (measured: it returns when a kernel in flight on another, non-blocking
 // stream ends).  So a block from here may be used on any stream at once, like
 // memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per context, blocks
-// of at most kKeepBlock) and given back when an allocation of this library fails.
-// Blocks belong to the context they were made in and are handed out, kept and freed in that one
+// of at most kKeepBlock) and given back when an allocation of this library fails
+// or fv_release_kept_memory is called.  Blocks belong to the context they were made in and are handed out, kept and freed in that one
 // only: when it has been replaced (cudaDeviceReset), its addresses mean nothing
 // any more, or something else.
 #include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
@@ -85,6 +85,13 @@ static bool give_back() {
     for (auto &b : it->second.by_size) cudaFree(b.second);
     g_kept.erase(it);
     return true;
+}
+
+extern "C" fv_status fv_release_kept_memory(void) {
+    return fv_host_guard([] {
+        give_back();
+        return FV_OK;
+    });
 }
 
 // An allocation, made again after kept memory was given back when there is none left.

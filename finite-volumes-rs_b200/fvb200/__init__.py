@@ -6,7 +6,7 @@ linalg::{DistributedMatrix, DistributedVector}, preconditioners::{
 IncompleteCholesky, IncompleteLowerUpper, DiagonalPreconditioner}, solvers::{conjugate_gradient,
 bi_conjugate_gradient_stab, LinearSolverOptions, LinearSolverInfo}).
 """
-from ._lib import FvError, lib  # noqa: F401
+from ._lib import FvError, lib, release_kept_memory  # noqa: F401
 from .linalg import (  # noqa: F401
     DiagonalPreconditioner, DistributedMatrix, DistributedVector, IdentityPreconditioner, IncompleteCholesky,
     IncompleteLowerUpper,

@@ -191,6 +191,7 @@ _SIGS = {
     "fv_dist_spmv": [vp, vp, vp, vp],
     "fv_dist_dot": [vp, vp, vp, dp, vp],
     "fv_dist_cg": [vp, vp, vp, vp, SolverOptions, P(SolverInfo), vp],
+    "fv_release_kept_memory": [],
     "fv_dist_bicgstab": [vp, vp, vp, vp, SolverOptions, P(SolverInfo), vp],
 }
 
@@ -240,6 +241,11 @@ def lib() -> C.CDLL:
 def check(status: int, what: str) -> None:
     if status != FV_OK:
         raise FvError(status, what)
+
+
+def release_kept_memory() -> None:
+    """Device memory kept for the next matrix or preconditioner goes back to the driver."""
+    check(lib().fv_release_kept_memory(), "release_kept_memory")
 
 
 def exported_symbols() -> list[str]:

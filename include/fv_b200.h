@@ -667,6 +667,10 @@ fv_status fv_dist_bicgstab(fv_dist *D, fv_precond *P, const double *b, double *x
 const char *fv_status_string(fv_status s);
 /* Text of the last CUDA error recorded by this thread (after FV_ERR_CUDA). */
 const char *fv_last_error(void);
+/* Gives the device memory kept for the next matrix or preconditioner (at most
+ * 512 MB) back to the driver, for a program whose own allocations run short; the
+ * library's own do so by themselves.  Waits for the device. */
+fv_status fv_release_kept_memory(void);
 /* Number of kernels this library has launched in this process (diagnostics). */
 uint64_t fv_launch_count(void);
 

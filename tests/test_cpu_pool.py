@@ -153,3 +153,8 @@ def test_the_other_allocations_get_kept_blocks_back_too(cu, allocator):
     assert f(90 * MB)
     assert cu.fake_used() == 90 * MB and cu.fake_count(BAD) == 0
     assert not f(31 * MB)
+
+def test_release_kept_memory(cu):
+    cu.pool_free(cu.pool_alloc(10 * MB))
+    assert cu.fv_release_kept_memory() == 0
+    assert cu.fake_used() == 0 and cu.fake_count(BAD) == 0
