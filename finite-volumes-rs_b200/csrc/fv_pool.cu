@@ -11,11 +11,14 @@
 // bytes, and that cudaFree waits for the device as every cudaFree of the blocks
 // did (measured: it returns when a kernel in flight on another, non-blocking
 // stream ends).  So a block from here may be used on any stream at once, like
-// memory from cudaMalloc.  Kept memory is bounded (kKeepBytes per context, blocks
-// of at most kKeepBlock) and given back when an allocation of this library fails
-// or fv_release_kept_memory is called.  Blocks belong to the context they were made in and are handed out, kept and freed in that one
-// only: when it has been replaced (cudaDeviceReset), its addresses mean nothing
-// any more, or something else.
+// memory from cudaMalloc.
+//
+// Kept memory is bounded (kKeepBytes per context, blocks of at most kKeepBlock;
+// the oldest make room for the next) and given back when an allocation of this
+// library fails or fv_release_kept_memory is called.  Blocks belong to the
+// context they were made in and are handed out, kept and freed in that one only:
+// when it has been replaced (cudaDeviceReset), its addresses mean nothing any
+// more, or something else.
 #include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
 
 #include <atomic>
@@ -68,8 +71,31 @@ struct Block {
     unsigned long long ctx;
 };
 struct Kept {
-    std::multimap<size_t, void *> by_size;
+    struct Entry {
+        void *p;
+        unsigned long long age;
+    };
+    using BySize = std::multimap<size_t, Entry>;
+    BySize by_size;
+    std::map<unsigned long long, BySize::iterator> by_age;  // the oldest first
+    unsigned long long next_age = 0;
     size_t bytes = 0;
+
+    void put(size_t size, void *p) {
+        const auto it = by_size.emplace(size, Entry{p, next_age});
+        try {
+            by_age.emplace(next_age++, it);
+        } catch (...) {
+            by_size.erase(it);
+            throw;
+        }
+        bytes += size;
+    }
+    void take(BySize::iterator it) {
+        bytes -= it->first;
+        by_age.erase(it->second.age);
+        by_size.erase(it);
+    }
 };
 std::mutex g_mu;
 std::unordered_map<void *, Block> g_live;     // blocks handed out that may be kept when freed
@@ -82,7 +108,7 @@ static bool give_back() {
     std::lock_guard<std::mutex> g(g_mu);
     auto it = g_kept.find(fv_bound_context_id());
     if (it == g_kept.end() || it->second.by_size.empty()) return false;
-    for (auto &b : it->second.by_size) cudaFree(b.second);
+    for (auto &b : it->second.by_size) cudaFree(b.second.p);
     g_kept.erase(it);
     return true;
 }
@@ -137,10 +163,10 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes) {
             Kept &k = g_kept[ctx];
             auto it = k.by_size.lower_bound(bytes);
             if (it != k.by_size.end() && it->first <= bytes + bytes / 4 + 4096) {
-                g_live[it->second] = Block{it->first, ctx};
-                *p = it->second;
-                k.bytes -= it->first;
-                k.by_size.erase(it);
+                void *const block = it->second.p;
+                g_live[block] = Block{it->first, ctx};
+                k.take(it);
+                *p = block;
                 return cudaSuccess;
             }
         }
@@ -180,12 +206,14 @@ void fv_blocks_free(void *const *blocks, int n) {
                 if (it != g_live.end() && it->second.ctx == ctx) {
                     const size_t bytes = it->second.bytes;
                     Kept &k = g_kept[ctx];
-                    if (k.bytes + bytes <= kKeepBytes) {
-                        k.by_size.emplace(bytes, blocks[i]);
-                        k.bytes += bytes;
-                        g_live.erase(it);
-                        kept = true;
+                    while (k.bytes + bytes > kKeepBytes) {  // the oldest make room
+                        const auto oldest = k.by_age.begin()->second;
+                        cudaFree(oldest->second.p);
+                        k.take(oldest);
                     }
+                    k.put(bytes, blocks[i]);
+                    g_live.erase(it);
+                    kept = true;
                 }
             } catch (...) {  // host memory for the bookkeeping: freed then
             }

@@ -158,3 +158,21 @@ def test_release_kept_memory(cu):
     cu.pool_free(cu.pool_alloc(10 * MB))
     assert cu.fv_release_kept_memory() == 0
     assert cu.fake_used() == 0 and cu.fake_count(BAD) == 0
+
+
+def test_the_oldest_kept_blocks_make_room(cu):
+    """A large system that is gone leaves full shelves; what is in use now is kept all the same."""
+    for p in [cu.pool_alloc(60 * MB) for _ in range(8)]:
+        cu.pool_free(p)
+    small = [cu.pool_alloc(10 * MB) for _ in range(4)]
+    for p in small:
+        cu.pool_free(p)
+    before = cu.fake_count(MALLOCS)
+    for _ in range(3):
+        again = [cu.pool_alloc(10 * MB) for _ in range(4)]
+        assert sorted(again) == sorted(small)
+        for p in again:
+            cu.pool_free(p)
+    fences = 3 * 4  # fv_blocks_free may allocate to wait for the device
+    assert cu.fake_count(MALLOCS) - before <= fences
+    assert cu.fake_used() <= 512 * MB and cu.fake_count(BAD) == 0
