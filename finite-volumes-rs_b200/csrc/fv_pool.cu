@@ -8,10 +8,14 @@
 //
 // A block is handed out again only after the device has finished all work
 // submitted before it was freed: fv_blocks_free first allocates and frees 256
-// bytes, and that cudaFree waits for the device as every cudaFree of the blocks
-// did (measured: it returns when a kernel in flight on another, non-blocking
-// stream ends).  So a block from here may be used on any stream at once, like
-// memory from cudaMalloc.
+// bytes, and cudaFree synchronises across all streams of the device (the CUDA
+// programming guide says so of cudaMalloc and cudaFree where it introduces the
+// stream-ordered allocator; measured: it returns when a kernel in flight on
+// another, non-blocking stream ends).  So a block from here may be used on any
+// stream at once, like memory from cudaMalloc.  cudaDeviceSynchronize would wait
+// as well, but a stream capture on any other host thread is invalidated by it, in
+// every capture mode; dropping an object leaves thread-local and relaxed captures
+// alone, as cudaFree of its blocks does.
 //
 // Kept memory is bounded (kKeepBytes per context, blocks of at most kKeepBlock;
 // the oldest make room for the next) and given back when an allocation of this
@@ -21,6 +25,7 @@
 // more, or something else.
 #include <cuda.h>  // CUcontext / CUresult types only; the driver calls are reached through the runtime
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -191,6 +196,7 @@ void fv_block_free(void *p) {
 }
 
 void fv_blocks_free(void *const *blocks, int n) {
+    if (std::all_of(blocks, blocks + n, [](void *p) { return !p; })) return;
     const unsigned long long ctx = fv_bound_context_id();
     void *fence = nullptr;
     const bool idle = ctx != 0 && cudaMalloc(&fence, 256) == cudaSuccess &&

@@ -26,7 +26,7 @@ struct State {
     size_t capacity = ~size_t(0) >> 1;
     unsigned long long next_ctx = 1;
     char *next = reinterpret_cast<char *>(0x700000000000);
-    long long mallocs = 0, frees = 0, syncs = 0, bad = 0;
+    long long mallocs = 0, frees = 0, bad = 0;
     bool no_ids = false;
 } g;
 std::recursive_mutex g_mu;
@@ -128,7 +128,7 @@ int fake_busy(void *p) {
     return it != g.device.end() && it->second.busy;
 }
 long long fake_count(int what) {
-    return what == 0 ? g.mallocs : what == 1 ? g.frees : what == 2 ? g.syncs : g.bad;
+    return what == 0 ? g.mallocs : what == 1 ? g.frees : g.bad;
 }
 size_t fake_used() { return g.used[t_dev]; }
 
@@ -160,7 +160,7 @@ cudaError_t cudaMalloc(void **p, size_t bytes) {
     g.used[t_dev] += bytes;
     return cudaSuccess;
 }
-// As the runtime's does, it waits until nothing uses *p any more (that memory only).
+// As the runtime's does, it waits for the device.
 cudaError_t cudaFree(void *p) {
     Lock l(g_mu);
     bind();
@@ -171,6 +171,8 @@ cudaError_t cudaFree(void *p) {
         ++g.bad;
         return ret(cudaErrorInvalidValue);
     }
+    for (auto &d : g.device)
+        if (d.second.dev == it->second.dev) d.second.busy = false;
     g.used[it->second.dev] -= it->second.bytes;
     g.device.erase(it);
     return cudaSuccess;
@@ -204,14 +206,6 @@ cudaError_t cudaMemsetAsync(void *p, int, size_t, cudaStream_t) {
         ++g.bad;
         return ret(cudaErrorInvalidValue);
     }
-    return cudaSuccess;
-}
-cudaError_t cudaDeviceSynchronize() {
-    Lock l(g_mu);
-    bind();
-    ++g.syncs;
-    for (auto &d : g.device)
-        if (d.second.dev == t_dev) d.second.busy = false;
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }

@@ -29,7 +29,7 @@ def lib_path(tmp_path_factory):
     return out
 
 
-MALLOCS, FREES, SYNCS, BAD = range(4)
+MALLOCS, FREES, BAD = range(3)
 
 
 @pytest.fixture
@@ -176,3 +176,13 @@ def test_the_oldest_kept_blocks_make_room(cu):
     fences = 3 * 4  # fv_blocks_free may allocate to wait for the device
     assert cu.fake_count(MALLOCS) - before <= fences
     assert cu.fake_used() <= 512 * MB and cu.fake_count(BAD) == 0
+
+
+def test_a_block_is_handed_out_again_only_when_its_work_is_done(cu):
+    p = cu.pool_alloc(MB)
+    cu.fake_use(p)
+    cu.pool_free(p)
+    assert cu.pool_alloc(MB) == p and not cu.fake_busy(p)
+    before = cu.fake_count(MALLOCS), cu.fake_count(FREES)
+    cu.pool_free(None)  # an object without blocks waits for nothing
+    assert (cu.fake_count(MALLOCS), cu.fake_count(FREES)) == before and cu.fake_count(BAD) == 0
