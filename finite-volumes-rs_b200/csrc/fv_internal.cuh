@@ -218,7 +218,9 @@ __device__ __forceinline__ unsigned long long fv_globaltimer() {
 #define FV_SENTINEL_U64 0xFFFFFFFFFFFFFFFFULL
 #define FV_SENTINEL_U32 0xFFFFFFFFu
 // Bounded waits give up after this many nanoseconds of wall time.
+#ifndef FV_WAIT_LIMIT_NS  // a test sets a short one
 #define FV_WAIT_LIMIT_NS 2000000000ULL
+#endif
 
 __device__ __forceinline__ unsigned long long fv_pack_value(double v) {
     unsigned long long b = (unsigned long long)__double_as_longlong(v);

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_apply(const __grid_
                                                                    int *err) {
     if (skip && *(volatile const int *)skip) return;  // the same answer in every CTA of the cluster
     extern __shared__ __align__(128) unsigned char res_smem[];
-    __shared__ unsigned long long bars[kResBuffers];
+    __shared__ unsigned long long bars[kResBars];
     fv_res_cta<T, ML, S> cta(a, res_smem, bars);
     fv_cluster_arrive();  // no push before every CTA's halo is reset
     cta.load(r);

@@ -59,6 +59,7 @@ constexpr size_t kResSmem = 226 * 1024;  // dynamic shared memory of a CTA (1 KB
 // of the instruction cache.)
 constexpr int kResBuffers = 4;
 constexpr int kResGroupBytes = 16 * 1024;
+constexpr int kResBars = kResBuffers + 1;  // an mbarrier per buffer, then the word that says a copy was given up
 
 // The plan of an apply: one cluster for a system, or several clusters, each with
 // some of the independent problems of a batch.  Every CTA has one list of steps, the levels of its
@@ -157,8 +158,11 @@ __device__ __forceinline__ void fv_sts(unsigned a, float v) {
 // step to the next lie only the operands' loads, the row's arithmetic and one
 // store: with all threads at one barrier per step the unpacking (about 400
 // cycles) set the pace.  buf: kResBuffers
-// groups of records; bars: kResBuffers mbarriers, initialised with count 1;
-// groups: copies made through them before, kept across calls.  halo0: first
+// groups of records; bars: kResBars words, the mbarriers initialised with count 1;
+// groups: copies made through them before, kept across calls.  A copy that does
+// not land in time, or while an error is raised, ends the work: only the steps'
+// barriers go on, bars[kResBuffers] is set, and the copies in flight are waited
+// for (bounded) before the return.  No further call may then use the mbarriers.  halo0: first
 // halo slot (the slots before it are the constant 0 and the idle lanes' slot).
 template <typename T, int ML, int S>
 __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec, int nsteps, int width, int group,
@@ -195,6 +199,23 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
         else
             asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(after_own), "r"(two) : "memory");
     };
+    // whether the copy of group g lands within the limit (t0: when the wait began); heed: an error ends it too
+    auto landed = [&](int g, unsigned long long &t0, bool heed) {
+        const unsigned b = (g0 + g) % kResBuffers, parity = ((g0 + g) / kResBuffers) & 1u;
+        unsigned done = 0;
+        for (unsigned it = 0; !done; ++it) {
+            asm volatile(
+                "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(mbase + 8 * b), "r"(parity)
+                : "memory");
+            if (!done && (it & 63u) == 63u) {
+                if (!t0) t0 = fv_globaltimer();
+                if ((heed && *(volatile int *)err) || fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS) return false;
+            }
+        }
+        return true;
+    };
     union Stage {
         uint4 q[PL];
         R r;
@@ -205,42 +226,28 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
     // the set's next step: steps left of its group, that group's successor, its record's address
     int left = 0, g = 0, todo = nsteps / S;
     unsigned src = 0;
+    bool gone = false;  // (the same in a warp) a copy was given up
     auto fetch = [&]() {
         if (todo == 0) return;
         --todo;
-        bool late = false;
         if (left == 0) {  // the set's first step of group g: its copy has landed
             // the step computed last lies in group g - 1: every record of group g - 2 has been read
             if (threadIdx.x == 0 && g > 1) copy(g - 2 + kResBuffers);
-            const unsigned b = (g0 + g) % kResBuffers, parity = ((g0 + g) / kResBuffers) & 1u;
-            unsigned done = 0;
             unsigned long long t0 = 0;
-            for (unsigned it = 0; !done && !late; ++it) {
-                asm volatile(
-                    "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                    : "=r"(done)
-                    : "r"(mbase + 8 * b), "r"(parity)
-                    : "memory");
-                if (!done && (it & 63u) == 63u) {
-                    if (!t0) t0 = fv_globaltimer();
-                    late = fv_globaltimer() - t0 > FV_WAIT_LIMIT_NS;
-                }
-            }
-            if (late) atomicOr(err, FV_DEV_TIMEOUT);
+            gone = __any_sync(0xffffffffu, !landed(g, t0, true));
             left = group / S;
-            src = bbase + (b * group + set) * step_bytes;
+            src = bbase + ((g0 + g) % kResBuffers * group + set) * step_bytes;
             ++g;
+            if (gone) {
+                if (!*(volatile int *)err) atomicOr(err, FV_DEV_TIMEOUT);
+                *(volatile unsigned long long *)&bars[kResBuffers] = 1;
+                return;
+            }
         }
         --left;
 #pragma unroll
         for (int p = 0; p < PL; ++p) u.q[p] = fv_lds16(src + (unsigned)(p * width) * 16u);
         src += S * step_bytes;
-        if (late) {  // an idle slot: the steps and their barriers go on
-#pragma unroll
-            for (int q = 0; q < ML; ++q) u.r.dep[q] = (uint16_t)(halo0 - 2);
-            u.r.self = (uint16_t)(halo0 - 1);
-            u.r.meta = u.r.push0 = 0;
-        }
         a_self = xbase + u.r.self * (unsigned)sizeof(T);
 #pragma unroll
         for (int q = 0; q < ML; ++q) a_dep[q] = xbase + u.r.dep[q] * (unsigned)sizeof(T);
@@ -254,7 +261,8 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
     if (threadIdx.x == 0)
         for (int g = 0; g < kResBuffers; ++g) copy(g);
     fetch();
-    for (int st = set; st < nsteps; st += S) {
+    int st = set;
+    for (; st < nsteps && !gone; st += S) {
         if (S > 1 && st > 0) wait_prev();
         T x, xv[ML];
 #pragma unroll
@@ -287,7 +295,16 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
         fetch();
         if (S == 1) end_own();
     }
+    for (; st < nsteps; st += S) {  // the barriers go on
+        if (S > 1 && st > 0) wait_prev();
+        end_own();
+    }
     if (S > 1 && set == 0 && nsteps > 0) wait_prev();  // the last step's arrivals are met
+    if (gone && threadIdx.x == 0) {  // it gave up group g - 1; the last copy it made is that of group g + 1
+        unsigned long long t0 = 0;
+        const int made = min(ng, max(kResBuffers, g - 2 + kResBuffers));
+        for (int q = g - 1; q < made && landed(q, t0, false);) ++q;
+    }
     groups = g0 + ng;
 }
 
@@ -319,8 +336,8 @@ struct fv_res_cta {
     int nr, ns;
     unsigned groups = 0;
 
-    // smem: fv_resident_smem bytes; bars: kResBuffers mbarriers.  A cluster
-    // barrier has to follow before the first sweeps.
+    // smem: fv_resident_smem bytes; mbar: kResBars words.  A cluster barrier has
+    // to follow before the first sweeps.
     __device__ __forceinline__ fv_res_cta(const fv_res_args &args, unsigned char *smem, unsigned long long *mbar)
         : a(args), buf(reinterpret_cast<uint4 *>(smem)), bars(mbar) {
         xs = reinterpret_cast<T *>(buf + kResBuffers * a.group * a.width * PL);
@@ -335,6 +352,7 @@ struct fv_res_cta {
             for (int b = 0; b < kResBuffers; ++b)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&bars[b])));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            bars[kResBuffers] = 0;
         }
         if (threadIdx.x < 2) xs[a.cap + threadIdx.x] = T(0);
         reset_halo();
@@ -364,13 +382,18 @@ struct fv_res_cta {
             }
         }
     }
-    // Between load and store: the block is synchronised before and after.
+    // Between load and store: the block is synchronised before and after.  Once a
+    // copy has been given up (err is raised then) the rows become NaN.
     __device__ __forceinline__ void sweeps(int *err) {
+        const bool ended = gave_up();  // read before the barrier, written after it
         __syncthreads();
-        if ((int)threadIdx.x < S * a.width)
+        if (!ended && (int)threadIdx.x < S * a.width)
             fv_resident_sweeps<T, ML, S>(rec, ns, a.width, a.group, xs, a.cap + 2, buf, bars, groups, a.push, err);
         __syncthreads();
+        if (gave_up())
+            for (int k = threadIdx.x; k < nr; k += kResThreads) xs[k] = T(NAN);
     }
+    __device__ __forceinline__ bool gave_up() const { return *(volatile unsigned long long *)&bars[kResBuffers] != 0; }
 };
 
 template <typename F>

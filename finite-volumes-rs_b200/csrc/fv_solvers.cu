@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_cg(const __grid_con
     SolverState *S = q.S;
     if (S->done) return;
     extern __shared__ __align__(128) unsigned char rs_smem[];
-    __shared__ unsigned long long bars[kResBuffers];
+    __shared__ unsigned long long bars[kResBars];
     RsShared *sh = reinterpret_cast<RsShared *>(rs_smem);
     fv_res_cta<double, ML, SETS> cta(a, rs_smem + kRsBytes, bars);
     rs_open(sh, S);
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_bicgstab(const __gr
     SolverState *S = q.S;
     if (S->done) return;
     extern __shared__ __align__(128) unsigned char rs_smem[];
-    __shared__ unsigned long long bars[kResBuffers];
+    __shared__ unsigned long long bars[kResBars];
     RsShared *sh = reinterpret_cast<RsShared *>(rs_smem);
     fv_res_cta<double, ML, SETS> cta(a, rs_smem + kRsBytes, bars);
     rs_open(sh, S);
