@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_apply(const __grid_
 
 // Bytes of a record, steps per copy.
 size_t res_rec_bytes(int ml, size_t tb) {
-    return fv_res_dispatch(ml, 1, [&](auto M, auto) {
+    return fv_res_dispatch(ml, 2, [&](auto M, auto) {
         return tb == 8 ? sizeof(fv_res_rec<double, M()>) : sizeof(fv_res_rec<float, M()>);
     });
 }
@@ -698,7 +698,7 @@ fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_reside
 template <typename T>
 cudaError_t fv_resident_records(const fv_resident *p, const fv_resident_src &s, bool unit_fwd, const T *l_val,
                                 const T *u_val, const T *dinv, void *rec, cudaStream_t st) {
-    fv_res_dispatch(p->ml, 1, [&](auto M, auto) {
+    fv_res_dispatch(p->ml, 2, [&](auto M, auto) {
         fv_note_launch(), k_res_records<T, M()><<<(unsigned)((p->nslots + 255) / 256), 256, 0, st>>>(
                               *p, s.n, unit_fwd, s.l_ptr, s.u_ptr, l_val, u_val, dinv, (uint4 *)rec);
         return 0;

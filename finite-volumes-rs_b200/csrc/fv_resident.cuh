@@ -170,7 +170,8 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
                                                    unsigned &groups, const uint32_t *__restrict__ push, int *err) {
     using R = fv_res_rec<T, ML>;
     constexpr int PL = (int)(sizeof(R) / 16);
-    const int set = S == 1 ? 0 : (int)threadIdx.x / width, lane = (int)threadIdx.x - set * width;
+    static_assert(S > 1, "a set waits for the one before it");
+    const int set = (int)threadIdx.x / width, lane = (int)threadIdx.x - set * width;
     const int ng = (nsteps + group - 1) / group;
     const unsigned xbase = (unsigned)__cvta_generic_to_shared(xs);
     const unsigned bbase = (unsigned)__cvta_generic_to_shared(buf) + (unsigned)lane * 16u;
@@ -194,10 +195,7 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
     };
     auto end_own = [&]() {
         __syncwarp();
-        if (S == 1)
-            asm volatile("barrier.cta.sync.aligned 1, %0;" ::"r"(width) : "memory");
-        else
-            asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(after_own), "r"(two) : "memory");
+        asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(after_own), "r"(two) : "memory");
     };
     // whether the copy of group g lands within the limit (t0: when the wait began); heed: an error ends it too
     auto landed = [&](int g, unsigned long long &t0, bool heed) {
@@ -263,7 +261,7 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
     fetch();
     int st = set;
     for (; st < nsteps && !gone; st += S) {
-        if (S > 1 && st > 0) wait_prev();
+        if (st > 0) wait_prev();
         T x, xv[ML];
 #pragma unroll
         for (int q = 0; q < ML; ++q) fv_lds(a_dep[q], xv[q]);
@@ -291,15 +289,14 @@ __device__ __forceinline__ void fv_resident_sweeps(const uint4 *__restrict__ rec
                 }
             }
         }
-        if (S > 1) end_own();
+        end_own();
         fetch();
-        if (S == 1) end_own();
     }
     for (; st < nsteps; st += S) {  // the barriers go on
-        if (S > 1 && st > 0) wait_prev();
+        if (st > 0) wait_prev();
         end_own();
     }
-    if (S > 1 && set == 0 && nsteps > 0) wait_prev();  // the last step's arrivals are met
+    if (set == 0 && nsteps > 0) wait_prev();  // the last step's arrivals are met
     if (gone && threadIdx.x == 0) {  // it gave up group g - 1; the last copy it made is that of group g + 1
         unsigned long long t0 = 0;
         const int made = min(ng, max(kResBuffers, g - 2 + kResBuffers));
@@ -401,8 +398,7 @@ auto fv_res_dispatch(int ml, int sets, F &&f) {
     auto by_sets = [&](auto M) {
         if (sets == 8) return f(M, std::integral_constant<int, 8>());
         if (sets == 4) return f(M, std::integral_constant<int, 4>());
-        if (sets == 2) return f(M, std::integral_constant<int, 2>());
-        return f(M, std::integral_constant<int, 1>());
+        return f(M, std::integral_constant<int, 2>());
     };
     if (ml == 2) return by_sets(std::integral_constant<int, 2>());
     if (ml == 3) return by_sets(std::integral_constant<int, 3>());
