@@ -2118,6 +2118,16 @@ extern "C" fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t
     return FV_OK;
 }
 
+extern "C" fv_status fv_precond_default_sweeps(fv_precond *P, int32_t restore, int32_t *resident) {
+    if (!P) return FV_ERR_INVALID;
+    if (restore && P->kind != 3) {
+        P->schedule = P->contiguous && !P->perm && !P->fill ? 4 : 1;
+        P->explicit_schedule = false;
+    }
+    if (resident) *resident = P->kind != 3 && use_resident(P) ? 1 : 0;
+    return FV_OK;
+}
+
 extern "C" fv_status fv_precond_destroy(fv_precond *P) {
     if (!P) return FV_OK;
     void *blocks[32] = {P->l_val, P->u_val, P->diag, P->dinv, P->tmp, P->done, P->ctrl, P->err, P->l32, P->u32,

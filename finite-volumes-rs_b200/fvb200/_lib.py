@@ -158,6 +158,7 @@ _SIGS = {
     "fv_precond_levels": [vp, ip, ip, ip, ip, vp],
     "fv_precond_destroy": [vp],
     "fv_precond_schedule": [vp, C.c_int32, P(C.c_int32), dp],
+    "fv_precond_default_sweeps": [vp, C.c_int32, P(C.c_int32)],
     "fv_tile_plan_host": [i64, C.c_int32, dp, ip, ip, C.c_int32, P(i64), ip, ip, ip, ip, dp],
     "fv_fill_pattern_host": [C.c_int32, C.c_int32, i64, ip, ip, P(i64), ip, ip, ip, P(C.c_uint8)],
     "fv_cg": [vp, vp, vp, vp, SolverOptions, P(SolverInfo), vp],

@@ -231,13 +231,18 @@ def autotune_tile(A, row_offsets, P, b, x, candidates=(256, 512, 1024, 2048), it
 
 
 def autotune_schedule(P, b, x, candidates=(1, 3), reps=3, stream=None):
-    """Pick the faster sweep schedule for this preconditioner (level chunks, or
-    level chunks with the next chunk prefetched: the same bits either way) by
-    timing a few applies of each; returns (chosen, {schedule: ms per apply})."""
+    """Pick the fastest sweeps for this preconditioner by timing a few applies
+    of each: the schedules named (level chunks, level chunks with the next
+    chunk prefetched) and, where the library's own choice is another form, that
+    one ("default"); the same bits any way.  Returns (chosen, {candidate: ms
+    per apply})."""
     import torch
     times = {}
-    for sch in candidates:
-        P.schedule(sch)
+    P.default_schedule()
+    own = P.resident() or P.schedule()[0] not in candidates
+    for sch in (("default",) if own else ()) + tuple(candidates):
+        if sch != "default":
+            P.schedule(sch)
         P.precondition(x, b, stream=stream)
         ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
         torch.cuda.synchronize()
@@ -248,5 +253,8 @@ def autotune_schedule(P, b, x, candidates=(1, 3), reps=3, stream=None):
         torch.cuda.synchronize()
         times[sch] = ev[0].elapsed_time(ev[1]) / reps
     best = min(times, key=times.get)
-    P.schedule(best)
+    if best == "default":
+        P.default_schedule()
+    else:
+        P.schedule(best)
     return best, times

@@ -398,6 +398,16 @@ class Preconditioner:
                                         st.ctypes.data_as(C.POINTER(C.c_double))), "schedule")
         return act.value, st
 
+    def resident(self) -> bool:
+        """Whether the applies sweep in one cluster's shared memory."""
+        r = C.c_int32()
+        check(lib().fv_precond_default_sweeps(self.handle, 0, C.byref(r)), "resident")
+        return bool(r.value)
+
+    def default_schedule(self) -> None:
+        """Forget a requested schedule: the library chooses the sweeps again."""
+        check(lib().fv_precond_default_sweeps(self.handle, 1, None), "default_schedule")
+
     def set_grid(self, blocks: int, rows_per_thread: int = 0):
         """Sweep launch shape (fv_precond_set_grid): blocks per launch and rows
         per thread of the reordered sweeps, 0 = defaults; same results for any shape."""
