@@ -170,6 +170,10 @@ class Clocks:
 
 def sweep_schedule(P):
     """Which sweep schedule the preconditioner uses, with its box-tile plan."""
+    if P.resident(batch=True):
+        return {"kind": "resident: each problem's sweeps in one cluster's shared memory (k_resident_apply)"}
+    if P.resident():
+        return {"kind": "resident: sweeps in one cluster's shared memory (k_resident_apply)"}
     if P.perm is not None:
         return {"kind": "reordered factorisation: contiguous levels, block tickets (k_sweep_seq)"}
     act, st = P.schedule()

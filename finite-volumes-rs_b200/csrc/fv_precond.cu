@@ -2124,7 +2124,10 @@ extern "C" fv_status fv_precond_default_sweeps(fv_precond *P, int32_t restore, i
         P->schedule = P->contiguous && !P->perm && !P->fill ? 4 : 1;
         P->explicit_schedule = false;
     }
-    if (resident) *resident = P->kind != 3 && use_resident(P) ? 1 : 0;
+    if (resident) {
+        const bool own = P->kind != 3 && default_sweeps(P);
+        *resident = (own && P->res ? 1 : 0) | (own && (P->batch_rec || P->batch_rec32) ? 2 : 0);
+    }
     return FV_OK;
 }
 

@@ -398,11 +398,12 @@ class Preconditioner:
                                         st.ctypes.data_as(C.POINTER(C.c_double))), "schedule")
         return act.value, st
 
-    def resident(self) -> bool:
-        """Whether the applies sweep in one cluster's shared memory."""
+    def resident(self, batch: bool = False) -> bool:
+        """Whether the applies sweep in one cluster's shared memory; batch: whether
+        those of the last batch run swept each problem in a cluster."""
         r = C.c_int32()
         check(lib().fv_precond_default_sweeps(self.handle, 0, C.byref(r)), "resident")
-        return bool(r.value)
+        return bool(r.value & (2 if batch else 1))
 
     def default_schedule(self) -> None:
         """Forget a requested schedule: the library chooses the sweeps again."""

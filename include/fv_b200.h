@@ -370,8 +370,9 @@ fv_status fv_precond_levels(const fv_precond *P, int32_t *fwd_level, int32_t *bw
 fv_status fv_precond_schedule(fv_precond *P, int32_t request, int32_t *active, double *stats);
 /* The library's own choice of sweeps.  restore != 0: a schedule requested before
  * is forgotten.  *resident (optional) receives 1 when the applies sweep in one
- * cluster's shared memory, 0 when by the schedule that fv_precond_schedule
- * reports.  The same bits either way. */
+ * cluster's shared memory, plus 2 when the runs of a batch sweep each problem in
+ * a cluster; without them, the schedule that fv_precond_schedule reports runs.
+ * The same bits any way. */
 fv_status fv_precond_default_sweeps(fv_precond *P, int32_t restore, int32_t *resident);
 /* Sweep launch shape: blocks of 256 threads per sweep launch (1..4736; 0 =
  * the default: 2 per SM for natural-order sweeps, up to 8 per SM for the

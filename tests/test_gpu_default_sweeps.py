@@ -1,5 +1,6 @@
 """The library's own choice of sweeps: queried, given up for an explicit schedule,
 taken up again, and among the tuner's candidates."""
+import numpy as np
 import pytest
 
 from cases import diffusion_2d, equation
@@ -34,3 +35,22 @@ def test_the_default_sweeps_can_be_asked_for_again(fv):
     P = fv.IncompleteCholesky.from_matrix(A, 0)
     best, times = autotune_schedule(P, b, fv.DistributedVector.from_size(A.nrows()))
     assert not P.resident() and best in (1, 3) and set(times) == {1, 3} and P.schedule()[0] == best
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_batch_says_when_each_problem_has_its_cluster(fv, precision):
+    from fvb200.batch import BatchCG, MeshBatch
+    meshes = [fv.Mesh.square(s, 0.2, 70 + s) for s in (9, 14)]
+    f = [m.fields(70, 1.0, 0.5, source_const=1.0) for m in meshes]
+    mb = MeshBatch(meshes)
+    zero = np.zeros(mb.n_boundary_faces)
+    eq = -fv.laplacian(fv.Orthogonal(), mb.face_field([q[0] for q in f])) - fv.source(mb.cell_field([q[2] for q in f]))
+    A, b = fv.assemble(eq, (zero, zero), mb)
+    x = fv.DistributedVector.from_size(mb.n_cells)
+    for ordering, clusters in (("boxes", True), (None, False)):
+        P = fv.IncompleteCholesky.from_matrix(A, 0, ordering=ordering, offsets=mb.cell_offsets if ordering else None)
+        assert not P.resident(batch=True)
+        BatchCG(A, mb.cell_offsets, 256).solve(P, b, x, precision=precision)
+        assert P.resident(batch=True) == clusters
+        P.schedule(1)
+        assert not P.resident(batch=True) and not P.resident()
