@@ -495,15 +495,24 @@ void fv_resident_free(fv_resident *p) {
 
 size_t fv_resident_record_bytes(const fv_resident *p, size_t tb) { return (size_t)p->nslots * res_rec_bytes(p->ml, tb); }
 
-// How to go on when the shared memory of eight thread sets' buffers and the rows
-// does not fit: the rows over twice the CTAs (65,522-row IC(0), 362 levels: 131 ->
-// 114 us per apply), else four sets.
-enum class ResTry { kFirst, kMoreCtas, kFewerSets };
+// How to go on when the shared memory of the buffers and the rows does not fit:
+// the rows over twice the CTAs (65,522-row IC(0), 362 levels: 131 -> 114 us per
+// apply), then half the thread sets and with them half the buffers (105,456-row
+// ILU(0): 204 us per apply with level chunks, 122 this way).
+struct ResTry {
+    bool more_ctas = false;
+    int half_sets = 0;
+    // found by the last try: shared memory was all that it lacked; its CTAs, the bytes of their rows and halos
+    bool full = false;
+    int C = 0;
+    size_t rows = 0;
+};
 
 static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
-                           const fv_resident_problems *problems, ResTry attempt, bool &full) {
+                           const fv_resident_problems *problems, ResTry &t) {
     *out = nullptr;
-    full = false;
+    const bool again = t.full;
+    t.full = false;
     const int64_t n = s.n;
     if (n <= 0 || n > (problems ? 148 : kResMaxCta) * 20000LL || s.max_side > 6 || !s.fwd_level || !s.bwd_level)
         return FV_OK;
@@ -523,7 +532,7 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     int C = 1, width = 32;
     const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
     while (C < kResMaxCta && (n > (int64_t)C * 18000 || lw > (int64_t)C * (s.sorted ? 32 : 128))) C *= 2;
-    if (attempt == ResTry::kMoreCtas && C < kResMaxCta) C *= 2;
+    if (t.more_ctas && !problems) C = std::min(2 * C, kResMaxCta);
     while (width < (s.sorted ? 256 : 128) && lw * (s.sorted ? 2 : 1) > (int64_t)C * width) width *= 2;
     std::vector<int32_t> cluster;  // of every problem
     int clusters = 1;
@@ -535,7 +544,8 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     // pace of a 100-cycle step; eight of up to 64 threads hide it.  Four -> eight,
     // us per apply in natural order: 8,192-row IC(0), 128 levels, 62 -> 51;
     // 131,072 rows, 512 levels, 158 -> 149.
-    const int sets = width > 64 ? 512 / width : attempt == ResTry::kFewerSets ? 4 : 8;
+    const int sets = (width > 64 ? 512 / width : 8) >> t.half_sets;
+    if (sets < 2) return FV_OK;
     fv_resident *p = new (std::nothrow) fv_resident();
     if (!p) return FV_ERR_ALLOC;
     p->C = C;
@@ -544,6 +554,16 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     p->sorted = s.sorted;
     p->sets = sets;
     p->ml = ml;
+    p->cap = (int32_t)((n + ctas - 1) / ctas);  // at least
+    const size_t buffers = fv_resident_smem(p, sizeof(double)) - (size_t)(p->cap + 2) * sizeof(double);
+    const size_t rows = again && t.C == C ? t.rows : (size_t)(p->cap + 2) * sizeof(double);
+    if (buffers + rows > kResSmem) {
+        t.full = true;
+        t.C = C;
+        t.rows = rows;
+        delete p;
+        return FV_OK;
+    }
     ResPattern a;
     a.n = n;
     a.ptr[0] = s.l_ptr, a.ptr[1] = s.u_ptr;
@@ -660,10 +680,13 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
         p->halo = std::max(p->halo, h_hc[c]);
     }
     p->nslots = (int64_t)h_sptr[ctas] * width;
-    const bool fits = !h_hc[ctas] && p->cap + p->halo + 2 < 65536 && res_launchable<double>(p) > 0 &&
+    const bool small = fv_resident_smem(p, sizeof(double)) <= kResSmem;
+    const bool fits = !h_hc[ctas] && p->cap + p->halo + 2 < 65536 && small && res_launchable<double>(p) > 0 &&
                       res_launchable<float>(p) > 0;
     if (!fits) {
-        full = sets == 8;
+        t.full = !h_hc[ctas] && !small;
+        t.C = C;
+        t.rows = (size_t)(p->cap + 2 + p->halo) * sizeof(double);
         cudaFreeAsync(tmp, st);
         fv_resident_free(p);
         return FV_OK;
@@ -689,10 +712,17 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
 
 fv_status fv_resident_build(const fv_resident_src &s, cudaStream_t st, fv_resident **out,
                             const fv_resident_problems *problems) {
-    bool full;
-    FV_TRY(res_build(s, st, out, problems, ResTry::kFirst, full));
-    if (full && !problems) FV_TRY(res_build(s, st, out, problems, ResTry::kMoreCtas, full));
-    return full ? res_build(s, st, out, problems, ResTry::kFewerSets, full) : FV_OK;
+    ResTry t;
+    FV_TRY(res_build(s, st, out, problems, t));
+    if (t.full && !problems) {
+        t.more_ctas = true;
+        FV_TRY(res_build(s, st, out, problems, t));
+    }
+    while (t.full) {  // ends with less than two sets
+        ++t.half_sets;
+        FV_TRY(res_build(s, st, out, problems, t));
+    }
+    return FV_OK;
 }
 
 template <typename T>
