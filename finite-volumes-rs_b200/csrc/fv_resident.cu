@@ -33,6 +33,8 @@ __global__ void k_res_level_start(int64_t n, int32_t nlev, const int32_t *__rest
 // ranges -- with the box-colour order the rows of a box follow each other along
 // their dependencies, so a box stays with one CTA.
 //
+// Narrow levels (res_build): bands of levels.
+//
 // Any other order: each level's rows are dealt in equal ranges (balanced, but a
 // CTA's share moves through the mesh from level to level), or, where the rows'
 // cell centres are known and every level stays balanced, the mesh is cut into
@@ -155,15 +157,15 @@ __global__ void k_res_cuts(int64_t n, int C, ResAxes *a) {
         before += w[k];
     }
 }
-// The balanced candidate, and the rows of every (axis, CTA, level) of the slabs.
-__global__ void k_res_owner(int64_t n, int C, int32_t nlev, const int32_t *__restrict__ order,
+// Bands of levels, or the balanced candidate and the rows of every (axis, CTA, level) of the slabs.
+__global__ void k_res_owner(int64_t n, int C, bool bands, int32_t nlev, const int32_t *__restrict__ order,
                             const int32_t *__restrict__ level, const int32_t *__restrict__ lstart,
                             const double4 *__restrict__ cell, const ResAxes *__restrict__ a,
                             uint32_t *__restrict__ owner, int32_t *__restrict__ hist) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int32_t i = order[p], l = level[i], s = lstart[l];
-    owner[i] = (uint32_t)((p - s) * C / (lstart[l + 1] - s));
+    owner[i] = bands ? (uint32_t)(p * C / n) : (uint32_t)((p - s) * C / (lstart[l + 1] - s));
     if (!cell) return;
     const double4 c = cell[i];
     for (int d = 0; d < 3; ++d)
@@ -416,6 +418,7 @@ int res_launchable(const fv_resident *p) {
 }
 
 constexpr int kResMaxCtas = 160;  // CTAs of all clusters
+constexpr size_t kResSparseBytes = 64u << 20;  // records of a plan of mostly idle slots, at most
 
 // Shares the problems out over clusters: the cluster size whose fullest CTA has
 // the fewest rows, problems to the emptiest cluster in descending size.
@@ -517,11 +520,25 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     if (n <= 0 || n > (problems ? 148 : kResMaxCta) * 20000LL || s.max_side > 6 || !s.fwd_level || !s.bwd_level)
         return FV_OK;
     if (problems && !s.sorted) return FV_OK;
+    const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
+    int C = 1, width = 32;
+    while (C < kResMaxCta && n > (int64_t)C * 18000) C *= 2;  // shared memory for the rows
+    // Narrow levels (long chains, channels): one step holds a level, so the rows go
+    // to the CTAs in bands of levels.  Dealt over the CTAs each level would be
+    // handed over and every row fill a step of its own (4 KB of records per row
+    // with 16 rows per level on 16 CTAs).  us per apply, dealt / in bands / level
+    // chunks: 100,000-row IC(0) 16 rows per level 1,662 / 998 / 11,749, 64 rows 494 /
+    // 301 / 2,940; 30,000 rows, 32 per level 249 / 187 / 1,851.  Above 64 rows a band's
+    // steps are 128 wide with four thread sets, and a 2D mesh (24,200 rows, 110 per
+    // level: 77 / 99) is better dealt, unless that leaves four slots to a row.  Rows
+    // sorted by level have their own rule below; chains among them do not.
+    const bool narrow = !problems && (s.sorted ? lw <= 32 && n > 12000 : lw <= 64 || (lw <= 128 && lw < 8 * C));
+    const bool wide = s.sorted && !narrow;
     // Rows sorted by level in one cluster: few wide levels, which more than 5,000
     // rows a CTA take longer than consecutive rows on all SMs.  us per apply with
     // 23 of launch and check, resident against consecutive: 32,768-row IC(0) 40 52,
     // 65,522 rows 50 55, 131,072 rows 60 49; ILU(0) 24,576 rows 47 62, 82,944 62 62.
-    if (s.sorted && !problems && n > kResMaxCta * 5000LL) return FV_OK;
+    if (wide && !problems && n > kResMaxCta * 5000LL) return FV_OK;
     // CTAs: enough shared memory for the rows, and as few as keep a level of a
     // CTA within 128 rows (natural order: more CTAs only add hand-offs) or as
     // many as leave it 32 (rows sorted by level: few, wide levels).  Measured as
@@ -529,11 +546,9 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     // 48,000-row ILU(0), natural, C x width: 4x128 84, 8x128 84, 16x64 96,
     // 16x32 100; 32,768-row IC(0), sorted: 16x256 36, 16x128
     // 38, 8x128 46, 8x64 48 (consecutive rows 52).
-    int C = 1, width = 32;
-    const int64_t lw = n / std::max(1, s.n_fwd_levels);  // rows per level
-    while (C < kResMaxCta && (n > (int64_t)C * 18000 || lw > (int64_t)C * (s.sorted ? 32 : 128))) C *= 2;
+    while (C < kResMaxCta && lw > (int64_t)C * (wide ? 32 : 128)) C *= 2;
     if (t.more_ctas && !problems) C = std::min(2 * C, kResMaxCta);
-    while (width < (s.sorted ? 256 : 128) && lw * (s.sorted ? 2 : 1) > (int64_t)C * width) width *= 2;
+    while (width < (wide ? 256 : 128) && lw * (wide ? 2 : 1) > (int64_t)(narrow ? 1 : C) * width) width *= 2;
     std::vector<int32_t> cluster;  // of every problem
     int clusters = 1;
     if (problems) FV_TRY(res_share_problems(*problems, s.n_fwd_levels, C, width, clusters, cluster));
@@ -551,7 +566,7 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     p->C = C;
     p->clusters = clusters;
     p->width = width;
-    p->sorted = s.sorted;
+    p->sorted = wide;
     p->sets = sets;
     p->ml = ml;
     p->cap = (int32_t)((n + ctas - 1) / ctas);  // at least
@@ -570,6 +585,7 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     a.col[0] = s.l_col, a.col[1] = s.u_col;
     a.level[0] = s.fwd_level, a.level[1] = s.bwd_level;
     a.nlev[0] = s.n_fwd_levels, a.nlev[1] = s.n_bwd_levels;
+    const double4 *cell = narrow || wide || problems || ctas == 1 ? nullptr : s.cell;
     const int64_t items = 2 * n, nk = (int64_t)ctas * a.keys(), nnz = s.nnz_l + s.nnz_u;
     const int64_t cm = std::max(items, nk) + 2;
     Layout pl, tl;
@@ -578,7 +594,7 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     const size_t t_owner = tl.take(4 * n), t_iota = tl.take(4 * items), t_key = tl.take(4 * items),
                  t_sorted = tl.take(4 * items), t_item = tl.take(4 * items), t_cnt = tl.take(4 * cm),
                  t_cnt2 = tl.take(4 * cm), t_hc = tl.take(4 * (ctas + 1)), t_prob = tl.take(problems ? 12 * (size_t)problems->n : 0), t_axes = tl.take(sizeof(ResAxes)),
-                 t_hist = tl.take(s.cell ? 12 * (size_t)C * a.nlev[0] : 0), t_lst = tl.take(4 * (a.nlev[0] + 2)),
+                 t_hist = tl.take(cell ? 12 * (size_t)C * a.nlev[0] : 0), t_lst = tl.take(4 * (a.nlev[0] + 2)),
                  t_mask = tl.take(4 * items), t_poff = tl.take(4 * (items + 1)), t_hslot = tl.take(2 * (nnz + 1)),
                  t_first = tl.take(4 * (nk + 1)), t_soff = tl.take(4 * (nk + 1));
     size_t sort_bytes = 0, scan_bytes = 0;
@@ -634,25 +650,27 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
         fv_note_launch(), k_res_root_count<<<grid(n), 256, 0, st>>>(n, lst, s.perm, problems->of_row, root0, nroot);
         fv_note_launch(), k_res_owner_batch<<<grid(n), 256, 0, st>>>(n, C, s.perm, problems->of_row, dcl, root0, nroot,
                                                                      s.l_ptr, s.l_col, owner);
-    } else if (s.sorted) {
+    } else if (ctas == 1) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(owner, 0, 4 * n, st);
+    } else if (wide) {
         fv_note_launch(), k_res_owner_sorted<<<grid(n), 256, 0, st>>>(n, C, lst, s.l_ptr, s.l_col, owner);
     } else {
         int32_t *hist = i32(t_hist);
         ResAxes *ax = (ResAxes *)(tmp + t_axes);
         const unsigned gs = std::min(grid(n), 296u);
-        if (s.cell) {
+        if (cell) {
             if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, 12 * (size_t)C * a.nlev[0], st);
             fv_note_launch(), k_res_axes_init<<<1, 256, 0, st>>>(ax);
-            fv_note_launch(), k_res_extent<<<gs, 256, 0, st>>>(n, s.cell, ax);
-            fv_note_launch(), k_res_bins<<<gs, 256, 0, st>>>(n, s.cell, ax);
+            fv_note_launch(), k_res_extent<<<gs, 256, 0, st>>>(n, cell, ax);
+            fv_note_launch(), k_res_bins<<<gs, 256, 0, st>>>(n, cell, ax);
             fv_note_launch(), k_res_cuts<<<1, 96, 0, st>>>(n, C, ax);
         }
-        fv_note_launch(), k_res_owner<<<grid(n), 256, 0, st>>>(n, C, a.nlev[0], s.fwd_order, s.fwd_level, lst, s.cell, ax,
-                                                               owner, hist);
-        if (s.cell) {
-            fv_note_launch(), k_res_cross<<<gs, 256, 0, st>>>(n, s.l_ptr, s.l_col, s.cell, owner, ax);
+        fv_note_launch(), k_res_owner<<<grid(n), 256, 0, st>>>(n, C, narrow, a.nlev[0], s.fwd_order, s.fwd_level, lst,
+                                                               cell, ax, owner, hist);
+        if (cell) {
+            fv_note_launch(), k_res_cross<<<gs, 256, 0, st>>>(n, s.l_ptr, s.l_col, cell, owner, ax);
             fv_note_launch(), k_res_choose<<<1, 256, 0, st>>>(C, width, a.nlev[0], lst, hist, ax);
-            fv_note_launch(), k_res_pick<<<grid(n), 256, 0, st>>>(n, s.cell, ax, owner);
+            fv_note_launch(), k_res_pick<<<grid(n), 256, 0, st>>>(n, cell, ax, owner);
         }
     }
     sort(owner, p->rows, n, ctas);
@@ -687,6 +705,15 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
         t.full = !h_hc[ctas] && !small;
         t.C = C;
         t.rows = (size_t)(p->cap + 2 + p->halo) * sizeof(double);
+        cudaFreeAsync(tmp, st);
+        fv_resident_free(p);
+        return FV_OK;
+    }
+    // A step is filled by a level of 32 rows or more.  Below 7 rows per level the
+    // idle slots are most of what the plan holds (64 bytes a slot and more, where
+    // the factor has some 100 a row), so only small plans are let be that sparse;
+    // the others' rows are swept by level chunks.
+    if (p->nslots > 5 * items && fv_resident_record_bytes(p, sizeof(double)) > kResSparseBytes) {
         cudaFreeAsync(tmp, st);
         fv_resident_free(p);
         return FV_OK;

@@ -20,3 +20,45 @@ def test_natural_orders_between_the_sizes_that_fit_at_once(fv, dim, side, fits):
     P, Q = _pair(fv, fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper, A)
     assert P.resident() == fits
     _same_apply(fv, P, Q, case["mesh"].n_cells)
+
+
+def _channel(nx, ny):
+    """5-point operator on nx x ny points, no mesh behind it: about nx rows per level."""
+    n = nx * ny
+    i = np.arange(n)
+    x, y = i % nx, i // nx
+    rows, cols, vals = [i], [i], [4.5 + 0.1 * np.sin(i)]
+    for ok, off in ((x > 0, -1), (x < nx - 1, 1), (y > 0, -nx), (y < ny - 1, nx)):
+        rows.append(i[ok])
+        cols.append(i[ok] + off)
+        vals.append(-1.0 + 0.01 * np.sin(i[ok] + (i[ok] + off)))
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    o = np.lexsort((c, r))
+    return np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]), c[o], v[o]
+
+
+@pytest.mark.parametrize("nx,n,fits", [(1, 5000, True), (1, 40_000, False), (2, 20_000, True), (4, 100_000, False),
+                                       (7, 60_000, True), (16, 100_000, True), (33, 50_000, True), (64, 300_000, True), (65, 30_000, True),
+                                       (100, 300_000, True),
+                                       (127, 40_000, True), (129, 40_000, True)])
+def test_narrow_levels(fv, nx, n, fits):
+    """Few rows per level: bands of levels, without a record's step for every row;
+    where idle slots would be most of a large plan, there is none."""
+    import torch
+    A = fv.DistributedMatrix.from_csr(*_channel(nx, n // nx))
+    rows = A.nrows()
+    fv.IncompleteCholesky.from_matrix(A, 0).close()  # the symbolic analysis stays with A
+    fv.release_kept_memory()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    P = fv.IncompleteCholesky.from_matrix(A, 0)
+    torch.cuda.synchronize()
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert P.resident() == fits
+    assert taken <= 128 << 20 or taken <= 800 * rows  # 5 slots of 64 bytes, twice; factor and vectors
+    Q = fv.IncompleteCholesky.from_matrix(A, 0)
+    Q.schedule(1)
+    _same_apply(fv, P, Q, rows)
+    P.refactor()
+    Q.refactor()
+    _same_apply(fv, P, Q, rows, 1)
