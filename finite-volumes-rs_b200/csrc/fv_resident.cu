@@ -718,6 +718,26 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
         fv_resident_free(p);
         return FV_OK;
     }
+    // Orders without locality (a random numbering, an unstructured mesh's own): the
+    // levels are few and wide and most rows' values go to other CTAs, so a step
+    // waits on hand-offs.  Fitted over 2D and 3D meshes of 8,000-180,000 rows in
+    // random and block-wise random orders (within 7 % in the median): an apply takes
+    // 33 us + (0.114 + 0.193 h) per step with h halo slots per row, level chunks 33 us +
+    // 1.0-3 per level.  us per apply, resident / level chunks: 64,800-row IC(0) random
+    // 85 / 54 (h 2.7, 80 steps, 22 levels), 63,888-row ILU(0) 100 / 63, 180,000 rows in
+    // random blocks of 512 110 / 89 (h 1.0, 190 steps, 24 levels); kept: 105,800 rows in
+    // such blocks 62 / 87 (h 1.0, 120 steps, 24 levels), 48,000 75 / 87.  Up to 30,000 rows whole iterations in
+    // the cluster win with any order (24,200 rows random, CG: 44 / 68 us each).
+    if (!problems && n > 30000) {
+        int steps = 0;
+        for (int c = 0; c < ctas; ++c) steps = std::max(steps, h_sptr[c + 1] - h_sptr[c]);
+        const double h = (double)p->halo / p->cap;
+        if (h > 0.95 && steps * (0.114 + 0.193 * h) > (h > 1.05 ? 1.0 : 2.2) * (a.nlev[0] + a.nlev[1])) {
+            cudaFreeAsync(tmp, st);
+            fv_resident_free(p);
+            return FV_OK;
+        }
+    }
     Layout sl;
     const size_t s_item = sl.take(4 * p->nslots), s_dep = sl.take(2 * (size_t)p->ml * p->nslots),
                  s_push = sl.take(8 * p->nslots);

@@ -62,3 +62,18 @@ def test_narrow_levels(fv, nx, n, fits):
     P.refactor()
     Q.refactor()
     _same_apply(fv, P, Q, rows, 1)
+
+
+@pytest.mark.parametrize("dim,side,block,fits", [(2, 100, 1, True), (2, 150, 1, False), (2, 150, 512, True),
+                                                 (3, 14, 1, True), (3, 22, 1, False)])
+def test_orders_without_locality(fv, dim, side, block, fits):
+    """Rows, or blocks of them, in random order: swept by level chunks where most values would be handed over."""
+    case = diffusion_2d(fv, side, seed=69) if dim == 2 else convdiff_3d(fv, side, seed=69)
+    A, _ = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    n = case["mesh"].n_cells
+    parts = np.array_split(np.arange(n, dtype=np.int32), n // block)
+    order = np.random.default_rng(8).permutation(len(parts))
+    perm = np.concatenate([parts[k] for k in order])
+    P, Q = _pair(fv, fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper, A, ordering=perm)
+    assert P.resident() == fits
+    _same_apply(fv, P, Q, n)
