@@ -566,7 +566,6 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     p->C = C;
     p->clusters = clusters;
     p->width = width;
-    p->sorted = wide;
     p->sets = sets;
     p->ml = ml;
     p->cap = (int32_t)((n + ctas - 1) / ctas);  // at least

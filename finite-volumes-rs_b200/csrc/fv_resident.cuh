@@ -71,7 +71,6 @@ struct fv_resident {
     int32_t cap = 0;               // most rows of a CTA
     int32_t halo = 0;              // most halo slots of a CTA
     int64_t nslots = 0;            // slots of all steps
-    bool sorted = false;           // rows sorted by forward level
     int32_t *cta_ptr = nullptr;    // [clusters * C + 1] first entry of a CTA in `rows`
     int32_t *rows = nullptr;       // slot k of CTA c holds row rows[cta_ptr[c] + k]
     int32_t *nat = nullptr;        // the same rows in the caller's numbering (null: no permutation)

@@ -1053,11 +1053,12 @@ fv_status loop_resident(const Workspace &w, const fv_csr *A, fv_precond *P, doub
     int *err = nullptr;
     const fv_resident *plan = P ? fv_precond_resident(P, &rec, &err) : nullptr;
     // Up to where whole iterations in one cluster beat kernels on all SMs, us per
-    // iteration (resident / kernels): CG natural 32,768 rows 95 / 102, 45,000
-    // 132 / 126; CG in box order 65,522 rows 47 / 55, 96,800 57 / 55; BiCGStab
-    // natural 48,000 rows 155 / 180, 82,944 223 / 177; 2,048 rows 32 / 49 (with
-    // sweeps of 0.14 us per level on both sides, now 0.11).
-    const int64_t most = BICG ? 50000 : plan && plan->sorted ? 75000 : 36000;
+    // iteration (resident / kernels, both with resident sweeps; natural, box order,
+    // permuted): CG 45,000 rows 98 / 110, 39 / 52, 38 / 52; 72,200 rows 119 / 121, 58 / 60,
+    // 56 / 59; 79,202 rows 124 / 126, 59 / 59, 57 / 57.  BiCGStab 48,000 rows 155 / 167,
+    // 96 / 106, 93 / 105; 63,888 rows 191 / 204, 116 / 119, 112 / 116; 73,002 rows 218 / 216,
+    // 134 / 127, 130 / 124.  1,800 rows, CG: 26 / 43, 22 / 38, 22 / 38.
+    const int64_t most = BICG ? 65000 : 75000;
     if (!plan || A->nrows > most) return FV_OK;
     const size_t smem = kRsBytes + fv_resident_smem(plan, sizeof(double));
     int L = plan->C;  // CTAs: those of the sweeps, and more where the vectors need them

@@ -77,3 +77,21 @@ def test_orders_without_locality(fv, dim, side, block, fits):
     P, Q = _pair(fv, fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper, A, ordering=perm)
     assert P.resident() == fits
     _same_apply(fv, P, Q, n)
+
+
+@pytest.mark.parametrize("dim,side,ordering", [(2, 142, None), (2, 193, None), (2, 194, None), (2, 193, "boxes"),
+                                               (3, 22, None), (3, 22, "boxes"), (3, 23, None)])
+def test_whole_iterations_up_to_their_rows(fv, dim, side, ordering):
+    """75,000 rows of CG and 65,000 of BiCGStab, just below and above: the kernels' bits and history."""
+    case = diffusion_2d(fv, side, seed=71) if dim == 2 else convdiff_3d(fv, side, seed=71)
+    solve = fv.conjugate_gradient if dim == 2 else fv.bi_conjugate_gradient_stab
+    A, b = fv.assemble(equation(fv, case), (case["bndi"], case["bnde"]), case["mesh"])
+    P, Q = _pair(fv, fv.IncompleteCholesky if dim == 2 else fv.IncompleteLowerUpper, A, ordering=ordering)
+    for tol, limit in ((0.0, 7), (1e-6, 300)):
+        got = []
+        for M in (P, Q):
+            x = fv.DistributedVector.from_size(A.nrows())
+            info = solve(x, A, b, M, None, fv.LinearSolverOptions(tol, tol, limit))
+            got.append((x.numpy(), np.array(info.history), info.iterations, info.status))
+        assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+        assert got[0][2:] == got[1][2:]
