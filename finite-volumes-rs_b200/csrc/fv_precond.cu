@@ -165,6 +165,11 @@ static fv_status resident_no_memory(fv_precond *P) {
     return FV_OK;
 }
 
+// What the plan adds to a factorisation's set-up (once per factor; PermutedSystem and
+// from_matrix make it): 0.05-0.1 ms on 2,048 rows (0.25 ms in all), and the mapping of
+// its memory where no kept block serves, 65,522 rows in box order 1.44 -> 2.4-2.9 ms
+// the first time.  With kept blocks the same factorisation takes 0.31 ms, without
+// plan and kept blocks it took 0.85.
 static fv_status resident_plan(fv_precond *P, const int32_t *perm, cudaStream_t st) {
     const fv_resident_src q = resident_src(P, perm);
     const fv_status s = fv_resident_build(q, st, &P->res);

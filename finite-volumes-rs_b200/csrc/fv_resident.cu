@@ -193,7 +193,8 @@ __global__ void k_res_cross(int64_t n, const int32_t *__restrict__ lp, const int
 // fullest CTA), when that is at most a quarter more than the balanced number
 // and the slabs at least halve the dependencies between CTAs (they do on 3D
 // meshes; on the 2D ones the balanced ranges move little from level to level
-// and the slabs were slower: 65,522-row IC(0) 219 us per apply against 139).
+// and the slabs were slower: 65,522-row IC(0) 195 us per apply against 108, where
+// 24,576-row ILU(0) takes 51 in slabs and 115 dealt).
 // One block.
 __global__ void k_res_choose(int C, int width, int32_t nlev, const int32_t *__restrict__ lstart,
                              const int32_t *__restrict__ hist, ResAxes *a) {
@@ -499,8 +500,8 @@ void fv_resident_free(fv_resident *p) {
 size_t fv_resident_record_bytes(const fv_resident *p, size_t tb) { return (size_t)p->nslots * res_rec_bytes(p->ml, tb); }
 
 // How to go on when the shared memory of the buffers and the rows does not fit:
-// the rows over twice the CTAs (65,522-row IC(0), 362 levels: 131 -> 114 us per
-// apply), then half the thread sets and with them half the buffers (105,456-row
+// the rows over twice the CTAs (65,522-row IC(0), 362 levels, on 4 CTAs with half the
+// sets and on 8: 170 -> 111 us per apply), then half the thread sets and with them half the buffers (105,456-row
 // ILU(0): 204 us per apply with level chunks, 122 this way).
 struct ResTry {
     bool more_ctas = false;
@@ -536,29 +537,30 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     const bool wide = s.sorted && !narrow;
     // Rows sorted by level in one cluster: few wide levels, which more than 5,000
     // rows a CTA take longer than consecutive rows on all SMs.  us per apply with
-    // 23 of launch and check, resident against consecutive: 32,768-row IC(0) 40 52,
-    // 65,522 rows 50 55, 131,072 rows 60 49; ILU(0) 24,576 rows 47 62, 82,944 62 62.
+    // 23 of launch and check, resident against consecutive: 32,768-row IC(0) 41 47,
+    // 80,000 rows 48 49, 131,072 rows 59 50; ILU(0) 24,576 rows 47 62, 82,944 62 62.
     if (wide && !problems && n > kResMaxCta * 5000LL) return FV_OK;
     // CTAs: enough shared memory for the rows, and as few as keep a level of a
     // CTA within 128 rows (natural order: more CTAs only add hand-offs) or as
     // many as leave it 32 (rows sorted by level: few, wide levels).  Measured as
     // us per apply, the launch and its status check (23 us) included:
-    // 48,000-row ILU(0), natural, C x width: 4x128 84, 8x128 84, 16x64 96,
-    // 16x32 100; 32,768-row IC(0), sorted: 16x256 36, 16x128
-    // 38, 8x128 46, 8x64 48 (consecutive rows 52).
+    // 48,000-row ILU(0), natural, C x width: 4x128 79, 8x128 87, 16x64 100, 16x32
+    // 105; 32,768-row IC(0), sorted: 16x256 40, 16x128 41, 8x128 50, 8x64 49
+    // (consecutive rows 47).
     while (C < kResMaxCta && lw > (int64_t)C * (wide ? 32 : 128)) C *= 2;
     if (t.more_ctas && !problems) C = std::min(2 * C, kResMaxCta);
     while (width < (wide ? 256 : 128) && lw * (wide ? 2 : 1) > (int64_t)(narrow ? 1 : C) * width) width *= 2;
     std::vector<int32_t> cluster;  // of every problem
     int clusters = 1;
     if (problems) FV_TRY(res_share_problems(*problems, s.n_fwd_levels, C, width, clusters, cluster));
-    // entries per record: a padded one costs a dependent subtraction (131,072-row
-    // IC(0) in natural order with 3 and 2 per side: 149 and 140 us per apply)
+    // entries per record: a padded one costs a dependent subtraction and its bytes
+    // (131,072-row IC(0) in natural order with 3 and 2 per side: 146 and 145 us per
+    // apply; the whole solve 94.2 and 92.7 ms)
     const int ml = s.max_side <= 2 ? 2 : s.max_side <= 3 ? 3 : s.max_side <= 4 ? 4 : 6, ctas = C * clusters;
     // Thread sets: with four, the unpacking of a record (some 500 cycles) sets the
     // pace of a 100-cycle step; eight of up to 64 threads hide it.  Four -> eight,
-    // us per apply in natural order: 8,192-row IC(0), 128 levels, 62 -> 51;
-    // 131,072 rows, 512 levels, 158 -> 149.
+    // us per apply in natural order: 8,192-row IC(0), 128 levels, 59 -> 48;
+    // 131,072 rows, 512 levels, 149 -> 145.
     const int sets = (width > 64 ? 512 / width : 8) >> t.half_sets;
     if (sets < 2) return FV_OK;
     fv_resident *p = new (std::nothrow) fv_resident();

@@ -13,9 +13,10 @@
 // memory (30 cycles), the row's FP64 chain (40), one store and one barrier.
 //
 // Measured per apply (both sweeps; level chunks -> resident): 131,072-row IC(0)
-// in natural order (512 levels) 568 -> 117 us, 24,576-row ILU(0) (64 levels)
-// 100 -> 28 us, 196,608-row ILU(0) (128 levels) 190 -> 52 us; 65,522-row IC(0)
-// in box order (18 wide levels; consecutive rows -> resident) 32 -> 27 us.
+// in natural order (512 levels) 569 -> 122 us, 24,576-row ILU(0) (64 levels)
+// 98 -> 28 us, 196,608-row ILU(0) (128 levels) 189 -> 52 us; 24,576-row ILU(0) in box
+// order (28 wide levels; consecutive rows -> resident) 39 -> 24 us, 65,522-row IC(0)
+// (18 levels) 26 -> 25 us.
 //
 // Rows are computed with the operations of k_sweep in the same order, so the
 // results are the same bits.
