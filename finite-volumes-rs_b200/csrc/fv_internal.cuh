@@ -77,6 +77,10 @@ void fv_blocks_free(void *const *blocks, int n);
 void fv_block_free(void *p);
 unsigned long long fv_current_context_id();  // 0 when unknown
 unsigned long long fv_bound_context_id();    // the current device's context, made current first; 0 when unknown
+// A pinned int of the context with this id (0: unknown), null without memory for
+// it; idle: nothing in flight writes it any more.
+int *fv_flag_take(unsigned long long ctx);
+void fv_flag_return(unsigned long long ctx, int *flag, bool idle);
 void fv_note_launch();
 void fv_note_launches(long long delta);  // graph replays add, captures (not run) subtract
 unsigned long long fv_launches_now();

@@ -30,6 +30,7 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "fv_internal.cuh"
 
@@ -226,4 +227,40 @@ void fv_blocks_free(void *const *blocks, int n) {
         }
         if (!kept) fv_block_free(blocks[i]);
     }
+}
+
+// Flags wait under their context's id: replacing a context frees its pinned
+// memory.  At most as many as were taken at once (freeing pinned memory may
+// synchronise the device, so a solve does not).
+static std::map<unsigned long long, std::vector<int *>> g_flags;
+
+int *fv_flag_take(unsigned long long ctx) {
+    if (ctx != 0) {
+        std::lock_guard<std::mutex> g(g_mu);
+        const auto it = g_flags.find(ctx);
+        if (it != g_flags.end() && !it->second.empty()) {
+            int *const flag = it->second.back();
+            it->second.pop_back();
+            return flag;
+        }
+    }
+    int *flag = nullptr;
+    if (cudaHostAlloc((void **)&flag, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        flag = nullptr;
+    }
+    return flag;
+}
+
+void fv_flag_return(unsigned long long ctx, int *flag, bool idle) {
+    if (!flag) return;
+    if (idle && ctx != 0) {
+        try {
+            std::lock_guard<std::mutex> g(g_mu);
+            g_flags[ctx].push_back(flag);
+            return;
+        } catch (...) {  // host memory for the list: freed then
+        }
+    }
+    cudaFreeHost(flag);
 }

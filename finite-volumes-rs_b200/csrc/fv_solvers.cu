@@ -922,28 +922,6 @@ fv_status apply_or_copy(fv_precond *P, const double *r, double *z, int64_t n, in
 
 int batch_size(int64_t n) { return n >= (1 << 20) ? 4 : 8; }
 
-// One pinned int per host thread for the done flag of loop_until_done,
-// allocated on first use and kept for the thread's life (freeing pinned
-// memory may synchronise the device); nullptr if it cannot be allocated.
-int *pinned_flag() {
-    struct Holder {
-        int *p = nullptr;
-        bool tried = false;
-        ~Holder() {
-            if (p) cudaFreeHost(p);
-        }
-    };
-    thread_local Holder h;
-    if (!h.tried) {
-        h.tried = true;
-        if (cudaHostAlloc((void **)&h.p, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
-            h.p = nullptr;
-            cudaGetLastError();
-        }
-    }
-    return h.p;
-}
-
 // Runs body(stream) -- one batch of iterations -- until the device state says
 // done.  The batch is captured once into a CUDA graph on a private stream (the
 // legacy default stream cannot be captured) and replayed, so the GPU runs the
@@ -974,7 +952,8 @@ fv_status loop_until_done(const Workspace &w, cudaStream_t st, Body body, Solver
         cudaGetLastError();
     }
     fv_status s = FV_OK;
-    int *done_h = pinned_flag();
+    const unsigned long long ctx = fv_bound_context_id();
+    int *done_h = fv_flag_take(ctx);
     cudaEvent_t evd = nullptr;
     if (graph_ok && done_h && cudaEventCreateWithFlags(&evd, cudaEventDisableTiming) == cudaSuccess) {
         // The next replay is queued before the host waits for the previous
@@ -1035,6 +1014,7 @@ fv_status loop_until_done(const Workspace &w, cudaStream_t st, Body body, Solver
             if (s != FV_OK || h.done) break;
         }
     }
+    fv_flag_return(ctx, done_h, s == FV_OK);  // after an error a copy into it may be under way
     if (evd) cudaEventDestroy(evd);
     if (gx) cudaGraphExecDestroy(gx);
     if (ev) cudaEventDestroy(ev);

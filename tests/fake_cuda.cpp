@@ -78,6 +78,9 @@ cudaError_t fv_block_alloc_raw(void **p, size_t bytes);
 cudaError_t fv_device_malloc_raw(void **p, size_t bytes);
 cudaError_t fv_malloc_async_raw(void **p, size_t bytes, cudaStream_t st);
 void fv_blocks_free(void *const *blocks, int n);
+unsigned long long fv_bound_context_id();
+int *fv_flag_take(unsigned long long ctx);
+void fv_flag_return(unsigned long long ctx, int *flag, bool idle);
 
 extern "C" {
 
@@ -94,6 +97,16 @@ void *stream_alloc(size_t bytes) {
     void *p = nullptr;
     return fv_malloc_async_raw(&p, bytes, nullptr) == cudaSuccess ? p : nullptr;
 }
+// Takes a flag, says whether its memory is there, and gives it back.
+int flag_is_there(int idle) {
+    const unsigned long long ctx = fv_bound_context_id();
+    int *const f = fv_flag_take(ctx);
+    Lock l(g_mu);
+    const bool there = f && g.host.count((char *)f);
+    fv_flag_return(ctx, f, idle != 0);
+    return there;
+}
+size_t fake_pinned() { return g.host.size(); }
 void pool_free(void *p) { fv_blocks_free(&p, 1); }
 void fake_reset() {
     Lock l(g_mu);

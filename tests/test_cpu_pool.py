@@ -186,3 +186,14 @@ def test_a_block_is_handed_out_again_only_when_its_work_is_done(cu):
     before = cu.fake_count(MALLOCS), cu.fake_count(FREES)
     cu.pool_free(None)  # an object without blocks waits for nothing
     assert (cu.fake_count(MALLOCS), cu.fake_count(FREES)) == before and cu.fake_count(BAD) == 0
+
+
+def test_flags_of_a_replaced_context(cu):
+    cu.fake_pinned.restype = C.c_size_t
+    for _ in range(3):
+        assert cu.flag_is_there(1)
+    assert cu.fake_pinned() == 1
+    cu.fake_replace_context()
+    assert cu.flag_is_there(1)
+    assert cu.flag_is_there(0) and cu.fake_pinned() == 0  # taken again, then freed: work was in flight
+    assert cu.fake_count(BAD) == 0
