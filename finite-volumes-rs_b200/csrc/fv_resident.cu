@@ -501,8 +501,9 @@ size_t fv_resident_record_bytes(const fv_resident *p, size_t tb) { return (size_
 
 // How to go on when the shared memory of the buffers and the rows does not fit:
 // the rows over twice the CTAs (65,522-row IC(0), 362 levels, on 4 CTAs with half the
-// sets and on 8: 170 -> 111 us per apply), then half the thread sets and with them half the buffers (105,456-row
-// ILU(0): 204 us per apply with level chunks, 122 this way).
+// sets and on 8: 170 -> 111 us per apply), then half the thread sets and with them
+// half the buffers (105,456-row ILU(0): 204 us per apply with level chunks, 122 this
+// way).
 struct ResTry {
     bool more_ctas = false;
     int half_sets = 0;
@@ -727,8 +728,9 @@ static fv_status res_build(const fv_resident_src &s, cudaStream_t st, fv_residen
     // 1.0-3 per level.  us per apply, resident / level chunks: 64,800-row IC(0) random
     // 85 / 54 (h 2.7, 80 steps, 22 levels), 63,888-row ILU(0) 100 / 63, 180,000 rows in
     // random blocks of 512 110 / 89 (h 1.0, 190 steps, 24 levels); kept: 105,800 rows in
-    // such blocks 62 / 87 (h 1.0, 120 steps, 24 levels), 48,000 75 / 87.  Up to 30,000 rows whole iterations in
-    // the cluster win with any order (24,200 rows random, CG: 44 / 68 us each).
+    // such blocks 62 / 87 (h 1.0, 120 steps, 24 levels), 48,000 75 / 87.  Up to 30,000
+    // rows whole iterations in the cluster win with any order (24,200 rows random, CG:
+    // 44 / 68 us each).
     if (!problems && n > 30000) {
         int steps = 0;
         for (int c = 0; c < ctas; ++c) steps = std::max(steps, h_sptr[c + 1] - h_sptr[c]);
